@@ -38,6 +38,12 @@ struct AmgPreconditioner::Level {
     DeviceArray<double> s_val;           // FP64 values (FP64 V-cycle; on level 0 also the Krylov matrix)
     DeviceArray<double> w;               // first Jacobi sweep (FP64 V-cycle)
     DeviceArray<float> s_val32, diag32, rd32, x32, b32, w32, t32;
+    // tree numbering (pcg_tree.cuh): maps, the columns' positions, and the level's vectors
+    int npos = 0;
+    DeviceArray<int> t_row, t_rank, t_pos, t_pcol, at;  // at: row -> position
+    DeviceArray<int4> t_memb;
+    DeviceArray<double> tb, tw, te;
+    DeviceArray<float> tb32, tw32, te32;
     void buildSell(const int* hptr, const int* hcol, cudaStream_t s) {
         SellPattern pat;
         pat.build(n, hptr, hcol);
@@ -51,7 +57,8 @@ struct AmgPreconditioner::Level {
 
 namespace {
 constexpr int kBlock = 256;
-constexpr double kOmega = 2.0 / 3.0;
+// Largest level whose whole V-cycle is kept as a dense matrix (8 MB at 1024 rows, read from L2).
+constexpr int kFoldRows = 1200;
 
 struct HostCsr {
     int n = 0;
@@ -255,6 +262,52 @@ __global__ void __cluster_dims__(kDenseCluster, 1, 1)
     for (int e = threadIdx.x; e < nr * n; e += blockDim.x) M[static_cast<long long>(r0) * n + e] = Ml[e];
 }
 
+// foldCoarse, first pass: column j of Y = M T, one block per j.  Column j of T has 1 - a_jj w_j at
+// j's aggregate and -a_ij w_j at each neighbour's.
+__global__ void kFoldColumns(int n, int nc, const int* __restrict__ ptr, const int* __restrict__ col,
+                             const double* __restrict__ diag, const double* __restrict__ val,
+                             const double* __restrict__ rd, const int* __restrict__ agg, const double* __restrict__ M,
+                             double* __restrict__ Y) {
+    const int j = blockIdx.x;
+    const double wj = rd[j];
+    const int k0 = ptr[j], k1 = ptr[j + 1];
+    for (int c = threadIdx.x; c < nc; c += blockDim.x) {
+        double y = (1.0 - diag[j] * wj) * M[static_cast<long long>(agg[j]) * nc + c];
+        for (int k = k0; k < k1; ++k) y -= val[k] * wj * M[static_cast<long long>(agg[col[k]]) * nc + c];
+        Y[static_cast<long long>(c) * n + j] = y;
+    }
+}
+
+// Second pass: the row of rank blockIdx.x, its entries by position.
+template <class T>
+__global__ void kFoldLines(int n, int npos, const int* __restrict__ pos, const int* __restrict__ row,
+                           const int* __restrict__ ptr, const int* __restrict__ col, const double* __restrict__ diag,
+                           const double* __restrict__ val, const double* __restrict__ rd, const int* __restrict__ agg,
+                           double gamma, const double* __restrict__ Y, const int* __restrict__ at, T* __restrict__ out) {
+    extern __shared__ double line[];
+    const int i = row[pos[blockIdx.x]];
+    const double wi = rd[i];
+    const int k0 = ptr[i], k1 = ptr[i + 1];
+    for (int p = threadIdx.x; p < npos; p += blockDim.x) {
+        const int j = row[p];
+        double b = 0.0;
+        if (j >= 0) {
+            b = (1.0 - diag[i] * wi) * Y[static_cast<long long>(agg[i]) * n + j];
+            for (int k = k0; k < k1; ++k) b -= val[k] * wi * Y[static_cast<long long>(agg[col[k]]) * n + j];
+            b *= gamma;
+        }
+        line[p] = b;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {  // a repeated pair has two entries: one thread adds them
+        line[at[i]] += 2.0 * wi - wi * diag[i] * wi;
+        for (int k = k0; k < k1; ++k) line[at[col[k]]] -= wi * val[k] * rd[col[k]];
+    }
+    __syncthreads();
+    for (int p = threadIdx.x; p < npos; p += blockDim.x)
+        out[static_cast<long long>(blockIdx.x) * npos + p] = static_cast<T>(line[p]);
+}
+
 __global__ void kDenseSolve(int n, const double* __restrict__ Minv, const double* __restrict__ b, double* __restrict__ x) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         double s = 0.0;
@@ -390,6 +443,7 @@ void AmgPreconditioner::buildStructure(const Dcsr<double>& A) {
     l0->nnz = A.nnz_off;
     l0->buildSell(cur.ptr.data(), cur.col.data(), ctx_.stream);
     levels_.push_back(l0);
+    std::vector<std::vector<int>> hptr, hcol, hagg;  // every level's pattern and aggregates
     while (cur.n > coarse_target && static_cast<int>(levels_.size()) < max_levels) {
         // aggregates from `passes` rounds of pairwise matching (2 by default: up to 4 rows)
         const int passes = levels_.size() == 1 ? passes0_ : passes_;
@@ -463,8 +517,14 @@ void AmgPreconditioner::buildStructure(const Dcsr<double>& A) {
         lv->buildSell(next.ptr.data(), next.col.data(), s);
         levels_.push_back(lv);
         ctx_.sync();
+        hptr.push_back(std::move(cur.ptr));
+        hcol.push_back(std::move(cur.col));
+        hagg.push_back(std::move(agg));
         cur = std::move(next);
     }
+    hptr.push_back(std::move(cur.ptr));
+    hcol.push_back(std::move(cur.col));
+    buildTree(hptr, hcol, hagg);
     for (Level* l : levels_) {
         l->x.resize(l->n);
         l->b.resize(l->n);
@@ -499,6 +559,155 @@ void AmgPreconditioner::buildStructure(const Dcsr<double>& A) {
                          levels_[i]->nnz, levels_[i]->n ? double(levels_[i]->nnz) / levels_[i]->n : 0.0);
         std::fprintf(stderr, "amg operator complexity %.3f\n", double(total) / double(levels_[0]->nnz + levels_[0]->n));
     }
+}
+
+void AmgPreconditioner::buildTree(const std::vector<std::vector<int>>& ptr, const std::vector<std::vector<int>>& col,
+                                  const std::vector<std::vector<int>>& agg) {
+    const int L = static_cast<int>(levels_.size());
+    tree_ = cfg_.amg_smoothing_steps <= 1 && L <= kMaxTreeLevels;
+    for (int l = 0; tree_ && l + 1 < L; ++l) {
+        std::vector<int> size(levels_[l + 1]->n, 0);
+        for (int I : agg[l])
+            if (++size[I] > 4) tree_ = false;
+    }
+    if (!tree_) return;
+    plan_.slices.assign(L, 0);
+    plan_.entries.assign(L, 0.0);
+    plan_.rows.assign(L, 0);
+    plan_.positions.assign(L, 0);
+    plan_.nnz = levels_[0]->nnz;
+    plan_.value_bytes = fp32_ ? 4 : 8;
+    plan_.level0_bytes = cfg_.precision == 1 ? 4 : 8;
+    // members of every row of level l + 1, in the order of their rows
+    const auto membersOf = [&](int l) {
+        std::vector<int4> m(levels_[l + 1]->n, make_int4(-1, -1, -1, -1));
+        for (int i = 0; i < levels_[l]->n; ++i) {
+            int4& q = m[agg[l][i]];
+            (q.x < 0 ? q.x : q.y < 0 ? q.y : q.z < 0 ? q.z : q.w) = i;
+        }
+        return m;
+    };
+    std::vector<int> order;  // rank -> row of the level above
+    for (int l = L - 1; l >= 0; --l) {
+        Level* lv = levels_[l];
+        const int n = lv->n;
+        std::vector<int> row, rank, pos(n), next(n);
+        if (l == L - 1) {
+            row.resize(n);
+            std::iota(row.begin(), row.end(), 0);
+            rank = row;
+            pos = row;
+            next = row;
+        } else {
+            const std::vector<int4> m = membersOf(l);
+            const long long npos = 4LL * levels_[l + 1]->n;
+            if (npos > 2LL * n + 64) break;  // mostly holes: this level and the finer ones keep their numbering
+            row.assign(npos, -1);
+            rank.assign(npos, -1);
+            int k = 0;
+            for (std::size_t c = 0; c < order.size(); ++c) {
+                const int4 q = m[order[c]];
+                const int rows[4] = {q.x, q.y, q.z, q.w};
+                for (int j = 0; j < 4; ++j) {
+                    if (rows[j] < 0) continue;
+                    row[4 * c + j] = rows[j];
+                    rank[4 * c + j] = k;
+                    pos[k] = static_cast<int>(4 * c) + j;
+                    next[k++] = rows[j];
+                }
+            }
+            plan_.slices[l] = (npos + 31) / 32;
+            double entries = 0.0;
+            for (long long p0 = 0; p0 < npos; p0 += 32) {
+                int w = 0;
+                for (long long p = p0; p < std::min(npos, p0 + 32); ++p)
+                    if (row[p] >= 0) w = std::max(w, ptr[l][row[p] + 1] - ptr[l][row[p]]);
+                entries += 32.0 * w;
+            }
+            plan_.entries[l] = entries;
+            if (!plan_.fits(l, ctx_.sm_count)) break;  // not even on the whole GPU
+        }
+        plan_.first = l;
+        lv->npos = static_cast<int>(row.size());
+        plan_.rows[l] = n;
+        plan_.positions[l] = lv->npos;
+        cudaStream_t s = ctx_.stream;
+        lv->t_row.upload(row, s);
+        lv->t_rank.upload(rank, s);
+        lv->t_pos.upload(pos, s);
+        if (l > 0) {
+            const std::vector<int4> m = membersOf(l - 1);
+            std::vector<int4> byPos(row.size(), make_int4(-1, -1, -1, -1));
+            for (std::size_t p = 0; p < row.size(); ++p)
+                if (row[p] >= 0) byPos[p] = m[row[p]];
+            lv->t_memb.upload(byPos, s);
+        }
+        if (l < L - 1) {
+            std::vector<int> at(n);
+            for (int k = 0; k < n; ++k) at[next[k]] = pos[k];
+            lv->at.upload(at, s);
+            std::vector<int> pcol(std::max<std::size_t>(col[l].size(), 1), 0);
+            for (int k = 0; k < ptr[l][n]; ++k) pcol[k] = at[col[l][k]];
+            lv->t_pcol.upload(pcol, s);
+        }
+        if (fp32_)
+            for (DeviceArray<float>* a : {&lv->tb32, &lv->tw32, &lv->te32}) {
+                a->resize(lv->npos);
+                a->zero(s);  // holes stay zero
+            }
+        else
+            for (DeviceArray<double>* a : {&lv->tb, &lv->tw, &lv->te}) {
+                a->resize(lv->npos);
+                a->zero(s);
+            }
+        ctx_.sync();
+        order = std::move(next);
+    }
+    // Level L - 2 and its V-cycle as one dense matrix (foldCoarse), where that level is small.
+    if (L >= 3 && plan_.first <= L - 2 && levels_[L - 2]->n <= kFoldRows) {
+        const std::size_t nc = levels_[L - 1]->n, n = levels_[L - 2]->n, np = levels_[L - 2]->npos;
+        fold_y_.resize(nc * n);
+        if (fp32_) folded32_.resize(n * np);
+        else folded_.resize(n * np);
+        plan_.folded = true;
+    }
+}
+
+// The V-cycle of level f = L - 2 as a matrix.  With W = omega D^-1, piecewise-constant P, the dense
+// inverse M of the coarsest level and T = P^T (I - A W), the cycle (one damped-Jacobi sweep
+// down and up, coarse correction scaled by gamma) maps b to (2 W - W A W + gamma T^T M T) b, which
+// foldCoarse forms in two passes, Y = M T and then its rows, per column of T from the matrix row
+// it comes from (A is symmetric).  One product with it replaces the residual, the dense solve
+// and the post sweep of that level, two grid barriers of the V-cycle fewer.
+void AmgPreconditioner::foldCoarse() {
+    if (!plan_.folded) return;
+    const int L = static_cast<int>(levels_.size());
+    const Level *f = levels_[L - 2], *c = levels_[L - 1];
+    kFoldColumns<<<f->n, kBlock, 0, ctx_.stream>>>(f->n, c->n, f->dptr, f->dcol, f->ddiag, f->dval, f->rdiag.data(),
+                                                   f->agg.data(), c->dense.data(), fold_y_.data());
+    const auto rows = [&](auto* out) {
+        kFoldLines<<<f->n, kBlock, sizeof(double) * f->npos, ctx_.stream>>>(
+            f->n, f->npos, f->t_pos.data(), f->t_row.data(), f->dptr, f->dcol, f->ddiag, f->dval, f->rdiag.data(),
+            f->agg.data(), gamma_, fold_y_.data(), f->at.data(), out);
+    };
+    if (fp32_) rows(folded32_.data());
+    else rows(folded_.data());
+    BSG_CUDA(cudaGetLastError());
+    ctx_.launches += 2;
+}
+
+int AmgPreconditioner::treePositions() const {
+    return plan_.first == 0 ? std::max(levels_.front()->npos, levels_.front()->n) : levels_.front()->n;
+}
+
+TreeView<double> AmgPreconditioner::treeView64() const {
+    return {static_cast<int>(levels_.size()), plan_.first, gamma_, omega_, d_tree_.data(), d_vl64_.data(),
+            d_tvec64_.data(), levels_.back()->dense.data(), folded_.data()};
+}
+
+TreeView<float> AmgPreconditioner::treeView32() const {
+    return {static_cast<int>(levels_.size()), plan_.first, static_cast<float>(gamma_), omega_, d_tree_.data(),
+            d_vl32_.data(), d_tvec32_.data(), dense32_.data(), folded32_.data()};
 }
 
 void AmgPreconditioner::update(const Dcsr<double>& A, bool numeric) {
@@ -549,6 +758,7 @@ void AmgPreconditioner::update(const Dcsr<double>& A, bool numeric) {
                                                                          last->dval, last->dense.data());
     ctx_.launched();
     BSG_CUDA(cudaGetLastError());
+    foldCoarse();
     // SELL-32 values for the persistent solver
     const int nn = last->n * last->n;
     if (fp32_) {
@@ -582,6 +792,7 @@ void AmgPreconditioner::uploadViews() {
                                         lv->t.data()};
     }
     d_views_.upload(views, ctx_.stream);
+    uploadTree();
     const int L = static_cast<int>(levels_.size());
     if (fp32_) {
         std::vector<VLevel<float>> v(L);
@@ -616,6 +827,28 @@ void AmgPreconditioner::uploadViews() {
         }
         d_vl64_.upload(v, ctx_.stream);
     }
+}
+
+void AmgPreconditioner::uploadTree() {
+    if (!tree_) return;
+    const int L = static_cast<int>(levels_.size());
+    std::vector<TreeLevel> t(L);
+    std::vector<double*> v64(3 * L, nullptr);
+    std::vector<float*> v32(3 * L, nullptr);
+    for (int l = plan_.first; l < L; ++l) {
+        Level* lv = levels_[l];
+        t[l] = TreeLevel{lv->n, lv->npos, lv->t_row.data(), lv->t_rank.data(), lv->t_pos.data(), lv->t_memb.data(),
+                         lv->dptr, lv->t_pcol.data(), lv->dval, lv->ddiag};
+        v64[3 * l] = lv->tb.data();
+        v64[3 * l + 1] = lv->tw.data();
+        v64[3 * l + 2] = lv->te.data();
+        v32[3 * l] = lv->tb32.data();
+        v32[3 * l + 1] = lv->tw32.data();
+        v32[3 * l + 2] = lv->te32.data();
+    }
+    d_tree_.upload(t, ctx_.stream);
+    if (fp32_) d_tvec32_.upload(v32, ctx_.stream);
+    else d_tvec64_.upload(v64, ctx_.stream);
 }
 
 SellMat<double> AmgPreconditioner::krylovMatrix() const {

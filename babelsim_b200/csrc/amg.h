@@ -14,6 +14,7 @@
 #include "linalg.h"
 #include "pcg_persistent.cuh"
 #include "pcg_sell.cuh"
+#include "pcg_tree.cuh"
 
 #include <vector>
 
@@ -45,11 +46,23 @@ public:
     double sellVcycleBytes() const;
     long long krylovEntries() const;  // padded level-0 SELL entries
 
+    // The tree numbering of the coarse levels (pcg_tree.cuh): built for one smoothing step and
+    // aggregates of at most four rows.
+    bool hasTree() const { return tree_; }
+    const TreePlan& treePlan() const { return plan_; }
+    int treePositions() const;  // entries the Krylov vectors need (rows of level 0, or its positions)
+    TreeView<double> treeView64() const;
+    TreeView<float> treeView32() const;
+
     struct Level;
 
 private:
     void buildStructure(const Dcsr<double>& A);
+    void buildTree(const std::vector<std::vector<int>>& ptr, const std::vector<std::vector<int>>& col,
+                   const std::vector<std::vector<int>>& agg);
     void uploadViews();
+    void uploadTree();
+    void foldCoarse();
     DeviceMesh& mesh_;
     Context& ctx_;
     SolverConfig cfg_;
@@ -62,6 +75,13 @@ private:
     DeviceArray<VLevel<double>> d_vl64_;
     DeviceArray<VLevel<float>> d_vl32_;
     DeviceArray<float> dense32_;
+    bool tree_ = false;
+    TreePlan plan_;
+    DeviceArray<double> fold_y_, folded_;  // foldCoarse
+    DeviceArray<float> folded32_;
+    DeviceArray<TreeLevel> d_tree_;
+    DeviceArray<double*> d_tvec64_;
+    DeviceArray<float*> d_tvec32_;
     // Damped-Jacobi weight and coarse-correction scale.  Piecewise-constant
     // aggregation under-corrects smooth error; scaling the coarse correction by
     // 1.8 (kept fixed, so the V-cycle stays a symmetric operator for CG) cut the

@@ -18,7 +18,7 @@
 namespace bsg {
 namespace {
 
-constexpr int BB = 256;  // threads per block
+constexpr int BB = 1024;  // threads per CTA, one CTA per SM
 
 // (A x)_i for the C components of row i of slice sl (lane = row within the slice).
 template <int C, class T>
@@ -55,15 +55,62 @@ __device__ __forceinline__ void sellProduct(const SellMat<T>& S, int sl, int lan
     for (int c = 0; c < C; ++c) acc[c] = (i < S.n ? d * x[C * i + c] : T(0)) + a[c];
 }
 
+// The same row split over K consecutive lanes (see sellRowSplit); every lane of the warp calls it.
+template <int C, class T>
+__device__ __forceinline__ void sellProductSplit(const SellMat<T>& S, const SplitUnit& u, int K,
+                                                 const T* __restrict__ x, T acc[C]) {
+    const int beg = S.sptr[u.s], w = (S.sptr[u.s + 1] - beg) >> 5;
+    const int* __restrict__ cp = S.col + beg + u.r;
+    const T* __restrict__ vp = S.val + beg + u.r;
+    const int i = 32 * u.s + u.r;
+    const bool own = u.q == 0 && i < S.n;  // this lane takes the diagonal
+#pragma unroll
+    for (int c = 0; c < C; ++c) acc[c] = own ? S.diag[i] * x[C * i + c] : T(0);
+    for (int k = u.q; k < w; k += K) {
+        const int j = __ldg(cp + 32 * k);
+        const T v = __ldg(vp + 32 * k);
+#pragma unroll
+        for (int c = 0; c < C; ++c) acc[c] += v * x[C * j + c];
+    }
+    for (int o = K >> 1; o > 0; o >>= 1)
+#pragma unroll
+        for (int c = 0; c < C; ++c) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
+}
+
+// f(i, (A x)_i) for every row i, one thread per row (on a cluster K lanes per row where the
+// system has fewer slices than the cluster has warps).
+template <int C, class G, class T, class F>
+__device__ __forceinline__ void productRows(const SellMat<T>& A, const Lanes& ln, const T* __restrict__ x, F f) {
+    if (kInCluster<G>) {
+        const int K = splitOf(A.nslices, ln.nwarps);
+        if (K > 1) {
+            for (int u = ln.gwarp; u < A.nslices * K; u += ln.nwarps) {
+                const SplitUnit su = splitUnit(u, K, ln.lane);
+                T acc[C];
+                sellProductSplit<C, T>(A, su, K, x, acc);
+                const int i = 32 * su.s + su.r;
+                if (su.q == 0 && i < A.n) f(i, acc);
+            }
+            return;
+        }
+    }
+    for (int sl = ln.gwarp; sl < A.nslices; sl += ln.nwarps) {
+        T acc[C];
+        sellProduct<C, T>(A, sl, ln.lane, x, acc);
+        const int i = 32 * sl + ln.lane;
+        if (i < A.n) f(i, acc);
+    }
+}
+
 // Products of vector entries are summed in FP64 whatever the vectors' type.
 template <class T>
 __device__ __forceinline__ double dd(T x) {
     return static_cast<double>(x);
 }
 
-template <int C, class T, class G>
+template <int C, class T, int BS, class G>
 __device__ void bicgBody(G& g, const BicgArgs<C, T>& a) {
-    const Lanes ln = lanes<BB>(g);
+    const Lanes ln = lanes<BS>(g);
     const SellMat<T>& A = a.A;
     const int n = A.n;
     BicgState& st = *a.st;
@@ -87,24 +134,19 @@ __device__ void bicgBody(G& g, const BicgArgs<C, T>& a) {
     double nb[2 * C];
 #pragma unroll
     for (int j = 0; j < 2 * C; ++j) nb[j] = 0.0;
-    for (int sl = ln.gwarp; sl < A.nslices; sl += ln.nwarps) {
-        T acc[C];
-        sellProduct<C, T>(A, sl, ln.lane, a.x, acc);
-        const int i = 32 * sl + ln.lane;
-        if (i < n) {
+    productRows<C, G>(A, ln, a.x, [&](int i, const T* acc) {
 #pragma unroll
-            for (int c = 0; c < C; ++c) {
-                const T bi = a.b[C * i + c], ri = bi - acc[c];
-                a.r[C * i + c] = ri;
-                a.r0[C * i + c] = ri;
-                a.p[C * i + c] = T(0);
-                a.v[C * i + c] = T(0);
-                nb[c] += dd(ri) * dd(ri);
-                nb[C + c] += dd(bi) * dd(bi);
-            }
+        for (int c = 0; c < C; ++c) {
+            const T bi = a.b[C * i + c], ri = bi - acc[c];
+            a.r[C * i + c] = ri;
+            a.r0[C * i + c] = ri;
+            a.p[C * i + c] = T(0);
+            a.v[C * i + c] = T(0);
+            nb[c] += dd(ri) * dd(ri);
+            nb[C + c] += dd(bi) * dd(bi);
         }
-    }
-    gridSum<2 * C, BB>(g, nb, a.partial, buf);
+    });
+    gridSum<2 * C, BS>(g, nb, a.partial, buf);
 #pragma unroll
     for (int c = 0; c < C; ++c) {
         rho[c] = nb[c];
@@ -149,19 +191,14 @@ __device__ void bicgBody(G& g, const BicgArgs<C, T>& a) {
         double r0v[C];
 #pragma unroll
         for (int c = 0; c < C; ++c) r0v[c] = 0.0;
-        for (int sl = ln.gwarp; sl < A.nslices; sl += ln.nwarps) {
-            T acc[C];
-            sellProduct<C, T>(A, sl, ln.lane, a.ph, acc);
-            const int i = 32 * sl + ln.lane;
-            if (i < n) {
+        productRows<C, G>(A, ln, a.ph, [&](int i, const T* acc) {
 #pragma unroll
-                for (int c = 0; c < C; ++c) {
-                    a.v[C * i + c] = acc[c];
-                    r0v[c] += dd(a.r0[C * i + c]) * dd(acc[c]);
-                }
+            for (int c = 0; c < C; ++c) {
+                a.v[C * i + c] = acc[c];
+                r0v[c] += dd(a.r0[C * i + c]) * dd(acc[c]);
             }
-        }
-        gridSum<C, BB>(g, r0v, a.partial, buf);
+        });
+        gridSum<C, BS>(g, r0v, a.partial, buf);
 #pragma unroll
         for (int c = 0; c < C; ++c) {
             if (!active(c)) continue;
@@ -183,7 +220,7 @@ __device__ void bicgBody(G& g, const BicgArgs<C, T>& a) {
                 ss[c] += dd(si) * dd(si);
             }
         }
-        gridSum<C, BB>(g, ss, a.partial, buf);
+        gridSum<C, BS>(g, ss, a.partial, buf);
 #pragma unroll
         for (int c = 0; c < C; ++c) {
             if (!active(c)) continue;
@@ -194,20 +231,15 @@ __device__ void bicgBody(G& g, const BicgArgs<C, T>& a) {
         double ts[2 * C];
 #pragma unroll
         for (int j = 0; j < 2 * C; ++j) ts[j] = 0.0;
-        for (int sl = ln.gwarp; sl < A.nslices; sl += ln.nwarps) {
-            T acc[C];
-            sellProduct<C, T>(A, sl, ln.lane, a.sh, acc);
-            const int i = 32 * sl + ln.lane;
-            if (i < n) {
+        productRows<C, G>(A, ln, a.sh, [&](int i, const T* acc) {
 #pragma unroll
-                for (int c = 0; c < C; ++c) {
-                    a.t[C * i + c] = acc[c];
-                    ts[2 * c] += dd(acc[c]) * dd(acc[c]);
-                    ts[2 * c + 1] += dd(acc[c]) * dd(a.r[C * i + c]);
-                }
+            for (int c = 0; c < C; ++c) {
+                a.t[C * i + c] = acc[c];
+                ts[2 * c] += dd(acc[c]) * dd(acc[c]);
+                ts[2 * c + 1] += dd(acc[c]) * dd(a.r[C * i + c]);
             }
-        }
-        gridSum<2 * C, BB>(g, ts, a.partial, buf);
+        });
+        gridSum<2 * C, BS>(g, ts, a.partial, buf);
 #pragma unroll
         for (int c = 0; c < C; ++c)
             if (active(c)) omega[c] = ts[2 * c] > 0.0 ? ts[2 * c + 1] / ts[2 * c] : 0.0;
@@ -233,7 +265,7 @@ __device__ void bicgBody(G& g, const BicgArgs<C, T>& a) {
                 nr[2 * c + 1] += dd(a.r0[C * i + c]) * dd(ri);
             }
         }
-        gridSum<2 * C, BB>(g, nr, a.partial, buf);
+        gridSum<2 * C, BS>(g, nr, a.partial, buf);
 #pragma unroll
         for (int c = 0; c < C; ++c) {
             if (done[c] == 3) { done[c] = 1; iters[c] += 1; continue; }
@@ -252,19 +284,14 @@ __device__ void bicgBody(G& g, const BicgArgs<C, T>& a) {
 #pragma unroll
     for (int c = 0; c < C; ++c) fr[c] = 0.0;
     g.sync();
-    for (int sl = ln.gwarp; sl < A.nslices; sl += ln.nwarps) {
-        T acc[C];
-        sellProduct<C, T>(A, sl, ln.lane, a.x, acc);
-        const int i = 32 * sl + ln.lane;
-        if (i < n) {
+    productRows<C, G>(A, ln, a.x, [&](int i, const T* acc) {
 #pragma unroll
-            for (int c = 0; c < C; ++c) {
-                const T ri = a.b[C * i + c] - acc[c];
-                fr[c] += dd(ri) * dd(ri);
-            }
+        for (int c = 0; c < C; ++c) {
+            const T ri = a.b[C * i + c] - acc[c];
+            fr[c] += dd(ri) * dd(ri);
         }
-    }
-    gridSum<C, BB>(g, fr, a.partial, buf);
+    });
+    gridSum<C, BS>(g, fr, a.partial, buf);
     if (g.rank() == 0 && threadIdx.x == 0) {
 #pragma unroll
         for (int c = 0; c < C; ++c) {
@@ -276,94 +303,87 @@ __device__ void bicgBody(G& g, const BicgArgs<C, T>& a) {
     }
 }
 
-// Whole-grid kernel at 4 blocks per SM (64 registers, no spills); the batched kernel keeps
-// 3 (80 registers).
-#ifndef BSG_BICG_MIN_BLOCKS
-#define BSG_BICG_MIN_BLOCKS 4
-#endif
 template <int C, class T>
-__global__ void __launch_bounds__(BB, BSG_BICG_MIN_BLOCKS) kBicgSell(BicgArgs<C, T> a, SegmentBarrier* bar) {
+__global__ void __launch_bounds__(BB, 1) kBicgSell(const __grid_constant__ BicgArgs<C, T> a, SegmentBarrier* bar) {
     GridGroup g{bar};
-    bicgBody<C, T>(g, a);
+    bicgBody<C, T, BB>(g, a);
 }
 
+// Up to kBatchArgs systems as one kernel argument (constant bank: no registers for pointers).
+constexpr int kBatchArgs = 32;
 template <int C>
-__global__ void __launch_bounds__(BB, 3)
-    kBicgSellBatch(const BicgArgs<C>* __restrict__ segs, const int* __restrict__ cta_begin, int nsegs,
-                   SegmentBarrier* bars) {
-    int lo = 0, hi = nsegs - 1;  // the system whose CTA range holds this block
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (cta_begin[mid] <= static_cast<int>(blockIdx.x)) lo = mid;
-        else hi = mid - 1;
-    }
-    SegmentGroup g{cta_begin[lo], cta_begin[lo + 1] - cta_begin[lo], bars + lo};
-    const BicgArgs<C> a = segs[lo];
-    bicgBody<C, double>(g, a);
+struct BicgArgsBlock {
+    BicgArgs<C> a[kBatchArgs];
+    int begin[kBatchArgs + 1];  // CTA ranges
+    int count;
+};
+
+// A batch: CTAs [begin[s], begin[s+1]) solve system s.
+template <int C>
+__global__ void __launch_bounds__(BB, 1)
+    kBicgSellBatch(const __grid_constant__ BicgArgsBlock<C> batch, SegmentBarrier* bars) {
+    int s = 0;  // the system whose CTA range holds this block
+    while (s + 1 < batch.count && batch.begin[s + 1] <= static_cast<int>(blockIdx.x)) ++s;
+    SegmentGroup g{batch.begin[s], batch.begin[s + 1] - batch.begin[s], bars + s};
+    bicgBody<C, double, BB>(g, batch.a[s]);
 }
+
+// A small system on one cluster.
+template <int C, class T>
+__global__ void __launch_bounds__(BB, 1) kBicgCluster(const __grid_constant__ BicgArgs<C, T> a) {
+    ClusterGroup g;
+    g.sync();  // every CTA's shared memory is live
+    bicgBody<C, T, BB>(g, a);
+}
+// Largest system one cluster solves faster than the grid (barrier 0.3 us instead of 1.3, but 16 SMs'
+// gathers).  Three right-hand sides, ms per solve, cluster / grid: 1000-cell Voronoi cube 0.57 / 0.91,
+// 4096 cells 0.65 / 0.99, 13824 cells 0.85 / 1.05, 21952 cells 1.44 / 1.08; 2D cavities of 16384
+// cells 0.17 / 0.24, 40000 cells 0.34 / 0.25.
+constexpr int kClusterRows = 16384;
 
 }  // namespace
 
-int bicgstabGrid(Context& ctx) {
-    static int per_sm = -1;
-    if (per_sm < 0) {
-        BSG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kBicgSell<3, double>, BB, 0));
-        int b = 0;
-        BSG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kBicgSellBatch<3>, BB, 0));
-        per_sm = std::min(per_sm, b);
-        if (per_sm <= 0) fail(kCuda, "persistent BiCGStab kernel cannot be resident");
-    }
-    return ctx.sm_count * std::min(per_sm, 4);
-}
-
-namespace {
-// Resident CTAs of one whole-grid launch of kBicgSell<C, T>.
 template <int C, class T>
-int singleGrid(Context& ctx) {
-    static int per_sm = -1;
-    if (per_sm < 0) {
-        BSG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kBicgSell<C, T>, BB, 0));
-        if (per_sm <= 0) fail(kCuda, "persistent BiCGStab kernel cannot be resident");
-    }
-    return ctx.sm_count * std::min(per_sm, 4);
-}
-}  // namespace
-
-template <int C, class T>
-void launchBicgstab(Context& ctx, const BicgArgs<C, T>& in) {
-    BicgArgs<C, T> args = in;
-    SegmentBarrier* bar = ctx.grid_barrier;
-    const int grid = singleGrid<C, T>(ctx);
-    resetBarriers(ctx, bar, 1, grid);
-    void* params[] = {&args, &bar};
+void launchBicgstab(Context& ctx, const BicgArgs<C, T>& args) {
     BSG_PROFILE(ctx, sizeof(T) == 4 ? "bicgstab3_persistent_fp32" : "bicgstab3_persistent");
+    if (args.A.n <= kClusterRows) {
+        launchCluster<kBicgCluster<C, T>>(ctx, 1, BB, 0, 0, args);
+        return;
+    }
+    SegmentBarrier* bar = ctx.grid_barrier;
+    const int grid = ctx.sm_count;
+    resetBarriers(ctx, bar, 1, grid);
+    BicgArgs<C, T> a = args;
+    void* params[] = {&a, &bar};
     BSG_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(kBicgSell<C, T>), grid, BB, params, 0, ctx.stream));
     ctx.launched();
 }
 
 template <int C>
 void launchBicgstabBatch(Context& ctx, BicgBatch<C>& batch) {
-    const int nsegs = static_cast<int>(batch.args.size());
-    if (nsegs == 0) return;
-    if (static_cast<int>(batch.cta_begin.size()) != nsegs + 1 || batch.cta_begin.front() != 0)
-        fail(kArgument, "batched BiCGStab: CTA table does not match the systems");
-    for (int k = 0; k < nsegs; ++k)
-        if (batch.cta_begin[k + 1] <= batch.cta_begin[k]) fail(kArgument, "batched BiCGStab: a system without CTAs");
-    const int total = batch.cta_begin.back();
-    if (total > bicgstabGrid(ctx)) fail(kArgument, "batched BiCGStab: CTA allotment exceeds the resident grid");
-    batch.d_args.upload(batch.args, ctx.stream);
-    batch.d_cta.upload(batch.cta_begin, ctx.stream);
-    batch.d_bars.resize(nsegs);
-    resetBarriers(ctx, batch.d_bars.data(), nsegs, total, batch.cta_begin.data());
-    const BicgArgs<C>* segs = batch.d_args.data();
-    const int* cta = batch.d_cta.data();
-    SegmentBarrier* bars = batch.d_bars.data();
-    int ns = nsegs;
-    void* params[] = {&segs, &cta, &ns, &bars};
     BSG_PROFILE(ctx, "bicgstab3_persistent_batch");
-    BSG_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(kBicgSellBatch<C>), total, BB, params, 0,
-                                         ctx.stream));
-    ctx.launched();
+    const std::size_t count = batch.args.size();
+    if (count == 0) return;
+    const std::size_t chunk = std::min(kBatchArgs, ctx.sm_count);
+    batch.d_bars.resize(std::max(batch.d_bars.size(), count));
+    for (std::size_t k0 = 0; k0 < count; k0 += chunk) {
+        BicgArgsBlock<C> block{};
+        block.count = static_cast<int>(std::min(chunk, count - k0));
+        std::vector<long long> slices(block.count);
+        for (int i = 0; i < block.count; ++i) {
+            block.a[i] = batch.args[k0 + i];
+            slices[i] = block.a[i].A.nslices;
+        }
+        const std::vector<int> begin = allotCtas(slices, BB / 32, ctx.sm_count);
+        std::copy(begin.begin(), begin.end(), block.begin);
+        SegmentBarrier* bars = batch.d_bars.data() + k0;
+        resetBarriers(ctx, bars, block.count, begin.back(), block.begin);
+        void* params[] = {&block, &bars};
+        BSG_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(kBicgSellBatch<C>), begin.back(), BB, params, 0,
+                                             ctx.stream));
+        ctx.launched();
+    }
+    batch.bars_used = static_cast<int>(count);
 }
 
 template void launchBicgstab<3, double>(Context&, const BicgArgs<3, double>&);

@@ -41,23 +41,22 @@ struct BicgArgs {
     const T* b;              // C-interleaved right-hand sides
     T* x;                    // C-interleaved initial guess / solution
     T *r, *r0, *p, *v, *ph, *sh, *t;  // C * n each
-    double* partial;         // 2 * ctas * 2C doubles
+    double* partial;         // 2 * ctas * kSumValues doubles
     BicgState* st;
 };
 
 template <int C>
 struct BicgBatch {
     std::vector<BicgArgs<C>> args;
-    std::vector<int> cta_begin;
-    DeviceArray<BicgArgs<C>> d_args;
-    DeviceArray<int> d_cta;
     DeviceArray<SegmentBarrier> d_bars;
+    int bars_used = 0;  // barriers of the last launch, for its error report
 };
 
-// Resident CTAs of the persistent BiCGStab kernel (the grid of one solve).
-int bicgstabGrid(Context& ctx);
+// One system, on one thread-block cluster when it is small, else on the whole grid.
 template <int C, class T>
 void launchBicgstab(Context& ctx, const BicgArgs<C, T>& args);
+// Independent systems side by side on CTA ranges of one cooperative launch (several when they
+// outnumber its argument block).
 template <int C>
 void launchBicgstabBatch(Context& ctx, BicgBatch<C>& batch);
 

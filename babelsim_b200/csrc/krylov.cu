@@ -9,6 +9,7 @@
 #include "amg.h"
 #include "bicgstab_sell.cuh"
 #include "pcg_sell.cuh"
+#include "pcg_tree.cuh"
 #include "sell.cuh"
 #include "bsg_device.cuh"
 #include "linalg.h"
@@ -531,7 +532,9 @@ struct KrylovSolver::Impl {
     DeviceArray<BicgState> bst;    // state of the persistent BiCGStab
     DeviceArray<unsigned> ticket;  // arrivals of the current reduction (reduceThenFinish), zero between launches
     DeviceArray<PcgState> pst;
-    DeviceArray<float> r32, s32, z32, p32a, p32b, q32, d32;  // FP32 inner solve of the refined path
+    DeviceArray<float> r32, s32, z32, p32a, p32b, q32, d32, x32;  // FP32 inner solve of the refined path
+    DeviceArray<double2> pair[4];  // the tree solver's paired vectors (pcg_tree.cuh)
+    DeviceArray<float2> pair32[4];
     // FP32 inner BiCGStab of the refined path: matrix copy (SELL values, diagonal) and
     // the C-interleaved right-hand side, correction and Krylov vectors
     DeviceArray<float> bval32, bdiag32, bb32, bx32, br32, br032, bp32, bv32, bph32, bsh32, bt32;
@@ -583,6 +586,11 @@ struct KrylovSolver::Impl {
     int grid(int n) const {
         const long long g = (static_cast<long long>(n) + kBlock - 1) / kBlock;
         return static_cast<int>(std::max<long long>(1, std::min<long long>(g, 4LL * ctx.sm_count)));
+    }
+    void ensureTree(std::size_t n) {
+        ensure(n);
+        for (DeviceArray<double2>& a : pair)
+            if (a.size() < n) a.resize(n);
     }
     void ensure(std::size_t n) {
         for (DeviceArray<double>* a : {&r, &z, &p, &q, &r0, &v, &ph, &sh, &t, &tmp})
@@ -670,8 +678,17 @@ SolveOutcome KrylovSolver::solveRefined(const Dcsr<double>& A, const SolverConfi
     Context& ctx = m.ctx;
     const int n = A.n;
     m.ensure(n);
-    for (DeviceArray<float>* a : {&m.r32, &m.s32, &m.z32, &m.p32a, &m.p32b, &m.q32, &m.d32})
-        if (a->size() < static_cast<std::size_t>(n)) a->resize(n);
+    const std::size_t entries = amg->hasTree() ? amg->treePositions() : n;
+    for (DeviceArray<float>* a : {&m.r32, &m.s32, &m.q32, &m.d32})
+        if (a->size() < entries) a->resize(entries);
+    if (amg->hasTree()) {
+        if (m.x32.size() < entries) m.x32.resize(entries);
+        for (DeviceArray<float2>& a : m.pair32)
+            if (a.size() < entries) a.resize(entries);
+    } else {
+        for (DeviceArray<float>* a : {&m.z32, &m.p32a, &m.p32b})
+            if (a->size() < entries) a->resize(entries);
+    }
     if (m.pst.size() < 1) m.pst.resize(1);
     SolveOutcome out;
     if (!cfg.warm_start) BSG_CUDA(cudaMemsetAsync(x, 0, sizeof(double) * n, ctx.stream));
@@ -695,10 +712,18 @@ SolveOutcome KrylovSolver::solveRefined(const Dcsr<double>& A, const SolverConfi
         h.atol = cfg.atol;
         h.rtol = cfg.rtol;
         BSG_CUDA(cudaMemcpyAsync(m.pst.data(), &h, sizeof(h), cudaMemcpyHostToDevice, ctx.stream));
-        SellPcgArgs<float, float> args{amg->krylovMatrix32(), amg->sellView32(), m.r32.data(), m.d32.data(),
-                                       m.s32.data(), m.z32.data(), m.p32a.data(), m.p32b.data(), m.q32.data(),
-                                       m.partial.data(), m.pst.data(), PhaseLog{}};
-        launchSellPcg(ctx, args);
+        if (amg->hasTree()) {
+            launchTreePcg<float, float>(ctx, amg->treePlan(),
+                                        {amg->krylovMatrix32(), amg->treeView32(), 0, n, m.r32.data(), m.d32.data(),
+                                         m.s32.data(), m.q32.data(), m.x32.data(), m.pair32[0].data(),
+                                         m.pair32[1].data(), m.pair32[2].data(), m.pair32[3].data(), m.partial.data(),
+                                         m.pst.data(), PhaseLog{}});
+        } else {
+            SellPcgArgs<float, float> args{amg->krylovMatrix32(), amg->sellView32(), m.r32.data(), m.d32.data(),
+                                           m.s32.data(), m.z32.data(), m.p32a.data(), m.p32b.data(), m.q32.data(),
+                                           m.partial.data(), m.pst.data(), PhaseLog{}};
+            launchSellPcg(ctx, args);
+        }
         BSG_CUDA(cudaMemcpyAsync(ctx.pinned, m.pst.data(), sizeof(PcgState), cudaMemcpyDeviceToHost, ctx.stream));
         kAddCorrection<<<g, 256, 0, ctx.stream>>>(n, x, m.d32.data());
         ctx.launched();
@@ -735,7 +760,8 @@ SolveOutcome KrylovSolver::solvePersistent(const Dcsr<double>& A, const SolverCo
     Context& ctx = m.ctx;
     const int n = A.n;
     if (cfg.precision == 1 && amg && amg->fp32VCycle()) return solveRefined(A, cfg, amg, b, x);
-    m.ensure(n);
+    if (amg && amg->hasTree()) m.ensureTree(amg->treePositions());
+    else m.ensure(n);
     if (m.pst.size() < 1) m.pst.resize(1);
     const AmgView<double> view = amg ? amg->deviceView() : AmgView<double>{};
     PcgState h{};
@@ -749,8 +775,18 @@ SolveOutcome KrylovSolver::solvePersistent(const Dcsr<double>& A, const SolverCo
     int used = 0;
     for (int attempt = 0; attempt < 3; ++attempt) {
         BSG_CUDA(cudaMemcpyAsync(m.pst.data(), &h, sizeof(h), cudaMemcpyHostToDevice, ctx.stream));
-        if (amg && amg->fp32VCycle()) {
-            // FP64 Krylov vectors and products, FP32 V-cycle, flexible beta
+        if (amg && amg->hasTree()) {
+            // FP64 Krylov vectors and products; an FP32 V-cycle takes the flexible beta
+            const auto solve = [&](auto view, int flexible) {
+                using TV = std::decay_t<decltype(view.gamma)>;
+                launchTreePcg<double, TV>(ctx, amg->treePlan(),
+                                          {amg->krylovMatrix(), view, 0, n, b, x, m.r.data(), m.q.data(),
+                                           m.ph.data(), m.pair[0].data(), m.pair[1].data(), m.pair[2].data(),
+                                           m.pair[3].data(), m.partial.data(), m.pst.data(), PhaseLog{}, flexible});
+            };
+            if (amg->fp32VCycle()) solve(amg->treeView32(), 1);
+            else solve(amg->treeView64(), 0);
+        } else if (amg && amg->fp32VCycle()) {
             SellPcgArgs<double, float> args{amg->krylovMatrix(), amg->sellView32(), b, x, m.r.data(), m.z.data(),
                                             m.p.data(), m.v.data(), m.q.data(), m.partial.data(), m.pst.data(),
                                             PhaseLog{}, 1, m.t.data()};
@@ -920,16 +956,13 @@ SolveOutcome KrylovSolver::solveScalar(const Dcsr<double>& A, const SolverConfig
     return out;
 }
 
-namespace {
-// CTAs for each system of a batch: about two level-0 slices per warp, at least one CTA,
-// scaled down in proportion (keeping one each) when the batch exceeds the resident grid.
-std::vector<int> allotCtas(const std::vector<long long>& slices, int capacity) {
+std::vector<int> allotCtas(const std::vector<long long>& slices, int slices_per_cta, int capacity) {
     const int k = static_cast<int>(slices.size());
     if (k > capacity) fail(kArgument, "batch larger than the resident grid: split it");
     std::vector<int> c(k);
     long long want = 0, total = 0;
     for (int i = 0; i < k; ++i) {
-        c[i] = static_cast<int>(std::max<long long>(1, (slices[i] + 15) / 16));
+        c[i] = static_cast<int>(std::max<long long>(1, (slices[i] + slices_per_cta - 1) / slices_per_cta));
         want += c[i];
         total += slices[i];
     }
@@ -946,7 +979,6 @@ std::vector<int> allotCtas(const std::vector<long long>& slices, int capacity) {
     for (int i = 0; i < k; ++i) begin[i + 1] = begin[i] + c[i];
     return begin;
 }
-}  // namespace
 
 void KrylovSolver::solveBatch(Context& ctx, std::vector<BatchSolve>& items) {
     const int K = static_cast<int>(items.size());
@@ -964,7 +996,8 @@ void KrylovSolver::solveBatch(Context& ctx, std::vector<BatchSolve>& items) {
             fail(kArgument, "batched solves take CG with the AMG preconditioner in FP64 or with an FP32 V-cycle");
         Impl& m = *it.solver->impl_;
         if (&m.ctx != &ctx) fail(kArgument, "batched solves must share one context");
-        m.ensure(it.A.n);
+        if (it.amg->hasTree()) m.ensureTree(it.amg->treePositions());
+        else m.ensure(it.A.n);
         if (m.pst.size() < 1) m.pst.resize(1);
         t[k].h.target2 = -1.0;
         t[k].h.warm = it.cfg.warm_start ? 1 : 0;
@@ -977,7 +1010,8 @@ void KrylovSolver::solveBatch(Context& ctx, std::vector<BatchSolve>& items) {
     if (norms.size() < static_cast<std::size_t>(K)) norms.resize(K);
     std::vector<PcgState> states(K);
     std::vector<double> nrm(K);
-    const int capacity = sellBatchCapacity(ctx);
+    TreeBatch<double, double> tree64;
+    TreeBatch<double, float> tree32;
     BatchLaunch<double, double> batch64;
     BatchLaunch<double, float> batch32;
     for (int attempt = 0; attempt < 3; ++attempt) {
@@ -985,43 +1019,53 @@ void KrylovSolver::solveBatch(Context& ctx, std::vector<BatchSolve>& items) {
         for (int k = 0; k < K; ++k)
             if (!t[k].done) active.push_back(k);
         if (active.empty()) break;
-        // one launch per V-cycle precision
-        for (int fp32 = 0; fp32 < 2; ++fp32) {
-            std::vector<int> group;
-            std::vector<long long> slices;
-            for (int k : active)
-                if (items[k].amg->fp32VCycle() == (fp32 == 1)) {
-                    group.push_back(k);
-                    slices.push_back(items[k].amg->krylovMatrix().nslices);
-                }
-            if (group.empty()) continue;
-            for (int k : group)
-                BSG_CUDA(cudaMemcpyAsync(items[k].solver->impl_->pst.data(), &t[k].h, sizeof(PcgState),
-                                         cudaMemcpyHostToDevice, ctx.stream));
-            if (fp32 == 0) {
-                batch64.args.clear();
-                for (int k : group) {
-                    Impl& m = *items[k].solver->impl_;
-                    batch64.args.push_back({items[k].amg->krylovMatrix(), items[k].amg->sellView64(), items[k].b,
-                                            items[k].x, m.r.data(), m.z.data(), m.p.data(), m.v.data(), m.q.data(),
-                                            m.partial.data(), m.pst.data(), PhaseLog{}, 0, m.t.data()});
-                }
-                batch64.cta_begin = allotCtas(slices, capacity);
-                launchSellPcgBatch(ctx, batch64);
+        // one launch per V-cycle precision: tree-numbered hierarchies (the default cycle) on the
+        // kernel with on-chip coarse levels, the others on CTA ranges of the streaming one
+        for (int k : active)
+            BSG_CUDA(cudaMemcpyAsync(items[k].solver->impl_->pst.data(), &t[k].h, sizeof(PcgState),
+                                     cudaMemcpyHostToDevice, ctx.stream));
+        tree64.args.clear();
+        tree32.args.clear();
+        batch64.args.clear();
+        batch32.args.clear();
+        std::vector<long long> slices64, slices32;
+        const auto addTree = [&](auto& batch, auto view, int k, int flexible) {
+            BatchSolve& it = items[k];
+            Impl& m = *it.solver->impl_;
+            batch.args.push_back({it.amg->krylovMatrix(), view, 0, it.A.n, it.b, it.x, m.r.data(), m.q.data(),
+                                  m.ph.data(), m.pair[0].data(), m.pair[1].data(), m.pair[2].data(), m.pair[3].data(),
+                                  m.partial.data(), m.pst.data(), PhaseLog{}, flexible});
+            batch.plans.push_back(&it.amg->treePlan());
+            batch.slices.push_back(it.amg->krylovMatrix().nslices);
+        };
+        const auto addSell = [&](auto& batch, auto view, int k, int flexible) {
+            BatchSolve& it = items[k];
+            Impl& m = *it.solver->impl_;
+            batch.args.push_back({it.amg->krylovMatrix(), view, it.b, it.x, m.r.data(), m.z.data(), m.p.data(),
+                                  m.v.data(), m.q.data(), m.partial.data(), m.pst.data(), PhaseLog{}, flexible,
+                                  m.t.data()});
+        };
+        tree64.plans.clear();
+        tree32.plans.clear();
+        tree64.slices.clear();
+        tree32.slices.clear();
+        for (int k : active) {
+            AmgPreconditioner& amg = *items[k].amg;
+            if (amg.hasTree()) {
+                if (amg.fp32VCycle()) addTree(tree32, amg.treeView32(), k, 1);
+                else addTree(tree64, amg.treeView64(), k, 0);
+            } else if (amg.fp32VCycle()) {
+                addSell(batch32, amg.sellView32(), k, 1);
+                slices32.push_back(amg.krylovMatrix().nslices);
             } else {
-                batch32.args.clear();
-                for (int k : group) {
-                    Impl& m = *items[k].solver->impl_;
-                    SellPcgArgs<double, float> a{items[k].amg->krylovMatrix(), items[k].amg->sellView32(),
-                                                 items[k].b, items[k].x, m.r.data(), m.z.data(), m.p.data(),
-                                                 m.v.data(), m.q.data(), m.partial.data(), m.pst.data(), PhaseLog{}, 1,
-                                                 m.t.data()};
-                    batch32.args.push_back(a);
-                }
-                batch32.cta_begin = allotCtas(slices, capacity);
-                launchSellPcgBatch(ctx, batch32);
+                addSell(batch64, amg.sellView64(), k, 0);
+                slices64.push_back(amg.krylovMatrix().nslices);
             }
         }
+        if (!tree64.args.empty()) launchTreePcgBatch(ctx, tree64);
+        if (!tree32.args.empty()) launchTreePcgBatch(ctx, tree32);
+        launchSellPcgBatch(ctx, batch64, slices64);
+        launchSellPcgBatch(ctx, batch32, slices32);
         // solve states and true residuals of every system of this attempt, read back together
         for (int k : active) {
             BatchSolve& it = items[k];
@@ -1041,8 +1085,10 @@ void KrylovSolver::solveBatch(Context& ctx, std::vector<BatchSolve>& items) {
             const PcgState& r = states[k];
             if (r.status == 3)
                 fail(kCuda, "batched persistent PCG: a segment barrier wait ran past its bound" +
-                                barrierReport(batch64.d_bars.data(), static_cast<int>(batch64.args.size())) +
-                                barrierReport(batch32.d_bars.data(), static_cast<int>(batch32.args.size())));
+                                barrierReport(tree64.d_bars.data(), tree64.bars_used) +
+                                barrierReport(tree32.d_bars.data(), tree32.bars_used) +
+                                barrierReport(batch64.d_bars.data(), static_cast<int>(batch64.d_bars.size())) +
+                                barrierReport(batch32.d_bars.data(), static_cast<int>(batch32.d_bars.size())));
             ++it.out.checks;
             if (attempt == 0) {
                 it.out.initial = std::sqrt(r.rr0);
@@ -1120,17 +1166,14 @@ void KrylovSolver::solveVector3Batch(Context& ctx, std::vector<BicgItem>& items,
         for (int k = 0; k < K; ++k)
             if (!(t[k].finished[0] && t[k].finished[1] && t[k].finished[2])) active.push_back(k);
         if (active.empty()) break;
-        std::vector<long long> slices;
         batch.args.clear();
         for (int k : active) {
             Impl& m = *items[k].solver->impl_;
             BSG_CUDA(cudaMemcpyAsync(m.bst.data(), &t[k].h, sizeof(BicgState), cudaMemcpyHostToDevice, ctx.stream));
             batch.args.push_back({sell[k], items[k].b, items[k].x, m.r.data(), m.r0.data(), m.p.data(), m.v.data(),
                                   m.ph.data(), m.sh.data(), m.t.data(), m.partial.data(), m.bst.data()});
-            slices.push_back(sell[k].nslices);
         }
         if (batched) {
-            batch.cta_begin = allotCtas(slices, bicgstabGrid(ctx));
             launchBicgstabBatch<3>(ctx, batch);
         } else {
             for (const auto& a : batch.args) launchBicgstab<3, double>(ctx, a);
@@ -1145,7 +1188,7 @@ void KrylovSolver::solveVector3Batch(Context& ctx, std::vector<BicgItem>& items,
             const BicgState& r = res[k];
             if (r.status == 3)
                 fail(kCuda, "persistent BiCGStab: a barrier wait ran past its bound" +
-                                (batched ? barrierReport(batch.d_bars.data(), static_cast<int>(batch.args.size()))
+                                (batched ? barrierReport(batch.d_bars.data(), batch.bars_used)
                                          : barrierReport(ctx.grid_barrier)));
             for (int c = 0; c < 3; ++c) {
                 if (tr.finished[c]) continue;

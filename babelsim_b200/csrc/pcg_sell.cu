@@ -8,20 +8,14 @@
 namespace bsg {
 namespace {
 
-#ifndef BSG_SELL_SB
-#define BSG_SELL_SB 256
-#endif
-constexpr int SB = BSG_SELL_SB;  // threads per block
-// Minimum resident blocks per SM the register budget must allow.  The single-system
-// kernels: 4 (64 registers) measured faster than 3 (80) on the 1M-cell cavity (FP64:
-// 2 %; FP32 V-cycle: 42.4 -> 40.3 ms per outer iteration; FP32 inner PCG: 49.6 ->
-// 45.5), 2 (128) slower.  The batched kernel keeps 3: at 64 registers it spills heavily.
-#ifndef BSG_SELL_MIN_BLOCKS
-#define BSG_SELL_MIN_BLOCKS 4
-#endif
-#ifndef BSG_SELL_BATCH_MIN_BLOCKS
-#define BSG_SELL_BATCH_MIN_BLOCKS 3
-#endif
+// This kernel serves the hierarchies pcg_tree.cu does not take (two smoothing steps, aggregates
+// of more than four rows).  One system: one CTA of 1024 threads per SM, since the grid barrier costs
+// by its arrivals (592 CTAs of 256 threads 2.1 us, 148 of 1024 1.3; two smoothing steps, 33k-cell
+// Voronoi cube: 7.30 against 6.77 ms per three solves).  A batch: CTAs of 256 threads, three per
+// SM, because its systems share the SMs in fine steps (eight cavities, 9.5 against 10.5 ms).
+constexpr int SB = 1024;
+constexpr int SBB = 256;
+constexpr int kBatchBlocks = 3;
 // Levels of at most this many rows compute their residual and its restriction in one
 // pass (coarse row by coarse row, kRowLanes lanes per member row), one barrier fewer.
 // On the 1M-cell solve (us per CG iteration, residual + restriction): 16k rows 11.8 ->
@@ -35,9 +29,6 @@ constexpr int kRestrictRows = BSG_RESTRICT_ROWS;
 #define BSG_ROW_LANES 8
 #endif
 constexpr int kRowLanes = BSG_ROW_LANES;
-template <class TK, class TV>
-constexpr int kSellMinBlocks = BSG_SELL_MIN_BLOCKS;
-
 __device__ __forceinline__ void mark(const PhaseLog& log, int id) {
     if (log.entries && blockIdx.x == 0 && threadIdx.x == 0) {
         const int k = *log.count;
@@ -73,27 +64,10 @@ __device__ __forceinline__ double emitRow(const VCycleView<TV>& V, const VLevel<
 
 // z = M r with M the V-cycle; returns this thread's share of r.z.  Level 0's b
 // and w were written by the phase that produced r.
-// Lanes per row on a level: the largest power of two (at most 32) that still
-// gives every (slice, lane-group) unit its own warp; 1 on the fine levels.
-__device__ __forceinline__ int splitOf(int nslices, int nwarps) {
-    int K = 1;
-    while (K < 32 && static_cast<long long>(nslices) * K * 2 <= nwarps) K *= 2;
-    return K;
-}
-
-// Unit u of a split sweep: slice s, the row r within it and this lane's part q.
-struct SplitUnit {
-    int s, r, q;
-};
-__device__ __forceinline__ SplitUnit splitUnit(int u, int K, int lane) {
-    const int rows = 32 / K;
-    return {u / K, (u % K) * rows + lane / K, lane % K};
-}
-
-template <class TK, class TV, class G>
+template <class TK, class TV, int BS, class G>
 __device__ double vcycle(G& g, const VCycleView<TV>& V, const TK* r, TK* z, const PhaseLog& log,
                          bool level0_residual_done = false) {
-    const Lanes c = lanes<SB>(g);
+    const Lanes c = lanes<BS>(g);
     const int L = V.levels;
     // ---- down
     for (int l = 0; l < L - 1; ++l) {
@@ -295,9 +269,9 @@ __device__ __forceinline__ void seedLevel0(const VLevel<TV>& f0, int i, TK ri) {
     f0.w[i] = f0.rd[i] * rv;
 }
 
-template <class TK, class TV, class G>
+template <class TK, class TV, int BS, class G>
 __device__ void pcgBody(G& g, const SellPcgArgs<TK, TV>& a) {
-    const Lanes c = lanes<SB>(g);
+    const Lanes c = lanes<BS>(g);
     const SellMat<TK>& A = a.A;
     const int n = A.n;
     int buf = 0;
@@ -326,7 +300,7 @@ __device__ void pcgBody(G& g, const SellPcgArgs<TK, TV>& a) {
             v[1] += static_cast<double>(a.b[i]) * static_cast<double>(a.b[i]);
         }
     }
-    gridSum<2, SB>(g, v, a.partial, buf);
+    gridSum<2, BS>(g, v, a.partial, buf);
     mark(a.log, 1);
     double target2 = target2_in;
     if (target2 < 0.0) {
@@ -348,12 +322,12 @@ __device__ void pcgBody(G& g, const SellPcgArgs<TK, TV>& a) {
         if (g.rank() == 0 && threadIdx.x == 0) st.status = 0;
         return;
     }
-    double w[1] = {vcycle<TK, TV>(g, a.V, a.r, a.z, a.log)};
+    double w[1] = {vcycle<TK, TV, BS>(g, a.V, a.r, a.z, a.log)};
     if (g.aborted()) {
         if (g.rank() == 0 && threadIdx.x == 0) st.status = 3;
         return;
     }
-    gridSum<1, SB>(g, w, a.partial, buf);
+    gridSum<1, BS>(g, w, a.partial, buf);
     mark(a.log, 4);
     double rz = w[0];
     double beta = 0.0;
@@ -385,7 +359,7 @@ __device__ void pcgBody(G& g, const SellPcgArgs<TK, TV>& a) {
                 pq[0] += static_cast<double>(pi) * static_cast<double>(qi);
             }
         }
-        gridSum<1, SB>(g, pq, a.partial, buf);
+        gridSum<1, BS>(g, pq, a.partial, buf);
         mark(a.log, 2);
         if (!(fabs(pq[0]) > 0.0) || !isfinite(pq[0])) { status = 2; break; }
         const double alpha = rz / pq[0];
@@ -424,7 +398,7 @@ __device__ void pcgBody(G& g, const SellPcgArgs<TK, TV>& a) {
                 if (a.flexible) nr[1] += static_cast<double>(ri) * static_cast<double>(a.z[i]);  // r_new . z_old
             }
         }
-        gridSum<2, SB>(g, nr, a.partial, buf);
+        gridSum<2, BS>(g, nr, a.partial, buf);
         mark(a.log, 3);
         rr = nr[0];
         const double rz_old_new = nr[1];
@@ -432,8 +406,8 @@ __device__ void pcgBody(G& g, const SellPcgArgs<TK, TV>& a) {
         if (!isfinite(rr)) { status = 2; break; }
         if (rr <= target2) { status = 0; break; }
         if (it >= max_iterations) break;
-        double zr[1] = {vcycle<TK, TV>(g, a.V, fuse ? rnext : a.r, a.z, a.log, fuse)};
-        gridSum<1, SB>(g, zr, a.partial, buf);
+        double zr[1] = {vcycle<TK, TV, BS>(g, a.V, fuse ? rnext : a.r, a.z, a.log, fuse)};
+        gridSum<1, BS>(g, zr, a.partial, buf);
         mark(a.log, 4);
         beta = a.flexible ? (zr[0] - rz_old_new) / rz : zr[0] / rz;
         rz = zr[0];
@@ -454,15 +428,15 @@ __device__ void pcgBody(G& g, const SellPcgArgs<TK, TV>& a) {
 }
 
 template <class TK, class TV>
-__global__ void __launch_bounds__(SB, (kSellMinBlocks<TK, TV>)) kPcgSell(SellPcgArgs<TK, TV> a, SegmentBarrier* bar) {
+__global__ void __launch_bounds__(SB, 1) kPcgSell(SellPcgArgs<TK, TV> a, SegmentBarrier* bar) {
     GridGroup g{bar};
-    pcgBody<TK, TV>(g, a);
+    pcgBody<TK, TV, SB>(g, a);
 }
 
 // A batch: CTAs [cta_begin[s], cta_begin[s+1]) solve system s with its own
 // arguments, barriers and reductions, independently of the other systems.
 template <class TK, class TV>
-__global__ void __launch_bounds__(SB, BSG_SELL_BATCH_MIN_BLOCKS)
+__global__ void __launch_bounds__(SBB, kBatchBlocks)
     kPcgSellBatch(const SellPcgArgs<TK, TV>* __restrict__ segs, const int* __restrict__ cta_begin, int nsegs,
                   SegmentBarrier* bars) {
     int lo = 0, hi = nsegs - 1;  // the segment whose CTA range holds this block
@@ -473,7 +447,7 @@ __global__ void __launch_bounds__(SB, BSG_SELL_BATCH_MIN_BLOCKS)
     }
     SegmentGroup g{cta_begin[lo], cta_begin[lo + 1] - cta_begin[lo], bars + lo};
     const SellPcgArgs<TK, TV> a = segs[lo];
-    pcgBody<TK, TV>(g, a);
+    pcgBody<TK, TV, SBB>(g, a);
 }
 
 template <class TK, class TV>
@@ -491,8 +465,8 @@ int batchGrid(Context& ctx) {
     static int per_sm = -1;
     if (per_sm < 0) {
         int a = 0, b = 0;
-        BSG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, kPcgSellBatch<double, double>, SB, 0));
-        BSG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kPcgSellBatch<double, float>, SB, 0));
+        BSG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, kPcgSellBatch<double, double>, SBB, 0));
+        BSG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kPcgSellBatch<double, float>, SBB, 0));
         per_sm = std::min(a, b);
         if (per_sm <= 0) fail(kCuda, "batched SELL PCG kernel cannot be resident");
     }
@@ -514,35 +488,40 @@ void launchSellPcg(Context& ctx, const SellPcgArgs<TK, TV>& in) {
     ctx.launched();
 }
 
-int sellBatchCapacity(Context& ctx) { return batchGrid(ctx); }
-
 template <class TK, class TV>
-void launchSellPcgBatch(Context& ctx, BatchLaunch<TK, TV>& batch) {
-    const int nsegs = static_cast<int>(batch.args.size());
-    if (nsegs == 0) return;
-    if (static_cast<int>(batch.cta_begin.size()) != nsegs + 1 || batch.cta_begin.front() != 0)
-        fail(kArgument, "batched PCG: CTA table does not match the systems");
-    for (int k = 0; k < nsegs; ++k)
-        if (batch.cta_begin[k + 1] <= batch.cta_begin[k]) fail(kArgument, "batched PCG: a system without CTAs");
-    const int total = batch.cta_begin.back();
-    if (total > batchGrid(ctx)) fail(kArgument, "batched PCG: CTA allotment exceeds the resident grid");
+void launchSellPcgBatch(Context& ctx, BatchLaunch<TK, TV>& batch, const std::vector<long long>& slices) {
+    const std::size_t count = batch.args.size();
+    if (count == 0) return;
+    if (slices.size() != count) fail(kArgument, "batched PCG: slice counts do not match the systems");
+    const std::size_t capacity = batchGrid(ctx);
     batch.d_args.upload(batch.args, ctx.stream);
-    batch.d_cta.upload(batch.cta_begin, ctx.stream);
-    batch.d_bars.resize(nsegs);
-    resetBarriers(ctx, batch.d_bars.data(), nsegs, total, batch.cta_begin.data());
-    const SellPcgArgs<TK, TV>* segs = batch.d_args.data();
-    const int* cta = batch.d_cta.data();
-    SegmentBarrier* bars = batch.d_bars.data();
-    int ns = nsegs;
-    void* params[] = {&segs, &cta, &ns, &bars};
-    BSG_PROFILE(ctx, "pcg_amg_persistent_batch");
-    BSG_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(kPcgSellBatch<TK, TV>), total, SB, params, 0,
-                                         ctx.stream));
-    ctx.launched();
+    batch.d_bars.resize(count);
+    std::vector<int> begin, at;  // CTA ranges of every launch, one after another
+    for (std::size_t k0 = 0; k0 < count; k0 += capacity) {
+        const std::size_t m = std::min(capacity, count - k0);
+        const std::vector<int> c = allotCtas({slices.begin() + k0, slices.begin() + k0 + m}, 2 * SBB / 32,
+                                             static_cast<int>(capacity));
+        at.push_back(static_cast<int>(begin.size()));
+        begin.insert(begin.end(), c.begin(), c.end());
+    }
+    batch.d_cta.upload(begin, ctx.stream);
+    for (std::size_t k0 = 0, q = 0; k0 < count; k0 += capacity, ++q) {
+        int ns = static_cast<int>(std::min(capacity, count - k0));
+        const int* ranges = begin.data() + at[q];
+        resetBarriers(ctx, batch.d_bars.data() + k0, ns, ranges[ns], ranges);
+        const SellPcgArgs<TK, TV>* segs = batch.d_args.data() + k0;
+        const int* cta = batch.d_cta.data() + at[q];
+        SegmentBarrier* bars = batch.d_bars.data() + k0;
+        void* params[] = {&segs, &cta, &ns, &bars};
+        BSG_PROFILE(ctx, "pcg_amg_persistent_batch");
+        BSG_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(kPcgSellBatch<TK, TV>), ranges[ns], SBB, params, 0,
+                                             ctx.stream));
+        ctx.launched();
+    }
 }
 
-template void launchSellPcgBatch<double, double>(Context&, BatchLaunch<double, double>&);
-template void launchSellPcgBatch<double, float>(Context&, BatchLaunch<double, float>&);
+template void launchSellPcgBatch<double, double>(Context&, BatchLaunch<double, double>&, const std::vector<long long>&);
+template void launchSellPcgBatch<double, float>(Context&, BatchLaunch<double, float>&, const std::vector<long long>&);
 template void launchSellPcg<double, double>(Context&, const SellPcgArgs<double, double>&);
 template void launchSellPcg<double, float>(Context&, const SellPcgArgs<double, float>&);
 template void launchSellPcg<float, float>(Context&, const SellPcgArgs<float, float>&);

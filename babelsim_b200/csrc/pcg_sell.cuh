@@ -86,21 +86,20 @@ void launchSellPcg(Context& ctx, const SellPcgArgs<TK, TV>& args);
 
 // Several independent systems (each with its own matrix, V-cycle, vectors, partials
 // and PcgState, anywhere in device memory) solved by one cooperative launch: system s
-// runs on CTAs [cta_begin[s], cta_begin[s+1]) with barriers of its own, so the systems
+// runs on a CTA range of its own with barriers of its own, so the systems
 // neither wait for nor perturb one another, and each runs the kernel a single solve on
-// that many CTAs would run.  The host fills args and cta_begin; the launch uploads them.
+// that many CTAs would run.
 template <class TK, class TV>
 struct BatchLaunch {
     std::vector<SellPcgArgs<TK, TV>> args;
-    std::vector<int> cta_begin;  // args.size() + 1 entries, first 0, last = total CTAs
     DeviceArray<SellPcgArgs<TK, TV>> d_args;
     DeviceArray<int> d_cta;
     DeviceArray<SegmentBarrier> d_bars;
 };
 
-// CTAs one batched launch may use (the co-resident grid of the persistent kernel).
-int sellBatchCapacity(Context& ctx);
+// `slices`: level-0 slices of each system, for the CTA shares; more systems than the co-resident
+// grid has CTAs take several launches.
 template <class TK, class TV>
-void launchSellPcgBatch(Context& ctx, BatchLaunch<TK, TV>& batch);
+void launchSellPcgBatch(Context& ctx, BatchLaunch<TK, TV>& batch, const std::vector<long long>& slices);
 
 }  // namespace bsg
