@@ -391,5 +391,6 @@ template void launchBicgstab<1, double>(Context&, const BicgArgs<1, double>&);
 template void launchBicgstab<3, float>(Context&, const BicgArgs<3, float>&);
 template void launchBicgstab<1, float>(Context&, const BicgArgs<1, float>&);
 template void launchBicgstabBatch<3>(Context&, BicgBatch<3>&);
+template void launchBicgstabBatch<1>(Context&, BicgBatch<1>&);
 
 }  // namespace bsg

@@ -1129,13 +1129,15 @@ void KrylovSolver::solveBatch(Context& ctx, std::vector<BatchSolve>& items) {
 #endif
 constexpr int kPersistentBicgstabRows = BSG_PERSISTENT_BICGSTAB_ROWS;
 
-void KrylovSolver::solveVector3Batch(Context& ctx, std::vector<BicgItem>& items, bool batched) {
+template <int C>
+void KrylovSolver::persistentBicgstab(Context& ctx, std::vector<BicgItem>& items, bool batched) {
     const int K = static_cast<int>(items.size());
     if (K == 0) return;
     struct Track {
         BicgState h{};
-        double scale[3] = {1, 1, 1}, target[3] = {0, 0, 0}, fin[3] = {0, 0, 0};
-        bool finished[3] = {false, false, false};
+        double scale[C], target[C] = {}, fin[C] = {};
+        bool finished[C] = {};
+        bool all() const { return std::all_of(finished, finished + C, [](bool f) { return f; }); }
     };
     std::vector<Track> t(K);
     std::vector<SellMat<double>> sell(K);
@@ -1144,12 +1146,12 @@ void KrylovSolver::solveVector3Batch(Context& ctx, std::vector<BicgItem>& items,
         if (!it.solver || &it.solver->impl_->ctx != &ctx) fail(kArgument, "batched BiCGStab: solvers must share ctx");
         Impl& m = *it.solver->impl_;
         const int n = it.A.n;
-        m.ensure(3 * static_cast<std::size_t>(n));
+        m.ensure(C * static_cast<std::size_t>(n));
         if (m.bst.size() < 1) m.bst.resize(1);
         sell[k] = m.sellOf(it.A);
-        if (!it.cfg.warm_start) BSG_CUDA(cudaMemsetAsync(it.x, 0, sizeof(double) * 3 * n, ctx.stream));
+        if (!it.cfg.warm_start) BSG_CUDA(cudaMemsetAsync(it.x, 0, sizeof(double) * C * n, ctx.stream));
         BicgState& h = t[k].h;
-        for (int c = 0; c < 3; ++c) {
+        for (int c = 0; c < C; ++c) {
             h.target2[c] = -1.0;
             h.done[c] = 0;
             h.iters[c] = 0;
@@ -1160,11 +1162,11 @@ void KrylovSolver::solveVector3Batch(Context& ctx, std::vector<BicgItem>& items,
         h.max_iters = it.cfg.max_iterations;
     }
     std::vector<BicgState> res(K);
-    BicgBatch<3> batch;
+    BicgBatch<C> batch;
     for (int attempt = 0; attempt < 3; ++attempt) {
         std::vector<int> active;
         for (int k = 0; k < K; ++k)
-            if (!(t[k].finished[0] && t[k].finished[1] && t[k].finished[2])) active.push_back(k);
+            if (!t[k].all()) active.push_back(k);
         if (active.empty()) break;
         batch.args.clear();
         for (int k : active) {
@@ -1174,9 +1176,9 @@ void KrylovSolver::solveVector3Batch(Context& ctx, std::vector<BicgItem>& items,
                                   m.ph.data(), m.sh.data(), m.t.data(), m.partial.data(), m.bst.data()});
         }
         if (batched) {
-            launchBicgstabBatch<3>(ctx, batch);
+            launchBicgstabBatch<C>(ctx, batch);
         } else {
-            for (const auto& a : batch.args) launchBicgstab<3, double>(ctx, a);
+            for (const auto& a : batch.args) launchBicgstab<C, double>(ctx, a);
         }
         for (int k : active)
             BSG_CUDA(cudaMemcpyAsync(&res[k], items[k].solver->impl_->bst.data(), sizeof(BicgState),
@@ -1190,7 +1192,7 @@ void KrylovSolver::solveVector3Batch(Context& ctx, std::vector<BicgItem>& items,
                 fail(kCuda, "persistent BiCGStab: a barrier wait ran past its bound" +
                                 (batched ? barrierReport(batch.d_bars.data(), batch.bars_used)
                                          : barrierReport(ctx.grid_barrier)));
-            for (int c = 0; c < 3; ++c) {
+            for (int c = 0; c < C; ++c) {
                 if (tr.finished[c]) continue;
                 SolveOutcome& o = it.out[c];
                 ++o.checks;
@@ -1205,7 +1207,9 @@ void KrylovSolver::solveVector3Batch(Context& ctx, std::vector<BicgItem>& items,
                 o.final_ = tr.fin[c];
                 o.relative = tr.fin[c] / tr.scale[c];
                 const bool ok = std::isfinite(tr.fin[c]) && tr.fin[c] <= tr.target[c];
-                o.status = ok ? 0 : (std::isfinite(tr.fin[c]) && r.done[c] != 2 ? 1 : 2);
+                // a breakdown that leaves a finite residual: numerical failure for a vector system, not
+                // converged for a scalar one
+                o.status = ok ? 0 : (std::isfinite(tr.fin[c]) && (C == 1 || r.done[c] != 2) ? 1 : 2);
                 if (ok || !std::isfinite(tr.fin[c]) || r.done[c] == 2 || r.iters[c] >= it.cfg.max_iterations) {
                     tr.finished[c] = true;
                     tr.h.done[c] = 1;
@@ -1216,13 +1220,17 @@ void KrylovSolver::solveVector3Batch(Context& ctx, std::vector<BicgItem>& items,
                 }
                 tr.h.iters[c] = r.iters[c];
             }
-            for (int c = 0; c < 3; ++c)
+            for (int c = 0; c < C; ++c)
                 if (tr.finished[c]) tr.h.done[c] = 1;
             // a restart recomputes r = b - A x from the current x; targets already set stay
-            for (int c = 0; c < 3; ++c)
+            for (int c = 0; c < C; ++c)
                 if (!tr.finished[c] && tr.h.target2[c] < 0.0) tr.h.target2[c] = r.target2[c];
         }
     }
+}
+
+void KrylovSolver::solveVector3Batch(Context& ctx, std::vector<BicgItem>& items, bool batched) {
+    persistentBicgstab<3>(ctx, items, batched);
 }
 
 // Mixed precision (precision 1) for the Jacobi BiCGStab solves (momentum, transport):
@@ -1343,16 +1351,16 @@ void KrylovSolver::lockstepBicgstab(const Dcsr<double>& A, const SolverConfig& c
         refinedBicgstab<C>(A, cfg, b, x, out);
         return;
     }
-    // the persistent kernel saves the launches and host checks that dominate small systems;
-    // large ones stream faster through the per-phase kernels' higher occupancy
-    if (persistent && C == 3 && A.n <= kPersistentBicgstabRows) {
+    // the persistent kernel saves the launches, the host checks every few iterations and the
+    // launches past convergence that such a check finds
+    if (persistent && A.n <= kPersistentBicgstabRows) {
         std::vector<BicgItem> one(1);
         one[0].solver = this;
         one[0].A = A;
         one[0].b = b;
         one[0].x = x;
         one[0].cfg = cfg;
-        solveVector3Batch(impl_->ctx, one, false);
+        persistentBicgstab<C>(impl_->ctx, one, false);
         for (int c = 0; c < C; ++c) out[c] = one[0].out[c];
         return;
     }

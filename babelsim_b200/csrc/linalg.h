@@ -57,7 +57,7 @@ struct BatchSolve {
     SolveOutcome out{};
 };
 
-// One 3-component system of a batched persistent BiCGStab solve (KrylovSolver::solveVector3Batch).
+// One system (one or three components) of a persistent BiCGStab solve (KrylovSolver::solveVector3Batch).
 struct BicgItem {
     KrylovSolver* solver = nullptr;       // owns this system's vectors, SELL copy and solve state
     Dcsr<double> A{};
@@ -157,6 +157,8 @@ public:
 private:
     SolveOutcome solveRefined(const Dcsr<double>& A, const SolverConfig& cfg, AmgPreconditioner* amg, const double* b,
                               double* x);
+    template <int C>
+    static void persistentBicgstab(Context& ctx, std::vector<BicgItem>& items, bool batched);
     template <int C>
     void lockstepBicgstab(const Dcsr<double>& A, const SolverConfig& cfg, const double* b, double* x,
                           SolveOutcome out[]);
