@@ -59,6 +59,8 @@ namespace {
 constexpr int kBlock = 256;
 // Largest level whose whole V-cycle is kept as a dense matrix (8 MB at 1024 rows, read from L2).
 constexpr int kFoldRows = 1200;
+// Smallest system whose coarse-correction scale is tried out (24 CG iterations cost it about 0.3 ms).
+constexpr int kTuneRows = 2048;
 
 struct HostCsr {
     int n = 0;
@@ -405,7 +407,10 @@ AmgPreconditioner::AmgPreconditioner(DeviceMesh& mesh, const SolverConfig& cfg)
     : mesh_(mesh), ctx_(*mesh.ctx), cfg_(cfg) {
     // Tuning overrides for experiments: Jacobi weight and coarse-correction scale.
     if (const char* w = std::getenv("BSG_AMG_OMEGA")) omega_ = std::atof(w);
-    if (const char* g = std::getenv("BSG_AMG_GAMMA")) gamma_ = std::atof(g);
+    if (const char* g = std::getenv("BSG_AMG_GAMMA")) {
+        gamma_ = std::atof(g);
+        tuned_ = true;
+    }
     if (!(omega_ > 0.0 && omega_ <= 1.0) || !(gamma_ > 0.0 && gamma_ <= 3.0))
         fail(kArgument, "AMG Jacobi weight must be in (0,1] and the correction scale in (0,3]");
     // FP32 V-cycle data on the mixed-precision path (FP64 Krylov vectors and true residual stay FP64)
@@ -565,6 +570,7 @@ void AmgPreconditioner::buildTree(const std::vector<std::vector<int>>& ptr, cons
                                   const std::vector<std::vector<int>>& agg) {
     const int L = static_cast<int>(levels_.size());
     tree_ = cfg_.amg_smoothing_steps <= 1 && L <= kMaxTreeLevels;
+    if (L < 2 || levels_[0]->n < kTuneRows) tuned_ = true;
     for (int l = 0; tree_ && l + 1 < L; ++l) {
         std::vector<int> size(levels_[l + 1]->n, 0);
         for (int I : agg[l])
@@ -694,6 +700,11 @@ void AmgPreconditioner::foldCoarse() {
     else rows(folded_.data());
     BSG_CUDA(cudaGetLastError());
     ctx_.launches += 2;
+}
+
+void AmgPreconditioner::setCorrection(double gamma) {
+    gamma_ = gamma;
+    foldCoarse();
 }
 
 int AmgPreconditioner::treePositions() const {

@@ -54,6 +54,14 @@ public:
     TreeView<double> treeView64() const;
     TreeView<float> treeView32() const;
 
+    // The coarse-correction scale of a hierarchy is chosen once, with its first matrix
+    // (KrylovSolver's tuneCorrection); fixed by a tuning override, and on systems so small that
+    // the trial would cost more than it gives.
+    bool wantsTuning() const { return tree_ && !tuned_; }
+    void tuned() { tuned_ = true; }
+    double correction() const { return gamma_; }
+    void setCorrection(double gamma);
+
     struct Level;
 
 private:
@@ -75,14 +83,14 @@ private:
     DeviceArray<VLevel<double>> d_vl64_;
     DeviceArray<VLevel<float>> d_vl32_;
     DeviceArray<float> dense32_;
-    bool tree_ = false;
+    bool tree_ = false, tuned_ = false;
     TreePlan plan_;
     DeviceArray<double> fold_y_, folded_;  // foldCoarse
     DeviceArray<float> folded32_;
     DeviceArray<TreeLevel> d_tree_;
     DeviceArray<double*> d_tvec64_;
     DeviceArray<float*> d_tvec32_;
-    // Damped-Jacobi weight and coarse-correction scale.  Piecewise-constant
+    // Damped-Jacobi weight and coarse-correction scale (the start value; see wantsTuning).  Piecewise-constant
     // aggregation under-corrects smooth error; scaling the coarse correction by
     // 1.8 (kept fixed, so the V-cycle stays a symmetric operator for CG) cut the
     // CG iterations of the 1M-cell Voronoi pressure systems from 81 to 23 per

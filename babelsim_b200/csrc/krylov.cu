@@ -754,6 +754,79 @@ SolveOutcome KrylovSolver::solveRefined(const Dcsr<double>& A, const SolverConfi
     return out;
 }
 
+namespace {
+// A fixed right-hand side of +-1 with every wavelength in it.
+__global__ void kSigns(int n, double* __restrict__ b) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    unsigned h = static_cast<unsigned>(i) * 2654435761u;
+    h ^= h >> 15;
+    h *= 2246822519u;
+    h ^= h >> 13;
+    b[i] = (h & 1u) ? 1.0 : -1.0;
+}
+constexpr int kTrialIterations = 24;
+// A hierarchy that gains this much in a trial converges fast enough as it is (1e-10 in about 50).
+constexpr double kTrialGood = 3e-5;
+}  // namespace
+
+// The coarse-correction scale of a new hierarchy.  Unsmoothed aggregation under-corrects smooth error;
+// how much depends on how the aggregates lie.  1.8 suits meshes whose couplings are alike in all
+// directions, but on stretched ones pairwise matching joins four cells in a row and the same
+// scale over-corrects.  Each trial is 24 CG iterations with a fixed right-hand side; their residuals
+// rank the scales as whole solves do (CG iterations to 1e-10 at 1.2 / 1.5 / 1.8: tanh-stretched channel
+// of 512k cells 59 / 78 / 103, 200k-cell O-grid 195 / 202 / 218, Voronoi cube 34 / 27 / 25, hex cube
+// 37 / 30 / 28), so the trials run only where 1.8 does badly, and the best one stays.
+void KrylovSolver::tuneCorrection(const Dcsr<double>& A, AmgPreconditioner& amg) {
+    Impl& m = *impl_;
+    Context& ctx = m.ctx;
+    amg.tuned();
+    m.ensureTree(amg.treePositions());
+    if (m.pst.size() < 1) m.pst.resize(1);
+    kSigns<<<gridFor(A.n, kBlock), kBlock, 0, ctx.stream>>>(A.n, m.t.data());
+    ctx.launched();
+    const auto reduction = [&]() -> double {
+        PcgState h{};
+        h.max_iterations = kTrialIterations;
+        BSG_CUDA(cudaMemcpyAsync(m.pst.data(), &h, sizeof(h), cudaMemcpyHostToDevice, ctx.stream));
+        launchTree(amg, A.n, m.t.data(), m.tmp.data());
+        BSG_CUDA(cudaMemcpyAsync(ctx.pinned, m.pst.data(), sizeof(PcgState), cudaMemcpyDeviceToHost, ctx.stream));
+        ctx.sync();
+        PcgState r;
+        std::memcpy(&r, ctx.pinned, sizeof(r));
+        if (r.status == 3)
+            fail(kCuda, "persistent PCG: a barrier wait ran past its bound" + barrierReport(ctx.grid_barrier));
+        return r.status == 1 && r.rr0 > 0.0 && std::isfinite(r.rr) ? std::sqrt(r.rr / r.rr0) : -1.0;
+    };
+    const double start = amg.correction();
+    double chosen = start, best = reduction();
+    if (best < kTrialGood) return;  // good, or no measure (breakdown)
+    for (const double gamma : {1.2, 1.5}) {
+        amg.setCorrection(gamma);
+        const double r = reduction();
+        if (r >= 0.0 && r < best) {
+            best = r;
+            chosen = gamma;
+        }
+    }
+    amg.setCorrection(chosen);
+}
+
+// The tree solver on this solver's workspace (FP64 Krylov vectors and products; an FP32 V-cycle takes
+// the flexible beta).
+void KrylovSolver::launchTree(AmgPreconditioner& amg, int n, const double* b, double* x) {
+    Impl& m = *impl_;
+    const auto solve = [&](auto view, int flexible) {
+        using TV = std::decay_t<decltype(view.gamma)>;
+        launchTreePcg<double, TV>(m.ctx, amg.treePlan(),
+                                  {amg.krylovMatrix(), view, 0, n, b, x, m.r.data(), m.q.data(), m.ph.data(),
+                                   m.pair[0].data(), m.pair[1].data(), m.pair[2].data(), m.pair[3].data(),
+                                   m.partial.data(), m.pst.data(), PhaseLog{}, flexible});
+    };
+    if (amg.fp32VCycle()) solve(amg.treeView32(), 1);
+    else solve(amg.treeView64(), 0);
+}
+
 SolveOutcome KrylovSolver::solvePersistent(const Dcsr<double>& A, const SolverConfig& cfg, AmgPreconditioner* amg,
                                            const double* jacobi_diag, const double* b, double* x) {
     Impl& m = *impl_;
@@ -762,6 +835,7 @@ SolveOutcome KrylovSolver::solvePersistent(const Dcsr<double>& A, const SolverCo
     if (cfg.precision == 1 && amg && amg->fp32VCycle()) return solveRefined(A, cfg, amg, b, x);
     if (amg && amg->hasTree()) m.ensureTree(amg->treePositions());
     else m.ensure(n);
+    if (amg && amg->wantsTuning()) tuneCorrection(A, *amg);
     if (m.pst.size() < 1) m.pst.resize(1);
     const AmgView<double> view = amg ? amg->deviceView() : AmgView<double>{};
     PcgState h{};
@@ -776,16 +850,7 @@ SolveOutcome KrylovSolver::solvePersistent(const Dcsr<double>& A, const SolverCo
     for (int attempt = 0; attempt < 3; ++attempt) {
         BSG_CUDA(cudaMemcpyAsync(m.pst.data(), &h, sizeof(h), cudaMemcpyHostToDevice, ctx.stream));
         if (amg && amg->hasTree()) {
-            // FP64 Krylov vectors and products; an FP32 V-cycle takes the flexible beta
-            const auto solve = [&](auto view, int flexible) {
-                using TV = std::decay_t<decltype(view.gamma)>;
-                launchTreePcg<double, TV>(ctx, amg->treePlan(),
-                                          {amg->krylovMatrix(), view, 0, n, b, x, m.r.data(), m.q.data(),
-                                           m.ph.data(), m.pair[0].data(), m.pair[1].data(), m.pair[2].data(),
-                                           m.pair[3].data(), m.partial.data(), m.pst.data(), PhaseLog{}, flexible});
-            };
-            if (amg->fp32VCycle()) solve(amg->treeView32(), 1);
-            else solve(amg->treeView64(), 0);
+            launchTree(*amg, n, b, x);
         } else if (amg && amg->fp32VCycle()) {
             SellPcgArgs<double, float> args{amg->krylovMatrix(), amg->sellView32(), b, x, m.r.data(), m.z.data(),
                                             m.p.data(), m.v.data(), m.q.data(), m.partial.data(), m.pst.data(),
@@ -998,6 +1063,7 @@ void KrylovSolver::solveBatch(Context& ctx, std::vector<BatchSolve>& items) {
         if (&m.ctx != &ctx) fail(kArgument, "batched solves must share one context");
         if (it.amg->hasTree()) m.ensureTree(it.amg->treePositions());
         else m.ensure(it.A.n);
+        if (it.amg->wantsTuning()) it.solver->tuneCorrection(it.A, *it.amg);
         if (m.pst.size() < 1) m.pst.resize(1);
         t[k].h.target2 = -1.0;
         t[k].h.warm = it.cfg.warm_start ? 1 : 0;

@@ -169,6 +169,8 @@ private:
                              const double* b, double* x);
     SolveOutcome solvePersistent(const Dcsr<double>& A, const SolverConfig& cfg, AmgPreconditioner* amg,
                                  const double* jacobi_diag, const double* b, double* x);
+    void launchTree(AmgPreconditioner& amg, int n, const double* b, double* x);
+    void tuneCorrection(const Dcsr<double>& A, AmgPreconditioner& amg);
     struct Impl;
     std::unique_ptr<Impl> impl_;
 };
