@@ -1,6 +1,7 @@
 // Aggregation AMG: host structure setup once per mesh, device numeric setup per
 // matrix version, device V-cycle.  See amg.h for the design.
 #include "amg.h"
+#include "amg_setup.h"
 #include "bsg_device.cuh"
 #include "pcg_sell.cuh"
 
@@ -44,14 +45,14 @@ struct AmgPreconditioner::Level {
     DeviceArray<int4> t_memb;
     DeviceArray<double> tb, tw, te;
     DeviceArray<float> tb32, tw32, te32;
-    void buildSell(const int* hptr, const int* hcol, cudaStream_t s) {
-        SellPattern pat;
-        pat.build(n, hptr, hcol);
-        nslices = pat.nslices;
-        sell_entries = pat.entries;
-        s_ptr.upload(pat.sptr, s);
-        if (pat.col.empty()) pat.col.push_back(0);
-        s_col.upload(pat.col, s);
+    // SELL-32 pattern from the level's CSR: row pointers on the host, both arrays on the device.
+    void buildSell(const int* hptr, const int* dptr_, const int* dcol_, cudaStream_t s) {
+        const std::vector<int> sptr = sellOffsets(n, hptr);
+        nslices = static_cast<int>(sptr.size()) - 1;
+        sell_entries = sptr.back();
+        s_ptr.upload(sptr, s);
+        s_col.resize(std::max<long long>(sell_entries, 1));
+        sellColumns(n, dptr_, dcol_, s_ptr.data(), s_col.data(), s);
     }
 };
 
@@ -62,70 +63,9 @@ constexpr int kFoldRows = 1200;
 // Smallest system whose coarse-correction scale is tried out (24 CG iterations cost it about 0.3 ms).
 constexpr int kTuneRows = 2048;
 
-struct HostCsr {
-    int n = 0;
-    std::vector<int> ptr, col;
-    std::vector<double> diag, val;
-};
-
-// Greedy pairwise matching on strongest negative couplings.
-std::vector<int> pairwise(const HostCsr& a, int& n_coarse) {
-    std::vector<int> mate(a.n, -1), agg(a.n, -1);
-    int next = 0;
-    for (int i = 0; i < a.n; ++i) {
-        if (agg[i] >= 0) continue;
-        int best = -1;
-        double bs = 0.0;
-        for (int k = a.ptr[i]; k < a.ptr[i + 1]; ++k) {
-            const int j = a.col[k];
-            if (j == i || agg[j] >= 0) continue;
-            const double s = -a.val[k];
-            if (s > bs) { bs = s; best = j; }
-        }
-        agg[i] = next;
-        if (best >= 0) agg[best] = next;
-        ++next;
-    }
-    n_coarse = next;
-    return agg;
-}
-
-// Galerkin coarse graph of piecewise-constant aggregation (host, structure + values).
-HostCsr coarsen(const HostCsr& a, const std::vector<int>& agg, int nc, std::vector<int>* slot_target) {
-    HostCsr c;
-    c.n = nc;
-    c.ptr.assign(nc + 1, 0);
-    c.diag.assign(nc, 0.0);
-    std::vector<std::vector<int>> members(nc);
-    for (int i = 0; i < a.n; ++i) members[agg[i]].push_back(i);
-    std::vector<int> marker(nc, -1);
-    std::vector<int> cols;
-    if (slot_target) slot_target->assign(a.ptr[a.n], -1);
-    for (int I = 0; I < nc; ++I) {
-        cols.clear();
-        for (int i : members[I]) {
-            c.diag[I] += a.diag[i];
-            for (int k = a.ptr[i]; k < a.ptr[i + 1]; ++k) {
-                const int J = agg[a.col[k]];
-                if (J == I) { c.diag[I] += a.val[k]; continue; }
-                if (marker[J] != I) { marker[J] = I; cols.push_back(J); }
-            }
-        }
-        std::sort(cols.begin(), cols.end());
-        const int base = static_cast<int>(c.col.size());
-        for (int J : cols) { c.col.push_back(J); c.val.push_back(0.0); }
-        c.ptr[I + 1] = static_cast<int>(c.col.size());
-        for (int i : members[I]) {
-            for (int k = a.ptr[i]; k < a.ptr[i + 1]; ++k) {
-                const int J = agg[a.col[k]];
-                if (J == I) continue;
-                const int pos = base + static_cast<int>(std::lower_bound(cols.begin(), cols.end(), J) - cols.begin());
-                c.val[pos] += a.val[k];
-                if (slot_target) (*slot_target)[k] = pos;
-            }
-        }
-    }
-    return c;
+__global__ void kGatherInts(int n, const int* __restrict__ index, const int* __restrict__ table, int* __restrict__ out) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) out[i] = table[index[i]];
 }
 
 __global__ void kRdiag(int n, double omega, const double* __restrict__ d, double* __restrict__ rd) {
@@ -446,20 +386,24 @@ void AmgPreconditioner::buildStructure(const Dcsr<double>& A) {
     auto* l0 = new Level();
     l0->n = A.n;
     l0->nnz = A.nnz_off;
-    l0->buildSell(cur.ptr.data(), cur.col.data(), ctx_.stream);
+    l0->buildSell(cur.ptr.data(), A.ptr, A.col, ctx_.stream);
     levels_.push_back(l0);
-    std::vector<std::vector<int>> hptr, hcol, hagg;  // every level's pattern and aggregates
+    std::vector<std::vector<int>> hptr, hagg;  // every level's row pointers and aggregates
     while (cur.n > coarse_target && static_cast<int>(levels_.size()) < max_levels) {
         // aggregates from `passes` rounds of pairwise matching (2 by default: up to 4 rows)
         const int passes = levels_.size() == 1 ? passes0_ : passes_;
         int n2 = cur.n;
         std::vector<int> agg(cur.n);
-        for (int i = 0; i < cur.n; ++i) agg[i] = i;
-        HostCsr work = cur;
+        std::iota(agg.begin(), agg.end(), 0);
+        HostCsr work;
         for (int pass = 0; pass < passes; ++pass) {
             int nn = 0;
-            const std::vector<int> a = pairwise(pass == 0 ? cur : work, nn);
-            if (pass + 1 < passes) work = coarsen(pass == 0 ? cur : work, a, nn, nullptr);
+            const HostCsr& from = pass == 0 ? cur : work;
+            const std::vector<int> a = pairwise(from, nn);
+            if (pass + 1 < passes) {
+                HostCsr coarse = coarsen(from, a, nn, nullptr);
+                work = std::move(coarse);
+            }
             for (int i = 0; i < cur.n; ++i) agg[i] = a[agg[i]];
             n2 = nn;
         }
@@ -467,46 +411,21 @@ void AmgPreconditioner::buildStructure(const Dcsr<double>& A) {
         // V-cycle their barriers and gathers without shrinking the problem
         if (3 * static_cast<long long>(n2) > 2 * static_cast<long long>(cur.n) && cur.n <= 1024) break;
         if (n2 >= cur.n) break;  // no coarsening possible
-        std::vector<int> target;
+        std::vector<int> target, agg_ptr, agg_rows;
         HostCsr next = coarsen(cur, agg, n2, &target);
-        Level* fine = levels_.back();
-        // transfer maps
-        std::vector<int> agg_ptr(n2 + 1, 0), agg_rows(cur.n);
-        for (int i = 0; i < cur.n; ++i) ++agg_ptr[agg[i] + 1];
-        for (int I = 0; I < n2; ++I) agg_ptr[I + 1] += agg_ptr[I];
-        {
-            std::vector<int> fill(agg_ptr.begin(), agg_ptr.end() - 1);
-            for (int i = 0; i < cur.n; ++i) agg_rows[fill[agg[i]]++] = i;
-        }
+        aggregateLists(agg, n2, agg_ptr, agg_rows);
         const long long cnnz = static_cast<long long>(next.col.size());
-        std::vector<int> cslot_ptr(cnnz + 1, 0), cslot_src(cur.ptr[cur.n]);
-        std::vector<int> cintra_ptr(n2 + 1, 0), cintra_src;
-        std::vector<int> counts(cnnz, 0);
-        for (int k = 0; k < cur.ptr[cur.n]; ++k)
-            if (target[k] >= 0) ++cslot_ptr[target[k] + 1];
-        for (long long c = 0; c < cnnz; ++c) cslot_ptr[c + 1] += cslot_ptr[c];
-        {
-            std::vector<int> fill(cslot_ptr.begin(), cslot_ptr.end() - 1);
-            for (int I = 0; I < n2; ++I)
-                for (int mm = agg_ptr[I]; mm < agg_ptr[I + 1]; ++mm) {
-                    const int i = agg_rows[mm];
-                    for (int k = cur.ptr[i]; k < cur.ptr[i + 1]; ++k) {
-                        if (target[k] >= 0) cslot_src[fill[target[k]]++] = k;
-                        else cintra_src.push_back(k);
-                    }
-                    cintra_ptr[I + 1] = static_cast<int>(cintra_src.size());
-                }
-            for (int I = 0; I < n2; ++I) cintra_ptr[I + 1] = std::max(cintra_ptr[I + 1], cintra_ptr[I]);
-        }
+        GalerkinMaps maps = galerkinMaps(cur, target, agg_ptr, agg_rows, static_cast<int>(cnnz));
+        if (maps.cintra_src.empty()) maps.cintra_src.push_back(0);
+        Level* fine = levels_.back();
         cudaStream_t s = ctx_.stream;
         fine->agg.upload(agg, s);
         fine->agg_ptr.upload(agg_ptr, s);
         fine->agg_rows.upload(agg_rows, s);
-        fine->cslot_ptr.upload(cslot_ptr, s);
-        fine->cslot_src.upload(cslot_src, s);
-        fine->cintra_ptr.upload(cintra_ptr, s);
-        if (cintra_src.empty()) cintra_src.push_back(0);
-        fine->cintra_src.upload(cintra_src, s);
+        fine->cslot_ptr.upload(maps.cslot_ptr, s);
+        fine->cslot_src.upload(maps.cslot_src, s);
+        fine->cintra_ptr.upload(maps.cintra_ptr, s);
+        fine->cintra_src.upload(maps.cintra_src, s);
         auto* lv = new Level();
         lv->n = n2;
         lv->nnz = cnnz;
@@ -519,17 +438,15 @@ void AmgPreconditioner::buildStructure(const Dcsr<double>& A) {
         lv->dcol = lv->col.data();
         lv->ddiag = lv->diag.data();
         lv->dval = lv->val.data();
-        lv->buildSell(next.ptr.data(), next.col.data(), s);
+        lv->buildSell(next.ptr.data(), lv->dptr, lv->dcol, s);
         levels_.push_back(lv);
-        ctx_.sync();
+        ctx_.sync();  // the host arrays go
         hptr.push_back(std::move(cur.ptr));
-        hcol.push_back(std::move(cur.col));
         hagg.push_back(std::move(agg));
         cur = std::move(next);
     }
     hptr.push_back(std::move(cur.ptr));
-    hcol.push_back(std::move(cur.col));
-    buildTree(hptr, hcol, hagg);
+    buildTree(hptr, hagg, A.col);
     for (Level* l : levels_) {
         l->x.resize(l->n);
         l->b.resize(l->n);
@@ -566,8 +483,8 @@ void AmgPreconditioner::buildStructure(const Dcsr<double>& A) {
     }
 }
 
-void AmgPreconditioner::buildTree(const std::vector<std::vector<int>>& ptr, const std::vector<std::vector<int>>& col,
-                                  const std::vector<std::vector<int>>& agg) {
+void AmgPreconditioner::buildTree(const std::vector<std::vector<int>>& ptr, const std::vector<std::vector<int>>& agg,
+                                  const int* fine_col) {
     const int L = static_cast<int>(levels_.size());
     tree_ = cfg_.amg_smoothing_steps <= 1 && L <= kMaxTreeLevels;
     if (L < 2 || levels_[0]->n < kTuneRows) tuned_ = true;
@@ -584,77 +501,56 @@ void AmgPreconditioner::buildTree(const std::vector<std::vector<int>>& ptr, cons
     plan_.nnz = levels_[0]->nnz;
     plan_.value_bytes = fp32_ ? 4 : 8;
     plan_.level0_bytes = cfg_.precision == 1 ? 4 : 8;
-    // members of every row of level l + 1, in the order of their rows
-    const auto membersOf = [&](int l) {
-        std::vector<int4> m(levels_[l + 1]->n, make_int4(-1, -1, -1, -1));
-        for (int i = 0; i < levels_[l]->n; ++i) {
-            int4& q = m[agg[l][i]];
-            (q.x < 0 ? q.x : q.y < 0 ? q.y : q.z < 0 ? q.z : q.w) = i;
-        }
-        return m;
-    };
     std::vector<int> order;  // rank -> row of the level above
     for (int l = L - 1; l >= 0; --l) {
         Level* lv = levels_[l];
         const int n = lv->n;
-        std::vector<int> row, rank, pos(n), next(n);
+        TreeMaps t;
         if (l == L - 1) {
-            row.resize(n);
-            std::iota(row.begin(), row.end(), 0);
-            rank = row;
-            pos = row;
-            next = row;
+            t.row.resize(n);
+            std::iota(t.row.begin(), t.row.end(), 0);
+            t.rank = t.pos = t.at = order = t.row;
         } else {
-            const std::vector<int4> m = membersOf(l);
             const long long npos = 4LL * levels_[l + 1]->n;
             if (npos > 2LL * n + 64) break;  // mostly holes: this level and the finer ones keep their numbering
-            row.assign(npos, -1);
-            rank.assign(npos, -1);
-            int k = 0;
-            for (std::size_t c = 0; c < order.size(); ++c) {
-                const int4 q = m[order[c]];
-                const int rows[4] = {q.x, q.y, q.z, q.w};
-                for (int j = 0; j < 4; ++j) {
-                    if (rows[j] < 0) continue;
-                    row[4 * c + j] = rows[j];
-                    rank[4 * c + j] = k;
-                    pos[k] = static_cast<int>(4 * c) + j;
-                    next[k++] = rows[j];
-                }
-            }
+            t = treeMaps(n, membersOf(agg[l], levels_[l + 1]->n), order);
             plan_.slices[l] = (npos + 31) / 32;
             double entries = 0.0;
             for (long long p0 = 0; p0 < npos; p0 += 32) {
                 int w = 0;
                 for (long long p = p0; p < std::min(npos, p0 + 32); ++p)
-                    if (row[p] >= 0) w = std::max(w, ptr[l][row[p] + 1] - ptr[l][row[p]]);
+                    if (t.row[p] >= 0) w = std::max(w, ptr[l][t.row[p] + 1] - ptr[l][t.row[p]]);
                 entries += 32.0 * w;
             }
             plan_.entries[l] = entries;
             if (!plan_.fits(l, ctx_.sm_count)) break;  // not even on the whole GPU
         }
         plan_.first = l;
-        lv->npos = static_cast<int>(row.size());
+        lv->npos = static_cast<int>(t.row.size());
         plan_.rows[l] = n;
         plan_.positions[l] = lv->npos;
         cudaStream_t s = ctx_.stream;
-        lv->t_row.upload(row, s);
-        lv->t_rank.upload(rank, s);
-        lv->t_pos.upload(pos, s);
+        lv->t_row.upload(t.row, s);
+        lv->t_rank.upload(t.rank, s);
+        lv->t_pos.upload(t.pos, s);
+        lv->at.upload(t.at, s);
+        std::vector<int4> byPos;
         if (l > 0) {
-            const std::vector<int4> m = membersOf(l - 1);
-            std::vector<int4> byPos(row.size(), make_int4(-1, -1, -1, -1));
-            for (std::size_t p = 0; p < row.size(); ++p)
-                if (row[p] >= 0) byPos[p] = m[row[p]];
+            const Members m = membersOf(agg[l - 1], n);
+            byPos.assign(t.row.size(), make_int4(-1, -1, -1, -1));
+            for (std::size_t p = 0; p < t.row.size(); ++p)
+                if (t.row[p] >= 0) byPos[p] = make_int4(m[t.row[p]][0], m[t.row[p]][1], m[t.row[p]][2], m[t.row[p]][3]);
             lv->t_memb.upload(byPos, s);
         }
-        if (l < L - 1) {
-            std::vector<int> at(n);
-            for (int k = 0; k < n; ++k) at[next[k]] = pos[k];
-            lv->at.upload(at, s);
-            std::vector<int> pcol(std::max<std::size_t>(col[l].size(), 1), 0);
-            for (int k = 0; k < ptr[l][n]; ++k) pcol[k] = at[col[l][k]];
-            lv->t_pcol.upload(pcol, s);
+        if (l < L - 1) {  // the columns' positions
+            const int nnz = ptr[l][n];
+            lv->t_pcol.resize(std::max(nnz, 1));
+            if (nnz > 0) {
+                kGatherInts<<<gridFor(nnz, kBlock), kBlock, 0, s>>>(nnz, l == 0 ? fine_col : lv->dcol, lv->at.data(),
+                                                                   lv->t_pcol.data());
+                BSG_CUDA(cudaGetLastError());
+                ctx_.launched();
+            }
         }
         if (fp32_)
             for (DeviceArray<float>* a : {&lv->tb32, &lv->tw32, &lv->te32}) {
@@ -666,8 +562,7 @@ void AmgPreconditioner::buildTree(const std::vector<std::vector<int>>& ptr, cons
                 a->resize(lv->npos);
                 a->zero(s);
             }
-        ctx_.sync();
-        order = std::move(next);
+        ctx_.sync();  // the host arrays go
     }
     // Level L - 2 and its V-cycle as one dense matrix (foldCoarse), where that level is small.
     if (L >= 3 && plan_.first <= L - 2 && levels_[L - 2]->n <= kFoldRows) {

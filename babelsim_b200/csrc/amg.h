@@ -66,8 +66,8 @@ public:
 
 private:
     void buildStructure(const Dcsr<double>& A);
-    void buildTree(const std::vector<std::vector<int>>& ptr, const std::vector<std::vector<int>>& col,
-                   const std::vector<std::vector<int>>& agg);
+    void buildTree(const std::vector<std::vector<int>>& ptr, const std::vector<std::vector<int>>& agg,
+                   const int* fine_col);
     void uploadViews();
     void uploadTree();
     void foldCoarse();

@@ -558,20 +558,17 @@ struct KrylovSolver::Impl {
     }
     SellMat<double> sellOf(const Dcsr<double>& A) {
         if (sell.ptr != A.ptr || sell.col != A.col || sell.n != A.n || sell.nnz != A.nnz_off) {
-            std::vector<int> hp(A.n + 1), hc(std::max<long long>(A.nnz_off, 1));
+            std::vector<int> hp(A.n + 1);
             BSG_CUDA(cudaMemcpyAsync(hp.data(), A.ptr, sizeof(int) * (A.n + 1), cudaMemcpyDeviceToHost, ctx.stream));
-            if (A.nnz_off > 0)
-                BSG_CUDA(cudaMemcpyAsync(hc.data(), A.col, sizeof(int) * A.nnz_off, cudaMemcpyDeviceToHost,
-                                         ctx.stream));
             ctx.sync();
-            SellPattern pat;
-            pat.build(A.n, hp.data(), hc.data());
-            if (pat.col.empty()) pat.col.push_back(0);
-            sell.sptr.upload(pat.sptr, ctx.stream);
-            sell.scol.upload(pat.col, ctx.stream);
-            sell.sval.resize(pat.col.size());
+            const std::vector<int> sptr = sellOffsets(A.n, hp.data());
+            sell.sptr.upload(sptr, ctx.stream);
+            sell.scol.resize(std::max(sptr.back(), 1));
+            sellColumns(A.n, A.ptr, A.col, sell.sptr.data(), sell.scol.data(), ctx.stream);
+            ctx.launched();
+            sell.sval.resize(std::max(sptr.back(), 1));
             sell.sval.zero(ctx.stream);   // padding entries stay zero
-            sell.nslices = pat.nslices;
+            sell.nslices = static_cast<int>(sptr.size()) - 1;
             sell.ptr = A.ptr;
             sell.col = A.col;
             sell.n = A.n;

@@ -35,38 +35,17 @@ struct SellMat {
     const T* diag = nullptr;    // n
 };
 
-// Host-side pattern: slice offsets and padded column indices of a CSR pattern.
-struct SellPattern {
-    int n = 0, nslices = 0;
-    long long entries = 0;
-    std::vector<int> sptr, col;
-    void build(int rows, const int* ptr, const int* colidx) {
-        n = rows;
-        nslices = (rows + kSellC - 1) / kSellC;
-        sptr.assign(nslices + 1, 0);
-        for (int s = 0; s < nslices; ++s) {
-            int w = 0;
-            for (int l = 0; l < kSellC; ++l) {
-                const int i = kSellC * s + l;
-                if (i < rows) w = std::max(w, ptr[i + 1] - ptr[i]);
-            }
-            sptr[s + 1] = sptr[s] + kSellC * w;
-        }
-        entries = sptr[nslices];
-        col.assign(static_cast<std::size_t>(entries), 0);
-        for (int s = 0; s < nslices; ++s) {
-            const int w = (sptr[s + 1] - sptr[s]) / kSellC;
-            for (int l = 0; l < kSellC; ++l) {
-                const int i = kSellC * s + l;
-                for (int k = 0; k < w; ++k) {
-                    int c = i < rows ? i : 0;
-                    if (i < rows && k < ptr[i + 1] - ptr[i]) c = colidx[ptr[i] + k];
-                    col[static_cast<std::size_t>(sptr[s]) + kSellC * k + l] = c;
-                }
-            }
-        }
+// Slice offsets (entries) of a CSR pattern.
+inline std::vector<int> sellOffsets(int rows, const int* ptr) {
+    const int nslices = (rows + kSellC - 1) / kSellC;
+    std::vector<int> sptr(nslices + 1, 0);
+    for (int s = 0; s < nslices; ++s) {
+        int w = 0;
+        for (int i = kSellC * s; i < std::min(rows, kSellC * (s + 1)); ++i) w = std::max(w, ptr[i + 1] - ptr[i]);
+        sptr[s + 1] = sptr[s] + kSellC * w;
     }
-};
+    return sptr;
+}
 
 #ifdef __CUDACC__
 // sum_k a_ik y(col_ik) over this lane's row of slice s (lane = row within the slice).
@@ -129,6 +108,23 @@ __device__ __forceinline__ T sellRowSplit(const SellMat<T>& A, int s, int r, int
     T a = a0 + a1;
     for (int o = K >> 1; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
     return a;
+}
+
+// Padded columns of a CSR pattern, one block per slice: padding entries hold their own row, rows
+// past n column 0.
+static __global__ void kSellColumns(int n, const int* __restrict__ ptr, const int* __restrict__ col,
+                                    const int* __restrict__ sptr, int* __restrict__ scol) {
+    const int s = blockIdx.x, beg = sptr[s], count = sptr[s + 1] - beg;
+    for (int e = threadIdx.x; e < count; e += blockDim.x) {
+        const int i = kSellC * s + (e & 31), k = e >> 5;
+        int c = 0;
+        if (i < n) c = k < ptr[i + 1] - ptr[i] ? col[ptr[i] + k] : i;
+        scol[beg + e] = c;
+    }
+}
+inline void sellColumns(int n, const int* ptr, const int* col, const int* sptr, int* scol, cudaStream_t stream) {
+    if (n > 0) kSellColumns<<<(n + kSellC - 1) / kSellC, 128, 0, stream>>>(n, ptr, col, sptr, scol);
+    BSG_CUDA(cudaGetLastError());
 }
 
 // Values of a CSR matrix (FP64) scattered into SELL positions, converted to T;
