@@ -5,8 +5,6 @@
 #include "bsg_device.cuh"
 #include "pcg_sell.cuh"
 
-#include <cooperative_groups.h>
-
 #include <algorithm>
 #include <cmath>
 #include <numeric>
@@ -127,81 +125,122 @@ __global__ void kDenseInverse(int n, const int* __restrict__ ptr, const int* __r
     }
 }
 
-// The same in-place Gauss-Jordan inverse on a cluster of kDenseCluster CTAs that
-// keeps the matrix in distributed shared memory: CTA q owns rows [q*rows, (q+1)*rows).
-// Step k: every CTA holds pivot row k in its own buffer pk[k & 1] (pushed there by
-// the row's owner during step k - 1), saves its rows' column k, updates its rows
-// exactly as kDenseInverse does, and the owner of row k + 1 pushes that row's new
-// values into every CTA's other buffer; one cluster barrier ends the step.  The
-// barrier orders the pushes of step k before their reads in step k + 1, and the
-// reads of a buffer in step k - 1 before its overwrite in step k.
-constexpr int kDenseCluster = 8;
-// Largest coarsest level whose rows, pivot buffers and column copy fit 8 CTAs of 200 KB:
-// ceil(n/8) n + 2n + ceil(n/8) doubles per CTA.
+// The same inverse in blocks of kInvBlock pivots on one thread-block cluster, the matrix in its CTAs'
+// shared memory: CTA q owns rows [q*rows, (q+1)*rows), a multiple of the block.  Per block, with D its
+// diagonal block and R its rows: the owner inverts D (one warp, Gauss-Jordan), forms D^-1 R, keeps it as
+// its rows (D^-1 in the block's own columns) and leaves a copy in memory; after a cluster barrier every
+// CTA reads that panel and takes it off its other rows, whose entries C in the block's columns
+// become -C D^-1.  2 n^3 flops are little (0.2 GFLOP at 440 rows); what counts is the chain, which is
+// two barriers and two block-wide passes per 16 pivots instead of one of each per pivot: see the
+// figures at kAmgCoarsestRows.
+constexpr int kInvBlock = 16;
+constexpr int kInvThreads = 256;
+// Largest coarsest level: 16 CTAs of 32 rows keep 440 rows (rows x n + the panel, 169 KB).  Time of one
+// inverse, pivot by pivot on 8 CTAs against in blocks on 16:
+//   256 rows 1.00 / 0.40 ms, 294 rows 1.10 / 0.40 ms, 400 rows 2.50 / 0.55 ms.
 constexpr int kAmgCoarsestRows = 440;
 
-__global__ void __cluster_dims__(kDenseCluster, 1, 1)
-    kDenseInverseCluster(int n, int rows, const int* __restrict__ ptr, const int* __restrict__ col,
-                         const double* __restrict__ diag, const double* __restrict__ val, double* __restrict__ M) {
-    namespace cg = cooperative_groups;
-    cg::cluster_group cluster = cg::this_cluster();
+__global__ void __launch_bounds__(kInvThreads, 1)
+    kDenseInverseBlocked(int n, int rows, const int* __restrict__ ptr, const int* __restrict__ col,
+                         const double* __restrict__ diag, const double* __restrict__ val, double* panel,
+                         double* __restrict__ M) {
     extern __shared__ double sh[];
-    double* Ml = sh;                                   // rows x n, this CTA's rows
-    double* pk = sh + static_cast<long long>(rows) * n;  // two pivot-row buffers of n
-    double* pc = pk + 2 * n;                           // column k of this CTA's rows
-    const int q = static_cast<int>(cluster.block_rank());
-    const int r0 = q * rows, r1 = min(n, r0 + rows), nr = max(0, r1 - r0);
-    for (int e = threadIdx.x; e < nr * n; e += blockDim.x) Ml[e] = 0.0;
+    double* Ml = sh;                                          // rows x n, this CTA's rows
+    double* R = sh + static_cast<long long>(rows) * n;        // kInvBlock x n, the block's rows
+    __shared__ double D[kInvBlock][kInvBlock + 1];
+    ClusterGroup g;
+    const int q = g.rank(), tid = threadIdx.x, lane = tid & 31;
+    const int r0 = min(n, q * rows), nr = min(n, r0 + rows) - r0;
+    for (int e = tid; e < nr * n; e += kInvThreads) Ml[e] = 0.0;
     __syncthreads();
-    for (int li = threadIdx.x; li < nr; li += blockDim.x) {
+    for (int li = tid; li < nr; li += kInvThreads) {
         const int i = r0 + li;
         Ml[static_cast<long long>(li) * n + i] = diag[i];
         for (int k = ptr[i]; k < ptr[i + 1]; ++k) Ml[static_cast<long long>(li) * n + col[k]] += val[k];
     }
     __syncthreads();
-    // row 0 into every CTA's buffer 0
-    if (q == 0)
-        for (int e = threadIdx.x; e < kDenseCluster * n; e += blockDim.x) {
-            double* dst = cluster.map_shared_rank(pk, e / n);
-            dst[e % n] = Ml[e % n];
-        }
-    cluster.sync();
-    // each thread owns one column slot of `rpp` rows per pass (one division, outside the step loop)
-    const int bd = static_cast<int>(blockDim.x);
-    const int rpp = n >= bd ? 1 : bd / n;
-    const int tj = n >= bd ? static_cast<int>(threadIdx.x) : static_cast<int>(threadIdx.x) % n;
-    const int tr = n >= bd ? 0 : static_cast<int>(threadIdx.x) / n;
-    const int jstep = n >= bd ? bd : n;
-    for (int k = 0; k < n; ++k) {
-        const double* prow = pk + (k & 1) * n;
-        const double p = 1.0 / prow[k];
-        for (int li = threadIdx.x; li < nr; li += blockDim.x) pc[li] = Ml[static_cast<long long>(li) * n + k];
-        __syncthreads();
-        if (tr < rpp)
-            for (int li = tr; li < nr; li += rpp) {
-                const int i = r0 + li;
-                double* row = Ml + static_cast<long long>(li) * n;
-                const double c = pc[li];
-                for (int j = tj; j < n; j += jstep) {
-                    double v;
-                    if (i == k) v = j == k ? p : prow[j] * p;
-                    else if (j == k) v = -c * p;
-                    else v = row[j] - c * prow[j] * p;
-                    row[j] = v;
+    for (int b0 = 0; b0 < n; b0 += kInvBlock) {
+        const int nb = min(kInvBlock, n - b0);
+        const bool owner = b0 >= r0 && b0 < r0 + nr;
+        double* out = panel + static_cast<long long>((b0 / kInvBlock) & 1) * kInvBlock * n;
+        if (owner) {
+            double* rowsB = Ml + static_cast<long long>(b0 - r0) * n;
+            if (tid < 32) {  // D^-1
+                for (int e = lane; e < nb * nb; e += 32) D[e / nb][e % nb] = rowsB[static_cast<long long>(e / nb) * n + b0 + e % nb];
+                __syncwarp();
+                for (int k = 0; k < nb; ++k) {
+                    const double p = 1.0 / D[k][k];
+                    double next[kInvBlock * kInvBlock / 32];
+#pragma unroll
+                    for (int u = 0; u < kInvBlock * kInvBlock / 32; ++u) {
+                        const int e = lane + 32 * u, i = e / kInvBlock, j = e % kInvBlock;
+                        next[u] = 0.0;
+                        if (i >= nb || j >= nb) continue;
+                        if (i == k) next[u] = j == k ? p : D[k][j] * p;
+                        else if (j == k) next[u] = -D[i][k] * p;
+                        else next[u] = D[i][j] - D[i][k] * D[k][j] * p;
+                    }
+                    __syncwarp();
+#pragma unroll
+                    for (int u = 0; u < kInvBlock * kInvBlock / 32; ++u) {
+                        const int e = lane + 32 * u, i = e / kInvBlock, j = e % kInvBlock;
+                        if (i < nb && j < nb) D[i][j] = next[u];
+                    }
+                    __syncwarp();
                 }
             }
-        __syncthreads();
-        const int next = k + 1;
-        if (next < n && next >= r0 && next < r1) {
-            const double* src = Ml + static_cast<long long>(next - r0) * n;
-            for (int e = threadIdx.x; e < kDenseCluster * n; e += blockDim.x) {
-                double* dst = cluster.map_shared_rank(pk + (next & 1) * n, e / n);
-                dst[e % n] = src[e % n];
+            __syncthreads();
+            for (int j = tid; j < n; j += kInvThreads) {  // one column of D^-1 R per thread
+                const bool own = j >= b0 && j < b0 + nb;
+                double in[kInvBlock];
+#pragma unroll
+                for (int k = 0; k < kInvBlock; ++k) in[k] = k < nb ? rowsB[static_cast<long long>(k) * n + j] : 0.0;
+                for (int i = 0; i < nb; ++i) {
+                    double v = 0.0;
+                    if (own) v = D[i][j - b0];
+                    else
+#pragma unroll
+                        for (int k = 0; k < kInvBlock; ++k) v += (k < nb ? D[i][k] : 0.0) * in[k];
+                    rowsB[static_cast<long long>(i) * n + j] = v;
+                    out[static_cast<long long>(i) * n + j] = v;
+                }
             }
         }
-        cluster.sync();
+        g.sync();  // the panel is in memory
+#pragma unroll 8
+        for (int e = tid; e < nb * n; e += kInvThreads) R[e] = out[e];
+        __syncthreads();
+        // four rows at a time, so an entry of R is read once for four updates
+        const int warp = tid >> 5, warps = kInvThreads / 32;
+        for (int l0 = 4 * warp; l0 < nr; l0 += 4 * warps) {
+            if (owner && l0 >= b0 - r0 && l0 < b0 - r0 + nb) continue;  // blocks are multiples of four rows
+            const int m = min(4, nr - l0);
+            double c[4][kInvBlock];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int k = 0; k < kInvBlock; ++k)
+                    c[i][k] = i < m && k < nb ? Ml[static_cast<long long>(l0 + i) * n + b0 + k] : 0.0;
+            __syncwarp();  // every lane has C before any of it is overwritten
+            for (int j = lane; j < n; j += 32) {
+                const bool own = j >= b0 && j < b0 + nb;
+                double v[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) v[i] = own || i >= m ? 0.0 : Ml[static_cast<long long>(l0 + i) * n + j];
+#pragma unroll
+                for (int k = 0; k < kInvBlock; ++k) {
+                    const double r = k < nb ? R[k * n + j] : 0.0;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) v[i] -= c[i][k] * r;
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    if (i < m) Ml[static_cast<long long>(l0 + i) * n + j] = v[i];
+            }
+        }
+        __syncthreads();  // rows, and R, before the next block (the panel alternates between two halves)
     }
-    for (int e = threadIdx.x; e < nr * n; e += blockDim.x) M[static_cast<long long>(r0) * n + e] = Ml[e];
+    for (int e = tid; e < nr * n; e += kInvThreads) M[static_cast<long long>(r0) * n + e] = Ml[e];
 }
 
 // foldCoarse, first pass: column j of Y = M T, one block per j.  Column j of T has 1 - a_jj w_j at
@@ -329,17 +368,19 @@ __global__ void kCopy(int n, const double* __restrict__ a, double* __restrict__ 
 namespace {
 // Dynamic shared memory of one CTA of the cluster inverse (the rest of the SM's
 // 228 KB stays for the driver's reserve).
-constexpr std::size_t kDenseClusterSmem = 200 * 1024;
+constexpr std::size_t kInverseSmem = 200 * 1024;
 
-bool clusterReady() {
-    static int ok = -1;
-    if (ok < 0) {
-        ok = cudaFuncSetAttribute(kDenseInverseCluster, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  static_cast<int>(kDenseClusterSmem)) == cudaSuccess;
-        if (ok && std::getenv("BSG_DENSE_SINGLE_BLOCK")) ok = 0;
-        cudaGetLastError();
-    }
-    return ok == 1;
+// CTAs of the cluster inverse's cluster, 0 where none can be had.
+int inverseCtas() {
+    static const int ctas = [] {
+        if (cudaFuncSetAttribute(kDenseInverseBlocked, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(kInverseSmem)) != cudaSuccess) {
+            cudaGetLastError();
+            return 0;
+        }
+        return clusterCtas<kDenseInverseBlocked>(kInvThreads, static_cast<int>(kInverseSmem));
+    }();
+    return ctas;
 }
 }  // namespace
 
@@ -654,15 +695,19 @@ void AmgPreconditioner::update(const Dcsr<double>& A, bool numeric) {
         ctx_.launched();
     }
     Level* last = levels_.back();
-    const int crow = (last->n + kDenseCluster - 1) / kDenseCluster;
-    const std::size_t csmem = sizeof(double) * (static_cast<std::size_t>(crow) * last->n + 2 * last->n + crow);
-    if (csmem <= kDenseClusterSmem && clusterReady()) {
-        kDenseInverseCluster<<<kDenseCluster, 1024, csmem, ctx_.stream>>>(last->n, crow, last->dptr, last->dcol,
-                                                                         last->ddiag, last->dval, last->dense.data());
-    } else
-    kDenseInverse<<<1, 1024, 2 * sizeof(double) * last->n, ctx_.stream>>>(last->n, last->dptr, last->dcol, last->ddiag,
-                                                                         last->dval, last->dense.data());
-    ctx_.launched();
+    const int ctas = inverseCtas();
+    const int irows = ctas > 0 ? (last->n + ctas * kInvBlock - 1) / (ctas * kInvBlock) * kInvBlock : 0;
+    const std::size_t ismem = sizeof(double) * (static_cast<std::size_t>(irows) + kInvBlock) * last->n;
+    if (ctas > 0 && ismem <= kInverseSmem) {
+        inv_panel_.resize(2 * static_cast<std::size_t>(kInvBlock) * last->n);
+        launchCluster<kDenseInverseBlocked>(ctx_, 1, kInvThreads, static_cast<int>(ismem), static_cast<int>(kInverseSmem),
+                                            last->n, irows, last->dptr, last->dcol, last->ddiag, last->dval,
+                                            inv_panel_.data(), last->dense.data());
+    } else {
+        kDenseInverse<<<1, 1024, 2 * sizeof(double) * last->n, ctx_.stream>>>(
+            last->n, last->dptr, last->dcol, last->ddiag, last->dval, last->dense.data());
+        ctx_.launched();
+    }
     BSG_CUDA(cudaGetLastError());
     foldCoarse();
     // SELL-32 values for the persistent solver

@@ -87,6 +87,7 @@ private:
     TreePlan plan_;
     DeviceArray<double> fold_y_, folded_;  // foldCoarse
     DeviceArray<float> folded32_;
+    DeviceArray<double> inv_panel_;        // kDenseInverseBlocked's panel, two halves
     DeviceArray<TreeLevel> d_tree_;
     DeviceArray<double*> d_tvec64_;
     DeviceArray<float*> d_tvec32_;
