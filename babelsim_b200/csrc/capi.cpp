@@ -32,9 +32,7 @@ struct bsg_system {
     std::unique_ptr<bsg::AmgPreconditioner> amg;
     bsg::JacobiPreconditioner jacobi;
     bsg::PcReusePolicy policy;
-    std::vector<double> diag, upper, lower;  // matrix values of the last update (caller's face order)
-    std::vector<double> slots;               // off-diagonal values in device slot order
-    bool ready = false;
+    bsg::SeamMatrix matrix;
     bsg_system_counters counters{};
 };
 struct bsg_mesh {
@@ -355,15 +353,7 @@ std::unique_ptr<bsg_system> makeSystem(bsg_mesh* mesh, int components) {
     s->unknown = std::make_unique<bsg::DeviceField>(m, 0, components);
     s->eq = std::make_unique<bsg::DeviceEquation>(*s->unknown, bsg::Options{});
     s->krylov = std::make_unique<bsg::KrylovSolver>(*m.ctx);
-    s->slots.assign(2 * static_cast<std::size_t>(m.n_interior), 0.0);
     return s;
-}
-
-bool sameValues(const std::vector<double>& kept, const double* v, std::size_t n) {
-    if (kept.size() != n) return false;
-    for (std::size_t i = 0; i < n; ++i)
-        if (kept[i] != v[i]) return false;  // exact equality; NaN always counts as changed
-    return true;
 }
 
 double secondsSince(std::chrono::steady_clock::time_point t) {
@@ -377,30 +367,13 @@ void systemSolve(bsg_system* s, const bsg::SolverConfig& cfg, const double* diag
     bsg::DeviceMesh& m = *s->mesh->mesh;
     bsg::Context& ctx = *m.ctx;
     const int N = m.n_cells, C = s->comps;
-    const std::size_t F = m.n_faces;
     bsg_system_counters& k = s->counters;
     const auto t0 = std::chrono::steady_clock::now();
     for (int i = 0; i < N; ++i)
         if (!std::isfinite(diagonal[i])) bsg::fail(bsg::kNumeric, "nonfinite matrix diagonal");
-    const bool changed = !s->ready || !sameValues(s->diag, diagonal, N) || !sameValues(s->upper, upper, F) ||
-                         !sameValues(s->lower, lower, F);
-    if (changed) {
-        s->diag.assign(diagonal, diagonal + N);
-        s->upper.assign(upper, upper + F);
-        s->lower.assign(lower, lower + F);
-        for (int i = 0; i < m.n_interior; ++i) {
-            const int f = m.interior_ext[i];
-            s->slots[m.h_slot_own[i]] = upper[f];
-            s->slots[m.h_slot_nbr[i]] = lower[f];
-        }
-        s->eq->diag.resize(N);
-        bsg::uploadCells(m, s->eq->diag.data(), diagonal, 1);
-        s->eq->val.upload(s->slots, ctx.stream);
-        s->ready = true;
-        ++k.matrix_value_updates;
-    } else {
-        ++k.rhs_only_solves;
-    }
+    const bool changed = s->matrix.update(m, diagonal, upper, lower, *s->eq);
+    if (changed) ++k.matrix_value_updates;
+    else ++k.rhs_only_solves;
     s->eq->src.resize(static_cast<std::size_t>(N) * C);
     bsg::uploadCells(m, s->eq->src.data(), source, C);
     s->unknown->v.resize(static_cast<std::size_t>(N) * C);

@@ -79,6 +79,18 @@ struct Reducer {
 
 // Cell arrays between the caller's numbering (host) and the device's (C values per cell):
 // a plain copy, or through the mesh's locality renumbering when it has one.
+// The matrix of a linear-system seam: the caller's arrays of the last update on the device (faces'
+// upper and lower values, cells' diagonal, two buffers in turn).
+struct DeviceEquation;
+struct SeamMatrix {
+    DeviceArray<double> raw[2];
+    DeviceArray<int> flag;
+    int held = 0;        // buffer of the last update
+    bool ready = false;
+    // Brings eq.diag and eq.val up to date; false when every value equals the last update's.
+    bool update(DeviceMesh& m, const double* diagonal, const double* upper, const double* lower, DeviceEquation& eq);
+};
+
 void uploadCells(DeviceMesh& m, double* device, const double* host, int C);
 void downloadCells(DeviceMesh& m, const double* device, double* host, int C);
 
