@@ -41,9 +41,17 @@ struct BicgArgs {
     const T* b;              // C-interleaved right-hand sides
     T* x;                    // C-interleaved initial guess / solution
     T *r, *r0, *p, *v, *ph, *sh, *t;  // C * n each
+    T *gph, *gsh;            // kGatherStride<C> * n each: ph and sh of the on-chip solver (see bicgstab_sell.cu)
     double* partial;         // 2 * ctas * kSumValues doubles
     BicgState* st;
+    long long entries;       // padded SELL entries of A
+    int chip = 0;            // set by the launch: bytes of shared memory for rows and vectors, 0: streamed
 };
+
+// Entries per row of the vectors that neighbours gather: three components take a 32-byte sector of
+// their own (24-byte rows straddle two every third time, and need three loads instead of two).
+template <int C>
+constexpr int kGatherStride = C == 3 ? 4 : C;
 
 template <int C>
 struct BicgBatch {

@@ -276,7 +276,7 @@ __device__ __forceinline__ int sumThroughBarrier(SegmentBarrier* bar, int rank, 
 // warp 0's work.  `buf` alternates between two halves of `partial` (kSumValues doubles per CTA
 // each, whatever NV is, so the halves of sums of different widths do not overlap) so a fast
 // block's next write never overtakes a slow block's read of the previous sum.
-constexpr int kSumValues = 8;
+constexpr int kSumValues = 10;
 template <int NV, int BS, class G>
 __device__ __forceinline__ void gridSum(G& g, double v[NV], double* partial, int& buf) {
     static_assert(NV <= kSumValues && BS / 32 <= 32, "one warp adds the block's warps");
