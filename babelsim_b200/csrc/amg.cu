@@ -751,7 +751,7 @@ void AmgPreconditioner::uploadViews() {
             Level* lv = levels_[l];
             const bool coarser = l + 1 < L;
             v[l].A = SellMat<float>{lv->n, lv->nslices, lv->s_ptr.data(), lv->s_col.data(), lv->s_val32.data(),
-                                    lv->diag32.data()};
+                                    lv->diag32.data(), sellStreams(lv->sell_entries, 4)};
             v[l].rd = lv->rd32.data();
             v[l].agg_ptr = coarser ? lv->agg_ptr.data() : nullptr;
             v[l].agg_rows = coarser ? lv->agg_rows.data() : nullptr;
@@ -767,7 +767,7 @@ void AmgPreconditioner::uploadViews() {
             Level* lv = levels_[l];
             const bool coarser = l + 1 < L;
             v[l].A = SellMat<double>{lv->n, lv->nslices, lv->s_ptr.data(), lv->s_col.data(), lv->s_val.data(),
-                                     lv->ddiag};
+                                     lv->ddiag, sellStreams(lv->sell_entries, 8)};
             v[l].rd = lv->rdiag.data();
             v[l].agg_ptr = coarser ? lv->agg_ptr.data() : nullptr;
             v[l].agg_rows = coarser ? lv->agg_rows.data() : nullptr;
@@ -804,12 +804,14 @@ void AmgPreconditioner::uploadTree() {
 
 SellMat<double> AmgPreconditioner::krylovMatrix() const {
     const Level* l = levels_.front();
-    return SellMat<double>{l->n, l->nslices, l->s_ptr.data(), l->s_col.data(), l->s_val.data(), l->ddiag};
+    return SellMat<double>{l->n, l->nslices, l->s_ptr.data(), l->s_col.data(), l->s_val.data(), l->ddiag,
+                           sellStreams(l->sell_entries, 8)};
 }
 
 SellMat<float> AmgPreconditioner::krylovMatrix32() const {
     const Level* l = levels_.front();
-    return SellMat<float>{l->n, l->nslices, l->s_ptr.data(), l->s_col.data(), l->s_val32.data(), l->diag32.data()};
+    return SellMat<float>{l->n, l->nslices, l->s_ptr.data(), l->s_col.data(), l->s_val32.data(), l->diag32.data(),
+                          sellStreams(l->sell_entries, 4)};
 }
 
 long long AmgPreconditioner::krylovEntries() const { return levels_.front()->sell_entries; }

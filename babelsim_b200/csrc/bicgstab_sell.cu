@@ -21,7 +21,7 @@ namespace {
 constexpr int BB = 1024;  // threads per CTA, one CTA per SM
 
 // (A x)_i for the C components of row i of slice sl (lane = row within the slice).
-template <int C, class T>
+template <int C, bool STREAM, class T>
 __device__ __forceinline__ void sellProduct(const SellMat<T>& S, int sl, int lane, const T* __restrict__ x, T acc[C]) {
     const int beg = S.sptr[sl], w = (S.sptr[sl + 1] - beg) >> 5;
     const int* __restrict__ cp = S.col + beg + lane;
@@ -35,8 +35,8 @@ __device__ __forceinline__ void sellProduct(const SellMat<T>& S, int sl, int lan
         T vv[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-            cc[u] = __ldg(cp + 32 * (k + u));
-            vv[u] = __ldg(vp + 32 * (k + u));
+            cc[u] = entryLoad<STREAM>(cp + 32 * (k + u));
+            vv[u] = entryLoad<STREAM>(vp + 32 * (k + u));
         }
 #pragma unroll
         for (int u = 0; u < 4; ++u)
@@ -44,8 +44,8 @@ __device__ __forceinline__ void sellProduct(const SellMat<T>& S, int sl, int lan
             for (int c = 0; c < C; ++c) a[c] += vv[u] * x[C * cc[u] + c];
     }
     for (; k < w; ++k) {
-        const int j = __ldg(cp + 32 * k);
-        const T v = __ldg(vp + 32 * k);
+        const int j = entryLoad<STREAM>(cp + 32 * k);
+        const T v = entryLoad<STREAM>(vp + 32 * k);
 #pragma unroll
         for (int c = 0; c < C; ++c) a[c] += v * x[C * j + c];
     }
@@ -60,7 +60,8 @@ template <int C, class T, class F>
 __device__ __forceinline__ void productRows(const SellMat<T>& A, const Lanes& ln, const T* __restrict__ x, F f) {
     for (int sl = ln.gwarp; sl < A.nslices; sl += ln.nwarps) {
         T acc[C];
-        sellProduct<C, T>(A, sl, ln.lane, x, acc);
+        if (A.stream) sellProduct<C, true>(A, sl, ln.lane, x, acc);
+        else sellProduct<C, false>(A, sl, ln.lane, x, acc);
         const int i = 32 * sl + ln.lane;
         if (i < A.n) f(i, acc);
     }

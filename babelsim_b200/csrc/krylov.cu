@@ -578,7 +578,8 @@ struct KrylovSolver::Impl {
             A.n, A.ptr, A.val, A.diag, sell.sptr.data(), 1.0, sell.sval.data(), nullptr, nullptr);
         BSG_CUDA(cudaGetLastError());
         ++ctx.launches;
-        return SellMat<double>{A.n, sell.nslices, sell.sptr.data(), sell.scol.data(), sell.sval.data(), A.diag};
+        return SellMat<double>{A.n, sell.nslices, sell.sptr.data(), sell.scol.data(), sell.sval.data(), A.diag,
+                               sellStreams(static_cast<long long>(sell.sval.size()), 8)};
     }
     int grid(int n) const {
         const long long g = (static_cast<long long>(n) + kBlock - 1) / kBlock;
@@ -1331,7 +1332,7 @@ void KrylovSolver::refinedBicgstab(const Dcsr<double>& A, const SolverConfig& cf
     };
     toFloat(entries, S.val, m.bval32.data());
     toFloat(n, A.diag, m.bdiag32.data());
-    const SellMat<float> S32{n, S.nslices, S.sptr, S.col, m.bval32.data(), m.bdiag32.data()};
+    const SellMat<float> S32{n, S.nslices, S.sptr, S.col, m.bval32.data(), m.bdiag32.data(), sellStreams(entries, 4)};
     if (!cfg.warm_start) BSG_CUDA(cudaMemsetAsync(x, 0, sizeof(double) * cn, ctx.stream));
     const int g = m.grid(n);
     double* result = m.partial.data() + 8 * 4096 - 8;

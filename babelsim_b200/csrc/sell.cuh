@@ -33,7 +33,15 @@ struct SellMat {
     const int* col = nullptr;
     const T* val = nullptr;
     const T* diag = nullptr;    // n
+    bool stream = false;        // entries pass L1 by
 };
+
+// Entries of a large matrix pass L1 by: each is used once per sweep, and kept in L1 they push out the
+// vectors that neighbouring rows gather.  A small one gains from what L1 still holds of it from the
+// sweep before.  By bytes of entries, kept / passed by (ms of pressure and momentum solves per outer
+// iteration): Voronoi 40 MB 9.1 / 10.4, 54 MB 10.0 / 10.6, 85 MB 15.9 / 15.1, 96 MB 16.7 / 15.6, 228 MB
+// 33.1 / 32.6; 2D cavity 39 MB 7.5 / 7.8; momentum and k-omega on a 1M-cell channel, 74 MB, 11.7 / 10.2.
+inline bool sellStreams(long long entries, int value_bytes) { return entries * (4 + value_bytes) > (64LL << 20); }
 
 // Slice offsets (entries) of a CSR pattern.
 inline std::vector<int> sellOffsets(int rows, const int* ptr) {
@@ -48,14 +56,34 @@ inline std::vector<int> sellOffsets(int rows, const int* ptr) {
 }
 
 #ifdef __CUDACC__
+// A matrix entry's load, past L1 if STREAM (see sellStreams).
+__device__ __forceinline__ int streamLoad(const int* p) {
+    int x;
+    asm("ld.global.nc.L1::no_allocate.b32 %0, [%1];" : "=r"(x) : "l"(p));
+    return x;
+}
+__device__ __forceinline__ float streamLoad(const float* p) {
+    float x;
+    asm("ld.global.nc.L1::no_allocate.f32 %0, [%1];" : "=f"(x) : "l"(p));
+    return x;
+}
+__device__ __forceinline__ double streamLoad(const double* p) {
+    double x;
+    asm("ld.global.nc.L1::no_allocate.f64 %0, [%1];" : "=d"(x) : "l"(p));
+    return x;
+}
+template <bool STREAM, class T>
+__device__ __forceinline__ T entryLoad(const T* p) {
+    return STREAM ? streamLoad(p) : __ldg(p);
+}
 // sum_k a_ik y(col_ik) over this lane's row of slice s (lane = row within the slice).
 // Entries go in batches of kSellBatch: all index and value loads of a batch first, then
 // all its gathers; the entries past the last full batch follow one at a time.  (A
 // predicated last batch, which would shorten a row's chain of dependent load rounds,
 // measured slower on the 1M-cell pressure solves: 36.8 against 31.0 ms per outer
 // iteration.)
-template <class T, class Y>
-__device__ __forceinline__ T sellRow(const SellMat<T>& A, int s, int lane, Y y) {
+template <bool STREAM, class T, class Y>
+__device__ __forceinline__ T sellRowAs(const SellMat<T>& A, int s, int lane, Y y) {
     const int beg = A.sptr[s];
     const int w = (A.sptr[s + 1] - beg) >> 5;
     const int* __restrict__ c = A.col + beg + lane;
@@ -67,8 +95,8 @@ __device__ __forceinline__ T sellRow(const SellMat<T>& A, int s, int lane, Y y) 
         T vv[kSellBatch];
 #pragma unroll
         for (int u = 0; u < kSellBatch; ++u) {
-            cc[u] = __ldg(c + 32 * (k + u));
-            vv[u] = __ldg(v + 32 * (k + u));
+            cc[u] = entryLoad<STREAM>(c + 32 * (k + u));
+            vv[u] = entryLoad<STREAM>(v + 32 * (k + u));
         }
         T yy[kSellBatch];
 #pragma unroll
@@ -79,8 +107,12 @@ __device__ __forceinline__ T sellRow(const SellMat<T>& A, int s, int lane, Y y) 
             if (u + 1 < kSellBatch) a1 += vv[u + 1] * yy[u + 1];
         }
     }
-    for (; k < w; ++k) a0 += __ldg(v + 32 * k) * y(__ldg(c + 32 * k));
+    for (; k < w; ++k) a0 += entryLoad<STREAM>(v + 32 * k) * y(entryLoad<STREAM>(c + 32 * k));
     return a0 + a1;
+}
+template <class T, class Y>
+__device__ __forceinline__ T sellRow(const SellMat<T>& A, int s, int lane, Y y) {
+    return A.stream ? sellRowAs<true>(A, s, lane, y) : sellRowAs<false>(A, s, lane, y);
 }
 
 // The same row sum split over K consecutive lanes (K a power of two, 2..32): lane q
