@@ -336,11 +336,6 @@ __global__ void kProlongSmooth(int n, const int* __restrict__ ptr, const int* __
     xo[i] = yi + rd[i] * (b[i] - ay);
 }
 
-__global__ void kProlong(int n, const int* __restrict__ agg, const double* __restrict__ xc, double* __restrict__ x) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) x[i] += xc[agg[i]];
-}
-
 // b_c[I] = sum over fine rows i of aggregate I of (b - A x)_i
 __global__ void kResidualRestrict(int nc, const int* __restrict__ agg_ptr, const int* __restrict__ agg_rows,
                                   const int* __restrict__ ptr, const int* __restrict__ col,
@@ -356,11 +351,6 @@ __global__ void kResidualRestrict(int nc, const int* __restrict__ agg_ptr, const
         s += b[i] - ax;
     }
     bc[I] = s;
-}
-
-__global__ void kCopy(int n, const double* __restrict__ a, double* __restrict__ b) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) b[i] = a[i];
 }
 
 }  // namespace

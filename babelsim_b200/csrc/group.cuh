@@ -156,11 +156,6 @@ struct ClusterGroup {
     }
 };
 
-template <class G>
-constexpr bool kInCluster = false;
-template <>
-constexpr bool kInCluster<ClusterGroup> = true;
-
 struct Lanes {
     int lane, gwarp, nwarps, gthread, nthreads;
 };

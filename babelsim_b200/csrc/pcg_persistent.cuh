@@ -15,8 +15,6 @@
 
 namespace bsg {
 
-constexpr int kMaxAmgLevels = 16;
-
 template <class T>
 struct AmgLevelView {
     int n;
