@@ -683,23 +683,32 @@ template <int C, class T>
 void launchBicgstab(Context& ctx, const BicgArgs<C, T>& args) {
     BSG_PROFILE(ctx, sizeof(T) == 4 ? "bicgstab3_persistent_fp32" : "bicgstab3_persistent");
     BicgArgs<C, T> a = args;
-    allowChip<kBicgChipCluster<C, T>>();
-    a.chip = chipBytes(a, clusterCtas<kBicgChipCluster<C, T>>(CB, kChipSmem));
-    if (a.chip && a.A.n <= kClusterRows) {
-        launchCluster<kBicgChipCluster<C, T>>(ctx, 1, CB, a.chip, kChipSmem, a);
-        return;
+    // FP32 systems are the inner solves of a refined one, which accepts the first iterate under its target:
+    // what the inner iterations round decides which one that is, to a part of the target.  They keep the
+    // streaming kernel's arithmetic (r0 . r of the residual that is kept, the diagonal last), at 0.96 against
+    // 0.86 ms for three right-hand sides on 110k cells.
+    if constexpr (sizeof(T) == 8) {
+        allowChip<kBicgChipCluster<C, T>>();
+        a.chip = chipBytes(a, clusterCtas<kBicgChipCluster<C, T>>(CB, kChipSmem));
+        if (a.chip && a.A.n <= kClusterRows) {
+            launchCluster<kBicgChipCluster<C, T>>(ctx, 1, CB, a.chip, kChipSmem, a);
+            return;
+        }
+        a.chip = chipBytes(a, ctx.sm_count);
     }
-    a.chip = chipBytes(a, ctx.sm_count);
     SegmentBarrier* bar = ctx.grid_barrier;
     const int grid = ctx.sm_count;
     resetBarriers(ctx, bar, 1, grid);
     void* params[] = {&a, &bar};
-    if (a.chip) {
-        allowChip<kBicgChip<C, T>>();
-        BSG_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(kBicgChip<C, T>), grid, CB, params, a.chip, ctx.stream));
-    } else {
-        BSG_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(kBicgSell<C, T>), grid, BB, params, 0, ctx.stream));
+    if constexpr (sizeof(T) == 8) {
+        if (a.chip) {
+            allowChip<kBicgChip<C, T>>();
+            BSG_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(kBicgChip<C, T>), grid, CB, params, a.chip, ctx.stream));
+            ctx.launched();
+            return;
+        }
     }
+    BSG_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(kBicgSell<C, T>), grid, BB, params, 0, ctx.stream));
     ctx.launched();
 }
 

@@ -41,7 +41,7 @@ struct BicgArgs {
     const T* b;              // C-interleaved right-hand sides
     T* x;                    // C-interleaved initial guess / solution
     T *r, *r0, *p, *v, *ph, *sh, *t;  // C * n each
-    T *gph, *gsh;            // kGatherStride<C> * n each: ph and sh of the on-chip solver (see bicgstab_sell.cu)
+    T *gph, *gsh;            // kGatherStride<C> * n each: ph and sh of the on-chip solver (FP64; see bicgstab_sell.cu)
     double* partial;         // 2 * ctas * kSumValues doubles
     BicgState* st;
     long long entries;       // padded SELL entries of A

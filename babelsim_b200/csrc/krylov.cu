@@ -537,7 +537,7 @@ struct KrylovSolver::Impl {
     DeviceArray<float2> pair32[4];
     // FP32 inner BiCGStab of the refined path: matrix copy (SELL values, diagonal) and
     // the C-interleaved right-hand side, correction and Krylov vectors
-    DeviceArray<float> bval32, bdiag32, bb32, bx32, br32, br032, bp32, bv32, bph32, bsh32, bt32, gph32, gsh32;
+    DeviceArray<float> bval32, bdiag32, bb32, bx32, br32, br032, bp32, bv32, bph32, bsh32, bt32;
     GmresWorkspace gmres;
     // SELL-32 copy of the matrix the BiCGStab products read: the pattern of the
     // last CSR pattern seen (a solver's systems all live on one mesh's cell->face
@@ -1319,8 +1319,6 @@ void KrylovSolver::refinedBicgstab(const Dcsr<double>& A, const SolverConfig& cf
     const long long entries = static_cast<long long>(m.sell.sval.size());
     for (DeviceArray<float>* a : {&m.bb32, &m.bx32, &m.br32, &m.br032, &m.bp32, &m.bv32, &m.bph32, &m.bsh32, &m.bt32})
         if (a->size() < static_cast<std::size_t>(cn)) a->resize(cn);
-    for (DeviceArray<float>* a : {&m.gph32, &m.gsh32})
-        if (a->size() < kGatherStride<C> * static_cast<std::size_t>(n)) a->resize(kGatherStride<C> * static_cast<std::size_t>(n));
     if (m.bval32.size() < static_cast<std::size_t>(entries)) m.bval32.resize(entries);
     if (m.bdiag32.size() < static_cast<std::size_t>(n)) m.bdiag32.resize(n);
     auto toFloat = [&](long long count, const double* from, float* to) {
@@ -1383,8 +1381,8 @@ void KrylovSolver::refinedBicgstab(const Dcsr<double>& A, const SolverConfig& cf
         h.max_iters = std::max(budget, 1);
         BSG_CUDA(cudaMemcpyAsync(m.bst.data(), &h, sizeof(h), cudaMemcpyHostToDevice, ctx.stream));
         BicgArgs<C, float> args{S32, m.bb32.data(), m.bx32.data(), m.br32.data(), m.br032.data(), m.bp32.data(),
-                                m.bv32.data(), m.bph32.data(), m.bsh32.data(), m.bt32.data(), m.gph32.data(),
-                                m.gsh32.data(), m.partial.data(), m.bst.data(), entries};
+                                m.bv32.data(), m.bph32.data(), m.bsh32.data(), m.bt32.data(), nullptr, nullptr,
+                                m.partial.data(), m.bst.data(), entries};
         launchBicgstab<C, float>(ctx, args);
         BicgState res;
         BSG_CUDA(cudaMemcpyAsync(&res, m.bst.data(), sizeof(res), cudaMemcpyDeviceToHost, ctx.stream));
