@@ -390,14 +390,19 @@ AmgPreconditioner::AmgPreconditioner(DeviceMesh& mesh, const SolverConfig& cfg)
     if (const char* p = std::getenv("BSG_AMG_PASSES")) passes_ = std::max(1, std::min(4, std::atoi(p)));
 }
 
-AmgPreconditioner::~AmgPreconditioner() {
+AmgPreconditioner::~AmgPreconditioner() { clearLevels(); }
+
+void AmgPreconditioner::clearLevels() {
     for (Level* l : levels_) delete l;
+    levels_.clear();
 }
 
 int AmgPreconditioner::levels() const { return static_cast<int>(levels_.size()); }
 long long AmgPreconditioner::coarseRows(int level) const { return levels_.at(level)->n; }
 
 void AmgPreconditioner::buildStructure(const Dcsr<double>& A) {
+    clearLevels();  // what an attempt that failed (stalled coarsening, no memory) left
+    plan_ = TreePlan{};
     HostCsr cur;
     cur.n = A.n;
     cur.ptr.resize(A.n + 1);
@@ -649,6 +654,8 @@ TreeView<float> AmgPreconditioner::treeView32() const {
 
 void AmgPreconditioner::update(const Dcsr<double>& A, bool numeric) {
     if (!built_) buildStructure(A);
+    if (!ready_) numeric = true;
+    ready_ = false;
     fine_ = A;
     Level* l0 = levels_[0];
     l0->dptr = A.ptr; l0->dcol = A.col; l0->ddiag = A.diag; l0->dval = A.val;
@@ -670,6 +677,7 @@ void AmgPreconditioner::update(const Dcsr<double>& A, bool numeric) {
         }
         BSG_CUDA(cudaGetLastError());
         uploadViews();
+        ready_ = true;
         return;
     }
     for (std::size_t l = 0; l + 1 < levels_.size(); ++l) {
@@ -719,6 +727,7 @@ void AmgPreconditioner::update(const Dcsr<double>& A, bool numeric) {
     }
     BSG_CUDA(cudaGetLastError());
     uploadViews();
+    ready_ = true;
 }
 
 void AmgPreconditioner::uploadViews() {

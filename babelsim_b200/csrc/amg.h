@@ -25,8 +25,10 @@ public:
     AmgPreconditioner(DeviceMesh& mesh, const SolverConfig& cfg);
     ~AmgPreconditioner() override;
     // Numeric setup for matrix A (same pattern as the mesh).  The structure is
-    // built on the first call.
+    // built on the first call, which sets the values up whatever `numeric` says.
     void update(const Dcsr<double>& A, bool numeric);
+    // An update has run to its end since the last failure: the hierarchy may be used.
+    bool ready() const { return ready_; }
     void apply(Context& ctx, const double* r, double* z) override;
     int levels() const;
     long long coarseRows(int level) const;
@@ -66,6 +68,7 @@ public:
 
 private:
     void buildStructure(const Dcsr<double>& A);
+    void clearLevels();
     void buildTree(const std::vector<std::vector<int>>& ptr, const std::vector<std::vector<int>>& agg,
                    const int* fine_col);
     void uploadViews();
@@ -75,7 +78,7 @@ private:
     Context& ctx_;
     SolverConfig cfg_;
     std::vector<Level*> levels_;
-    bool built_ = false;
+    bool built_ = false, ready_ = false;
     Dcsr<double> fine_{};
     DeviceArray<AmgLevelView<double>> d_views_;
     bool fp32_ = false;

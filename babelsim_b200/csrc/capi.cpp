@@ -386,7 +386,11 @@ void systemSolve(bsg_system* s, const bsg::SolverConfig& cfg, const double* diag
     bool lagged = false;
     if (use_amg) {
         if (!s->amg) s->amg = std::make_unique<bsg::AmgPreconditioner>(m, cfg);
-        const bool rebuild = s->policy.needRebuild(changed, cfg);
+        bool rebuild = s->policy.needRebuild(changed, cfg);
+        if (!rebuild && !s->amg->ready()) {  // an update that failed left no hierarchy to reuse
+            s->policy.rebuilt();
+            rebuild = true;
+        }
         if (rebuild || changed) s->amg->update(A, rebuild);
         if (rebuild) ++k.preconditioner_setups;
         lagged = s->policy.lagged();
