@@ -362,15 +362,15 @@ constexpr std::size_t kInverseSmem = 200 * 1024;
 
 // CTAs of the cluster inverse's cluster, 0 where none can be had.
 int inverseCtas() {
-    static const int ctas = [] {
+    static PerDevice ctas;
+    return ctas.get(currentDevice(), [] {
         if (cudaFuncSetAttribute(kDenseInverseBlocked, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  static_cast<int>(kInverseSmem)) != cudaSuccess) {
             cudaGetLastError();
             return 0;
         }
         return clusterCtas<kDenseInverseBlocked>(kInvThreads, static_cast<int>(kInverseSmem));
-    }();
-    return ctas;
+    });
 }
 }  // namespace
 

@@ -668,15 +668,6 @@ int chipBytes(const BicgArgs<C, T>& a, int ctas) {
     return bytes <= kChipSmem ? static_cast<int>(bytes) : 0;
 }
 
-template <auto Kernel>
-void allowChip() {
-    static const bool once = [] {
-        BSG_CUDA(cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kChipSmem));
-        return true;
-    }();
-    (void)once;
-}
-
 }  // namespace
 
 template <int C, class T>
@@ -688,7 +679,7 @@ void launchBicgstab(Context& ctx, const BicgArgs<C, T>& args) {
     // streaming kernel's arithmetic (r0 . r of the residual that is kept, the diagonal last), at 0.96 against
     // 0.86 ms for three right-hand sides on 110k cells.
     if constexpr (sizeof(T) == 8) {
-        allowChip<kBicgChipCluster<C, T>>();
+        allowSharedMemory<kBicgChipCluster<C, T>>(kChipSmem);
         a.chip = chipBytes(a, clusterCtas<kBicgChipCluster<C, T>>(CB, kChipSmem));
         if (a.chip && a.A.n <= kClusterRows) {
             launchCluster<kBicgChipCluster<C, T>>(ctx, 1, CB, a.chip, kChipSmem, a);
@@ -702,7 +693,7 @@ void launchBicgstab(Context& ctx, const BicgArgs<C, T>& args) {
     void* params[] = {&a, &bar};
     if constexpr (sizeof(T) == 8) {
         if (a.chip) {
-            allowChip<kBicgChip<C, T>>();
+            allowSharedMemory<kBicgChip<C, T>>(kChipSmem);
             BSG_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(kBicgChip<C, T>), grid, CB, params, a.chip, ctx.stream));
             ctx.launched();
             return;

@@ -9,6 +9,7 @@
 #pragma once
 
 #include "bsg_internal.h"
+#include "per_device.h"
 
 #ifdef __CUDACC__
 #include <cooperative_groups.h>
@@ -188,29 +189,46 @@ __device__ __forceinline__ SplitUnit splitUnit(int u, int K, int lane) {
     return {u / K, (u % K) * rows + lane / K, lane % K};
 }
 
+// The device that attributes set now belong to.
+inline int currentDevice() {
+    int device = 0;
+    BSG_CUDA(cudaGetDevice(&device));
+    return device;
+}
+
+// Lets Kernel take up to `bytes` (the same in every call) of dynamic shared memory on this device.
+template <auto Kernel>
+void allowSharedMemory(int bytes) {
+    static PerDevice done;
+    done.get(currentDevice(), [&] {
+        BSG_CUDA(cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+        return 1;
+    });
+}
+
 // CTAs per cluster for Kernel at `block` threads and up to `smem` bytes of dynamic shared
 // memory: 16 where the device can place such a cluster, else the portable 8.
 template <auto Kernel>
 int clusterCtas(int block, int smem = 0) {
-    static int ctas = 0;
-    if (ctas) return ctas;
-    ctas = 8;
-    if (cudaFuncSetAttribute(Kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3(kMaxClusterCtas);
-        cfg.blockDim = dim3(block);
-        cfg.dynamicSmemBytes = smem;
-        cudaLaunchAttribute at{};
-        at.id = cudaLaunchAttributeClusterDimension;
-        at.val.clusterDim.x = kMaxClusterCtas;
-        at.val.clusterDim.y = at.val.clusterDim.z = 1;
-        cfg.attrs = &at;
-        cfg.numAttrs = 1;
+    static PerDevice ctas;
+    return ctas.get(currentDevice(), [&] {
         int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, Kernel, &cfg) == cudaSuccess && n > 0) ctas = kMaxClusterCtas;
-    }
-    cudaGetLastError();
-    return ctas;
+        if (cudaFuncSetAttribute(Kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
+            cudaLaunchConfig_t cfg{};
+            cfg.gridDim = dim3(kMaxClusterCtas);
+            cfg.blockDim = dim3(block);
+            cfg.dynamicSmemBytes = smem;
+            cudaLaunchAttribute at{};
+            at.id = cudaLaunchAttributeClusterDimension;
+            at.val.clusterDim.x = kMaxClusterCtas;
+            at.val.clusterDim.y = at.val.clusterDim.z = 1;
+            cfg.attrs = &at;
+            cfg.numAttrs = 1;
+            if (cudaOccupancyMaxActiveClusters(&n, Kernel, &cfg) != cudaSuccess) n = 0;
+        }
+        cudaGetLastError();
+        return n > 0 ? kMaxClusterCtas : 8;
+    });
 }
 
 // `clusters` clusters of Kernel on the context's stream, with `smem` (at most `max_smem`) bytes

@@ -860,15 +860,6 @@ __global__ void __launch_bounds__(TB, 1) kPcgTreeCluster(const __grid_constant__
     g.sync();  // every CTA's shared memory is live
     treeBody<TK, TV>(g, a);
 }
-template <auto Kernel>
-void allowRows() {
-    static const bool once = [] {
-        BSG_CUDA(cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTreeSmem));
-        return true;
-    }();
-    (void)once;
-}
-
 template <class TK, class TV>
 void place(const TreePlan& plan, TreePcgArgs<TK, TV>& a, int ctas) {
     const TreePlan::Place p = plan.place(ctas);
@@ -918,13 +909,13 @@ template <class TK, class TV>
 void launchTreePcg(Context& ctx, const TreePlan& plan, TreePcgArgs<TK, TV> a) {
     a.log = PhaseLog{ctx.phase_entries, ctx.phase_capacity, ctx.phase_count};
     if (plan.nnz <= kClusterEntries) {
-        allowRows<kPcgTreeCluster<TK, TV>>();
+        allowSharedMemory<kPcgTreeCluster<TK, TV>>(kTreeSmem);
         place(plan, a, clusterCtas<kPcgTreeCluster<TK, TV>>(TB, kTreeSmem));
         BSG_PROFILE(ctx, "pcg_amg_persistent");
         launchCluster<kPcgTreeCluster<TK, TV>>(ctx, 1, TB, a.smem, kTreeSmem, a);
         return;
     }
-    allowRows<kPcgTree<TK, TV>>();
+    allowSharedMemory<kPcgTree<TK, TV>>(kTreeSmem);
     const int grid = ctx.sm_count;
     place(plan, a, grid);
     SegmentBarrier* bar = ctx.grid_barrier;
@@ -939,7 +930,7 @@ template <class TK, class TV>
 void launchTreePcgBatch(Context& ctx, TreeBatch<TK, TV>& batch) {
     const std::size_t count = batch.args.size();
     if (count == 0) return;
-    allowRows<kPcgTreeBatch<TK, TV>>();
+    allowSharedMemory<kPcgTreeBatch<TK, TV>>(kTreeSmem);
     const std::size_t chunk = std::min(kBatchArgs, ctx.sm_count);
     batch.d_bars.resize(std::max(batch.d_bars.size(), count));
     for (std::size_t k0 = 0; k0 < count; k0 += chunk) {
