@@ -626,21 +626,20 @@ __global__ void __launch_bounds__(BB, 1) kBicgSell(const __grid_constant__ BicgA
     bicgBody<C, T, BB>(g, a);
 }
 
-// Up to kBatchArgs systems as one kernel argument (constant bank: no registers for pointers).
-constexpr int kBatchArgs = 32;
+// The systems of a batched launch as one kernel argument.
 template <int C>
 struct BicgArgsBlock {
     BicgArgs<C> a[kBatchArgs];
     int begin[kBatchArgs + 1];  // CTA ranges
     int count;
 };
+static_assert(sizeof(BicgArgsBlock<3>) + sizeof(void*) <= kKernelArgumentBytes, "one kernel argument");
 
 // A batch: CTAs [begin[s], begin[s+1]) solve system s.
 template <int C>
 __global__ void __launch_bounds__(BB, 1)
     kBicgSellBatch(const __grid_constant__ BicgArgsBlock<C> batch, SegmentBarrier* bars) {
-    int s = 0;  // the system whose CTA range holds this block
-    while (s + 1 < batch.count && batch.begin[s + 1] <= static_cast<int>(blockIdx.x)) ++s;
+    const int s = systemOfBlock(batch.begin, batch.count);
     SegmentGroup g{batch.begin[s], batch.begin[s + 1] - batch.begin[s], bars + s};
     bicgBody<C, double, BB>(g, batch.a[s]);
 }
@@ -708,17 +707,16 @@ void launchBicgstabBatch(Context& ctx, BicgBatch<C>& batch) {
     BSG_PROFILE(ctx, "bicgstab3_persistent_batch");
     const std::size_t count = batch.args.size();
     if (count == 0) return;
-    const std::size_t chunk = std::min(kBatchArgs, ctx.sm_count);
     batch.d_bars.resize(std::max(batch.d_bars.size(), count));
-    for (std::size_t k0 = 0; k0 < count; k0 += chunk) {
+    std::vector<long long> slices(count);
+    for (std::size_t i = 0; i < count; ++i) slices[i] = batch.args[i].A.nslices;
+    const std::vector<std::size_t> launches = batchLaunches(slices, BB / 32, ctx.sm_count);
+    for (std::size_t l = 0; l + 1 < launches.size(); ++l) {
+        const std::size_t k0 = launches[l], k1 = launches[l + 1];
         BicgArgsBlock<C> block{};
-        block.count = static_cast<int>(std::min(chunk, count - k0));
-        std::vector<long long> slices(block.count);
-        for (int i = 0; i < block.count; ++i) {
-            block.a[i] = batch.args[k0 + i];
-            slices[i] = block.a[i].A.nslices;
-        }
-        const std::vector<int> begin = allotCtas(slices, BB / 32, ctx.sm_count);
+        block.count = static_cast<int>(k1 - k0);
+        std::copy(batch.args.begin() + k0, batch.args.begin() + k1, block.a);
+        const std::vector<int> begin = allotCtas({slices.begin() + k0, slices.begin() + k1}, BB / 32, ctx.sm_count);
         std::copy(begin.begin(), begin.end(), block.begin);
         SegmentBarrier* bars = batch.d_bars.data() + k0;
         resetBarriers(ctx, bars, block.count, begin.back(), block.begin);

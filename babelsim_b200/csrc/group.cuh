@@ -11,6 +11,8 @@
 #include "bsg_internal.h"
 #include "per_device.h"
 
+#include <algorithm>
+
 #ifdef __CUDACC__
 #include <cooperative_groups.h>
 #endif
@@ -21,6 +23,11 @@ namespace bsg {
 // this many CTAs (16 is the hardware's non-portable maximum).
 constexpr int kMaxClusterCtas = 16;
 
+// Systems of one batched launch: their arguments are one kernel argument (constant bank: read where they
+// are used they take no registers; from global or shared memory they spilled the solvers' loops), which
+// CUDA limits to kKernelArgumentBytes.
+constexpr int kBatchArgs = 128;
+constexpr std::size_t kKernelArgumentBytes = 32764;
 #ifdef __CUDACC__
 constexpr long long kBarrierCycles = 4000000000LL;  // about 2 s at the B200's clock
 
@@ -359,10 +366,30 @@ __device__ void gridSum(ClusterGroup& g, double v[NV], double*, int& buf) {
 
 #endif
 
+#ifdef __CUDACC__
+// The system whose CTA range [begin[s], begin[s + 1]) holds this block.
+__device__ __forceinline__ int systemOfBlock(const int* begin, int count) {
+    int lo = 0, hi = count - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (begin[mid] <= static_cast<int>(blockIdx.x)) lo = mid;
+        else hi = mid - 1;
+    }
+    return lo;
+}
+#endif
+
 // CTA ranges of a batch's systems in one cooperative launch: begin[i]..begin[i+1], about
 // `slices_per_cta` level-0 slices each and at least one CTA, scaled down in proportion (keeping one each) when
 // the batch exceeds the resident grid.  Within the grid a system's share is its own size's alone,
 // so its arithmetic does not depend on its neighbours.
 std::vector<int> allotCtas(const std::vector<long long>& slices, int slices_per_cta, int capacity);
+
+// The systems of a batch's launches, one after another: [c[i], c[i + 1]).  A launch takes up to kBatchArgs
+// systems (and no more than CTAs), but past kBatchSideBySide of them only while each still gets the CTAs its size
+// asks for: 64 cavities of 512 cells take 0.33 ms for a pressure solve in one launch and 0.65 in two,
+// 64 of 4096 cells, which fill the GPU 37 at a time, 1.60 in one and 1.41 in two.
+constexpr int kBatchSideBySide = 32;
+std::vector<std::size_t> batchLaunches(const std::vector<long long>& slices, int slices_per_cta, int capacity);
 
 }  // namespace bsg

@@ -1043,6 +1043,23 @@ std::vector<int> allotCtas(const std::vector<long long>& slices, int slices_per_
     return begin;
 }
 
+std::vector<std::size_t> batchLaunches(const std::vector<long long>& slices, int slices_per_cta, int capacity) {
+    const std::size_t most = std::max(1, std::min(kBatchArgs, capacity));
+    std::vector<std::size_t> begin{0};
+    long long want = 0;
+    for (std::size_t i = 0; i < slices.size(); ++i) {
+        const long long ctas = std::max<long long>(1, (slices[i] + slices_per_cta - 1) / slices_per_cta);
+        const std::size_t systems = i - begin.back();
+        if (systems == most || (systems >= kBatchSideBySide && want + ctas > capacity)) {
+            begin.push_back(i);
+            want = 0;
+        }
+        want += ctas;
+    }
+    begin.push_back(slices.size());
+    return begin;
+}
+
 void KrylovSolver::solveBatch(Context& ctx, std::vector<BatchSolve>& items) {
     const int K = static_cast<int>(items.size());
     if (K == 0) return;

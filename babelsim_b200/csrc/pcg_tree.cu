@@ -834,22 +834,20 @@ __global__ void __launch_bounds__(TB, 1) kPcgTree(const __grid_constant__ TreePc
     treeBody<TK, TV>(g, a);
 }
 
-// Up to kBatchArgs systems as one kernel argument: read from the constant bank where they are
-// used, they take no registers (from global or shared memory they spilled the solver's loops).
-constexpr int kBatchArgs = 32;
+// The systems of a batched launch as one kernel argument.
 template <class TK, class TV>
 struct TreeArgsBlock {
     TreePcgArgs<TK, TV> a[kBatchArgs];
     int begin[kBatchArgs + 1];  // CTA ranges
     int count;
 };
+static_assert(sizeof(TreeArgsBlock<double, double>) + sizeof(void*) <= kKernelArgumentBytes, "one kernel argument");
 
 // A batch: CTAs [begin[s], begin[s+1]) solve system s.
 template <class TK, class TV>
 __global__ void __launch_bounds__(TB, 1)
     kPcgTreeBatch(const __grid_constant__ TreeArgsBlock<TK, TV> batch, SegmentBarrier* bars) {
-    int s = 0;  // the segment whose CTA range holds this block
-    while (s + 1 < batch.count && batch.begin[s + 1] <= static_cast<int>(blockIdx.x)) ++s;
+    const int s = systemOfBlock(batch.begin, batch.count);
     SegmentGroup g{batch.begin[s], batch.begin[s + 1] - batch.begin[s], bars + s};
     treeBody<TK, TV>(g, batch.a[s]);
 }
@@ -932,14 +930,14 @@ void launchTreePcgBatch(Context& ctx, TreeBatch<TK, TV>& batch) {
     const std::size_t count = batch.args.size();
     if (count == 0) return;
     allowSharedMemory<kPcgTreeBatch<TK, TV>>(kTreeSmem);
-    const std::size_t chunk = std::min(kBatchArgs, ctx.sm_count);
     batch.d_bars.resize(std::max(batch.d_bars.size(), count));
-    for (std::size_t k0 = 0; k0 < count; k0 += chunk) {
+    const std::vector<long long> slices(batch.slices.begin(), batch.slices.end());
+    const std::vector<std::size_t> launches = batchLaunches(slices, TB / 32, ctx.sm_count);
+    for (std::size_t l = 0; l + 1 < launches.size(); ++l) {
+        const std::size_t k0 = launches[l], k1 = launches[l + 1];
         TreeArgsBlock<TK, TV> block{};
-        const int m = block.count = static_cast<int>(std::min(chunk, count - k0));
-        std::vector<long long> slices(m);
-        for (int i = 0; i < m; ++i) slices[i] = batch.slices[k0 + i];
-        const std::vector<int> begin = allotCtas(slices, TB / 32, ctx.sm_count);
+        const int m = block.count = static_cast<int>(k1 - k0);
+        const std::vector<int> begin = allotCtas({slices.begin() + k0, slices.begin() + k1}, TB / 32, ctx.sm_count);
         std::copy(begin.begin(), begin.end(), block.begin);
         int smem = 0;
         for (int i = 0; i < m; ++i) {
