@@ -112,9 +112,19 @@ struct SegmentBarrier {
 
 constexpr int kMaxPersistentCtas = 8192;  // CTAs of one persistent launch, at most
 
+// First of the `ctas` entries of the progress record that a launch takes; `next` is the end of the previous
+// launch's.  Ranges follow one another round the record, so the latest launches' do not overlap.
+inline int takeProgress(int& next, int ctas) {
+    const int at = next + ctas > kMaxPersistentCtas ? 0 : next;
+    next = at + ctas;
+    return at;
+}
+
 struct Context;
 // Sets `n` device barriers to their launch state (no arrivals, no abort, progress
-// recorded in ctx.progress, whose first `ctas` entries are zeroed), in stream order.
+// recorded in the next `ctas` entries of ctx.progress, which are zeroed), in stream order.
+// Each launch takes entries of its own, round the record: a report reads what its launch wrote
+// although others followed before the host looked.
 // Barrier k covers CTAs [cta_begin[k], cta_begin[k+1]); without cta_begin, the one
 // barrier covers all `ctas`.
 void resetBarriers(Context& ctx, SegmentBarrier* dev, int n, int ctas, const int* cta_begin = nullptr);
@@ -133,6 +143,7 @@ struct Context {
     double* pinned = nullptr;            // 64 doubles of pinned host memory
     SegmentBarrier* grid_barrier = nullptr;  // device: the barrier of whole-grid persistent launches
     unsigned* progress = nullptr;            // device, kMaxPersistentCtas: barrier numbers per CTA
+    int progress_next = 0;                   // first entry of the next launch
     // Per-kernel timing: while `profiling`, every instrumented launch is
     // bracketed by two events on `stream`; profileReport() resolves them.
     bool profiling = false;

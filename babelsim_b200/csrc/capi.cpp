@@ -95,14 +95,15 @@ Context::~Context() {
 
 void resetBarriers(Context& ctx, SegmentBarrier* dev, int n, int ctas, const int* cta_begin) {
     if (ctas > kMaxPersistentCtas) fail(kArgument, "persistent launch larger than its progress record");
+    unsigned* progress = ctx.progress + takeProgress(ctx.progress_next, ctas);
     std::vector<SegmentBarrier> h(static_cast<std::size_t>(n));
     for (int k = 0; k < n; ++k) {
         const int c0 = cta_begin ? cta_begin[k] : 0, c1 = cta_begin ? cta_begin[k + 1] : ctas;
-        h[k] = SegmentBarrier{0u, 0, 0, 0u, 0u, c0, c1 - c0, 0, ctx.progress};
+        h[k] = SegmentBarrier{0u, 0, 0, 0u, 0u, c0, c1 - c0, 0, progress};
     }
     // pageable source: the call returns once the bytes are staged, so `h` may go
     BSG_CUDA(cudaMemcpyAsync(dev, h.data(), sizeof(SegmentBarrier) * h.size(), cudaMemcpyHostToDevice, ctx.stream));
-    BSG_CUDA(cudaMemsetAsync(ctx.progress, 0, sizeof(unsigned) * ctas, ctx.stream));
+    BSG_CUDA(cudaMemsetAsync(progress, 0, sizeof(unsigned) * ctas, ctx.stream));
 }
 
 std::string barrierReport(const SegmentBarrier* dev) {
