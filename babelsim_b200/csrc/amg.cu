@@ -395,6 +395,9 @@ AmgPreconditioner::~AmgPreconditioner() { clearLevels(); }
 void AmgPreconditioner::clearLevels() {
     for (Level* l : levels_) delete l;
     levels_.clear();
+    host_ptr_.clear();
+    host_agg_.clear();
+    cg_ready_ = tree_ = false;
 }
 
 int AmgPreconditioner::levels() const { return static_cast<int>(levels_.size()); }
@@ -402,7 +405,6 @@ long long AmgPreconditioner::coarseRows(int level) const { return levels_.at(lev
 
 void AmgPreconditioner::buildStructure(const Dcsr<double>& A) {
     clearLevels();  // what an attempt that failed (stalled coarsening, no memory) left
-    plan_ = TreePlan{};
     HostCsr cur;
     cur.n = A.n;
     cur.ptr.resize(A.n + 1);
@@ -424,7 +426,6 @@ void AmgPreconditioner::buildStructure(const Dcsr<double>& A) {
     l0->nnz = A.nnz_off;
     l0->buildSell(cur.ptr.data(), A.ptr, A.col, ctx_.stream);
     levels_.push_back(l0);
-    std::vector<std::vector<int>> hptr, hagg;  // every level's row pointers and aggregates
     while (cur.n > coarse_target && static_cast<int>(levels_.size()) < max_levels) {
         // aggregates from `passes` rounds of pairwise matching (2 by default: up to 4 rows)
         const int passes = levels_.size() == 1 ? passes0_ : passes_;
@@ -477,12 +478,11 @@ void AmgPreconditioner::buildStructure(const Dcsr<double>& A) {
         lv->buildSell(next.ptr.data(), lv->dptr, lv->dcol, s);
         levels_.push_back(lv);
         ctx_.sync();  // the host arrays go
-        hptr.push_back(std::move(cur.ptr));
-        hagg.push_back(std::move(agg));
+        host_ptr_.push_back(std::move(cur.ptr));
+        host_agg_.push_back(std::move(agg));
         cur = std::move(next);
     }
-    hptr.push_back(std::move(cur.ptr));
-    buildTree(hptr, hagg, A.col);
+    host_ptr_.push_back(std::move(cur.ptr));
     for (Level* l : levels_) {
         l->x.resize(l->n);
         l->b.resize(l->n);
@@ -519,9 +519,20 @@ void AmgPreconditioner::buildStructure(const Dcsr<double>& A) {
     }
 }
 
-void AmgPreconditioner::buildTree(const std::vector<std::vector<int>>& ptr, const std::vector<std::vector<int>>& agg,
-                                  const int* fine_col) {
+void AmgPreconditioner::prepareCg() {
+    if (cg_ready_) return;
+    buildTree();
+    foldCoarse();
+    uploadTree();
+    std::vector<std::vector<int>>().swap(host_ptr_);
+    std::vector<std::vector<int>>().swap(host_agg_);
+    cg_ready_ = true;
+}
+
+void AmgPreconditioner::buildTree() {
+    const std::vector<std::vector<int>>&ptr = host_ptr_, &agg = host_agg_;
     const int L = static_cast<int>(levels_.size());
+    plan_ = TreePlan{};
     tree_ = cfg_.amg_smoothing_steps <= 1 && L <= kMaxTreeLevels;
     if (L < 2 || levels_[0]->n < kTuneRows) tuned_ = true;
     for (int l = 0; tree_ && l + 1 < L; ++l) {
@@ -582,7 +593,7 @@ void AmgPreconditioner::buildTree(const std::vector<std::vector<int>>& ptr, cons
             const int nnz = ptr[l][n];
             lv->t_pcol.resize(std::max(nnz, 1));
             if (nnz > 0) {
-                kGatherInts<<<gridFor(nnz, kBlock), kBlock, 0, s>>>(nnz, l == 0 ? fine_col : lv->dcol, lv->at.data(),
+                kGatherInts<<<gridFor(nnz, kBlock), kBlock, 0, s>>>(nnz, lv->dcol, lv->at.data(),
                                                                    lv->t_pcol.data());
                 BSG_CUDA(cudaGetLastError());
                 ctx_.launched();
@@ -707,7 +718,7 @@ void AmgPreconditioner::update(const Dcsr<double>& A, bool numeric) {
         ctx_.launched();
     }
     BSG_CUDA(cudaGetLastError());
-    foldCoarse();
+    if (cg_ready_) foldCoarse();
     // SELL-32 values for the persistent solver
     const int nn = last->n * last->n;
     if (fp32_) {
@@ -780,7 +791,7 @@ void AmgPreconditioner::uploadViews() {
 }
 
 void AmgPreconditioner::uploadTree() {
-    if (!tree_) return;
+    if (!tree_) return;  // also before prepareCg
     const int L = static_cast<int>(levels_.size());
     std::vector<TreeLevel> t(L);
     std::vector<double*> v64(3 * L, nullptr);

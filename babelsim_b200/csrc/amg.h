@@ -48,8 +48,10 @@ public:
     double sellVcycleBytes() const;
     long long krylovEntries() const;  // padded level-0 SELL entries
 
-    // The tree numbering of the coarse levels (pcg_tree.cuh): built for one smoothing step and
-    // aggregates of at most four rows.
+    // What only the persistent CG solvers read, built before their first solve: the tree numbering of the
+    // coarse levels (pcg_tree.cuh; for one smoothing step and aggregates of at most four rows) and the folded
+    // coarse matrix.  GMRES, which applies the V-cycle level by level, never asks for it.
+    void prepareCg();
     bool hasTree() const { return tree_; }
     const TreePlan& treePlan() const { return plan_; }
     int treePositions() const;  // entries the Krylov vectors need (rows of level 0, or its positions)
@@ -69,8 +71,7 @@ public:
 private:
     void buildStructure(const Dcsr<double>& A);
     void clearLevels();
-    void buildTree(const std::vector<std::vector<int>>& ptr, const std::vector<std::vector<int>>& agg,
-                   const int* fine_col);
+    void buildTree();
     void uploadViews();
     void uploadTree();
     void foldCoarse();
@@ -86,7 +87,8 @@ private:
     DeviceArray<VLevel<double>> d_vl64_;
     DeviceArray<VLevel<float>> d_vl32_;
     DeviceArray<float> dense32_;
-    bool tree_ = false, tuned_ = false;
+    std::vector<std::vector<int>> host_ptr_, host_agg_;  // levels' row pointers and aggregates, until prepareCg
+    bool cg_ready_ = false, tree_ = false, tuned_ = false;
     TreePlan plan_;
     DeviceArray<double> fold_y_, folded_;  // foldCoarse
     DeviceArray<float> folded32_;

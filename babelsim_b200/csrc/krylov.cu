@@ -830,6 +830,7 @@ SolveOutcome KrylovSolver::solvePersistent(const Dcsr<double>& A, const SolverCo
     Impl& m = *impl_;
     Context& ctx = m.ctx;
     const int n = A.n;
+    if (amg) amg->prepareCg();
     if (cfg.precision == 1 && amg && amg->fp32VCycle()) return solveRefined(A, cfg, amg, b, x);
     if (amg && amg->hasTree()) m.ensureTree(amg->treePositions());
     else m.ensure(n);
@@ -1076,6 +1077,7 @@ void KrylovSolver::solveBatch(Context& ctx, std::vector<BatchSolve>& items) {
             fail(kArgument, "batched solves take CG with the AMG preconditioner in FP64 or with an FP32 V-cycle");
         Impl& m = *it.solver->impl_;
         if (&m.ctx != &ctx) fail(kArgument, "batched solves must share one context");
+        it.amg->prepareCg();
         if (it.amg->hasTree()) m.ensureTree(it.amg->treePositions());
         else m.ensure(it.A.n);
         if (it.amg->wantsTuning()) it.solver->tuneCorrection(it.A, *it.amg);
