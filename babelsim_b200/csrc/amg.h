@@ -90,8 +90,9 @@ private:
     std::vector<std::vector<int>> host_ptr_, host_agg_;  // levels' row pointers and aggregates, until prepareCg
     bool cg_ready_ = false, tree_ = false, tuned_ = false;
     TreePlan plan_;
-    DeviceArray<double> fold_y_, folded_;  // foldCoarse
-    DeviceArray<float> folded32_;
+    DeviceArray<char> tree_store_;         // everything buildTree makes
+    double *fold_y_ = nullptr, *folded_ = nullptr;  // foldCoarse
+    float* folded32_ = nullptr;
     DeviceArray<double> inv_panel_;        // kDenseInverseBlocked's panel, two halves
     DeviceArray<TreeLevel> d_tree_;
     DeviceArray<double*> d_tvec64_;

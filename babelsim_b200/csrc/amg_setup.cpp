@@ -222,4 +222,27 @@ TreeMaps treeMaps(int n, const Members& members, std::vector<int>& order) {
     return t;
 }
 
+double paddedEntries(const TreeMaps& t, const std::vector<int>& ptr) {
+    const int npos = static_cast<int>(t.row.size()), slices = (npos + 31) / 32;
+    std::vector<long long> sums(hostThreads(), 0);
+    parallelRanges(slices, kGrain / 32, [&](int s0, int s1, int thread) {
+        long long sum = 0;
+        for (int s = s0; s < s1; ++s) {
+            int w = 0;
+            for (int p = 32 * s; p < std::min(npos, 32 * (s + 1)); ++p)
+                if (t.row[p] >= 0) w = std::max(w, ptr[t.row[p] + 1] - ptr[t.row[p]]);
+            sum += w;
+        }
+        sums[thread] = sum;
+    });
+    return 32.0 * static_cast<double>(std::accumulate(sums.begin(), sums.end(), 0LL));
+}
+
+void membersByPosition(const TreeMaps& t, const Members& members, int* out) {
+    parallelRanges(static_cast<int>(t.row.size()), kGrain, [&](int p0, int p1, int) {
+        for (int p = p0; p < p1; ++p)
+            if (t.row[p] >= 0) std::copy(members[t.row[p]].begin(), members[t.row[p]].end(), out + 4 * static_cast<std::size_t>(p));
+    });
+}
+
 }  // namespace bsg

@@ -44,5 +44,9 @@ struct TreeMaps {
 using Members = std::vector<std::array<int, 4>>;  // a coarse row's fine rows, -1 past the last
 Members membersOf(const std::vector<int>& agg, int nc);
 TreeMaps treeMaps(int n, const Members& members, std::vector<int>& order);
+// Entries of the level's rows by position, padded to the widest row of every 32 positions.
+double paddedEntries(const TreeMaps& t, const std::vector<int>& ptr);
+// out[4 p ..]: the members of the row at position p; holes are left as they are.
+void membersByPosition(const TreeMaps& t, const Members& members, int* out);
 
 }  // namespace bsg

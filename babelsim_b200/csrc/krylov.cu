@@ -783,9 +783,12 @@ void KrylovSolver::tuneCorrection(const Dcsr<double>& A, AmgPreconditioner& amg)
     if (m.pst.size() < 1) m.pst.resize(1);
     kSigns<<<gridFor(A.n, kBlock), kBlock, 0, ctx.stream>>>(A.n, m.t.data());
     ctx.launched();
-    const auto reduction = [&]() -> double {
+    // the residual's reduction; a trial that may stop there ends once it has gained `enough`
+    const auto reduction = [&](double enough) -> double {
         PcgState h{};
         h.max_iterations = kTrialIterations;
+        h.target2 = enough > 0.0 ? -1.0 : 0.0;
+        h.rtol = enough;
         BSG_CUDA(cudaMemcpyAsync(m.pst.data(), &h, sizeof(h), cudaMemcpyHostToDevice, ctx.stream));
         launchTree(amg, A.n, m.t.data(), m.tmp.data());
         BSG_CUDA(cudaMemcpyAsync(ctx.pinned, m.pst.data(), sizeof(PcgState), cudaMemcpyDeviceToHost, ctx.stream));
@@ -794,14 +797,14 @@ void KrylovSolver::tuneCorrection(const Dcsr<double>& A, AmgPreconditioner& amg)
         std::memcpy(&r, ctx.pinned, sizeof(r));
         if (r.status == 3)
             fail(kCuda, "persistent PCG: a barrier wait ran past its bound" + barrierReport(ctx.grid_barrier));
-        return r.status == 1 && r.rr0 > 0.0 && std::isfinite(r.rr) ? std::sqrt(r.rr / r.rr0) : -1.0;
+        return r.status < 2 && r.rr0 > 0.0 && std::isfinite(r.rr) ? std::sqrt(r.rr / r.rr0) : -1.0;
     };
     const double start = amg.correction();
-    double chosen = start, best = reduction();
-    if (best < kTrialGood) return;  // good, or no measure (breakdown)
+    double chosen = start, best = reduction(kTrialGood);
+    if (best <= kTrialGood) return;  // good, or no measure (breakdown)
     for (const double gamma : {1.2, 1.5}) {
         amg.setCorrection(gamma);
-        const double r = reduction();
+        const double r = reduction(0.0);
         if (r >= 0.0 && r < best) {
             best = r;
             chosen = gamma;
