@@ -655,10 +655,10 @@ constexpr int kClusterRows = 8192;
 // Bytes of shared memory per CTA that hold the system's rows and vectors on `ctas` CTAs; 0 where there
 // is no room (keeping the rows alone was tried: 110k-cell Voronoi cube 1.24 ms against 1.06 streamed).
 template <int C, class T>
-int chipBytes(const BicgArgs<C, T>& a, int ctas) {
-    const int per = (a.A.nslices + ctas - 1) / ctas;  // slices of the fullest CTA
+int chipBytes(int nslices, long long entries, int ctas) {
+    const int per = (nslices + ctas - 1) / ctas;  // slices of the fullest CTA
     const int k = chipLanes(per);
-    const double wide = a.A.nslices > 0 ? static_cast<double>(a.entries) / (32.0 * a.A.nslices) : 0.0;
+    const double wide = nslices > 0 ? static_cast<double>(entries) / (32.0 * nslices) : 0.0;
     const double steps = k == 0 ? wide : wide / (1 << k) + 0.5;
     // a few per cent for slices wider than the mean (a unit that does not fit is read from memory)
     const double rows = 1.06 * (per << k) * steps * 32.0 * (sizeof(T) + 4.0) + 2048.0;
@@ -667,7 +667,27 @@ int chipBytes(const BicgArgs<C, T>& a, int ctas) {
     return bytes <= kChipSmem ? static_cast<int>(bytes) : 0;
 }
 
+// Where a system runs on chip: the bytes per CTA of a cluster or of the grid (0: streamed).
+struct ChipPlace {
+    bool cluster;
+    int bytes;
+};
+template <int C, class T>
+ChipPlace chipPlace(Context& ctx, const SellMat<T>& A, long long entries) {
+    if (A.n <= kClusterRows) {
+        allowSharedMemory<kBicgChipCluster<C, T>>(kChipSmem);
+        const int bytes = chipBytes<C, T>(A.nslices, entries, clusterCtas<kBicgChipCluster<C, T>>(CB, kChipSmem));
+        if (bytes) return {true, bytes};
+    }
+    return {false, chipBytes<C, T>(A.nslices, entries, ctx.sm_count)};
+}
+
 }  // namespace
+
+template <int C>
+bool bicgstabOnChip(Context& ctx, const SellMat<double>& A, long long entries) {
+    return chipPlace<C, double>(ctx, A, entries).bytes > 0;
+}
 
 template <int C, class T>
 void launchBicgstab(Context& ctx, const BicgArgs<C, T>& args) {
@@ -678,13 +698,12 @@ void launchBicgstab(Context& ctx, const BicgArgs<C, T>& args) {
     // streaming kernel's arithmetic (r0 . r of the residual that is kept, the diagonal last), at 0.96 against
     // 0.86 ms for three right-hand sides on 110k cells.
     if constexpr (sizeof(T) == 8) {
-        allowSharedMemory<kBicgChipCluster<C, T>>(kChipSmem);
-        a.chip = chipBytes(a, clusterCtas<kBicgChipCluster<C, T>>(CB, kChipSmem));
-        if (a.chip && a.A.n <= kClusterRows) {
+        const ChipPlace place = chipPlace<C, T>(ctx, a.A, a.entries);
+        a.chip = place.bytes;
+        if (place.cluster) {
             launchCluster<kBicgChipCluster<C, T>>(ctx, 1, CB, a.chip, kChipSmem, a);
             return;
         }
-        a.chip = chipBytes(a, ctx.sm_count);
     }
     SegmentBarrier* bar = ctx.grid_barrier;
     const int grid = ctx.sm_count;
@@ -728,6 +747,8 @@ void launchBicgstabBatch(Context& ctx, BicgBatch<C>& batch) {
     batch.bars_used = static_cast<int>(count);
 }
 
+template bool bicgstabOnChip<3>(Context&, const SellMat<double>&, long long);
+template bool bicgstabOnChip<1>(Context&, const SellMat<double>&, long long);
 template void launchBicgstab<3, double>(Context&, const BicgArgs<3, double>&);
 template void launchBicgstab<1, double>(Context&, const BicgArgs<1, double>&);
 template void launchBicgstab<3, float>(Context&, const BicgArgs<3, float>&);

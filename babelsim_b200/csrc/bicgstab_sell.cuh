@@ -60,6 +60,11 @@ struct BicgBatch {
     int bars_used = 0;  // barriers of the last launch, for its error report
 };
 
+// Whether launchBicgstab keeps an FP64 system with `entries` padded SELL entries on chip, where it needs gph
+// and gsh.
+template <int C>
+bool bicgstabOnChip(Context& ctx, const SellMat<double>& A, long long entries);
+
 // One system, on one thread-block cluster when it is small, else on the whole grid.
 template <int C, class T>
 void launchBicgstab(Context& ctx, const BicgArgs<C, T>& args);

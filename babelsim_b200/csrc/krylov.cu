@@ -585,10 +585,12 @@ struct KrylovSolver::Impl {
         const long long g = (static_cast<long long>(n) + kBlock - 1) / kBlock;
         return static_cast<int>(std::max<long long>(1, std::min<long long>(g, 4LL * ctx.sm_count)));
     }
-    void ensureTree(std::size_t n) {
+    // Vectors of the tree solver; a hierarchy whose level 0 streams in every launch uses the first two pairs only.
+    void ensureTree(const AmgPreconditioner& amg) {
+        const std::size_t n = amg.treePositions();
         ensure(n);
-        for (DeviceArray<double2>& a : pair)
-            if (a.size() < n) a.resize(n);
+        for (int k = 0; k < (amg.treePlan().first == 0 ? 4 : 2); ++k)
+            if (pair[k].size() < n) pair[k].resize(n);
     }
     void ensure(std::size_t n) {
         for (DeviceArray<double>* a : {&r, &z, &p, &q, &r0, &v, &ph, &sh, &t, &tmp})
@@ -681,8 +683,8 @@ SolveOutcome KrylovSolver::solveRefined(const Dcsr<double>& A, const SolverConfi
         if (a->size() < entries) a->resize(entries);
     if (amg->hasTree()) {
         if (m.x32.size() < entries) m.x32.resize(entries);
-        for (DeviceArray<float2>& a : m.pair32)
-            if (a.size() < entries) a.resize(entries);
+        for (int k = 0; k < (amg->treePlan().first == 0 ? 4 : 2); ++k)
+            if (m.pair32[k].size() < entries) m.pair32[k].resize(entries);
     } else {
         for (DeviceArray<float>* a : {&m.z32, &m.p32a, &m.p32b})
             if (a->size() < entries) a->resize(entries);
@@ -779,7 +781,7 @@ void KrylovSolver::tuneCorrection(const Dcsr<double>& A, AmgPreconditioner& amg)
     Impl& m = *impl_;
     Context& ctx = m.ctx;
     amg.tuned();
-    m.ensureTree(amg.treePositions());
+    m.ensureTree(amg);
     if (m.pst.size() < 1) m.pst.resize(1);
     kSigns<<<gridFor(A.n, kBlock), kBlock, 0, ctx.stream>>>(A.n, m.t.data());
     ctx.launched();
@@ -835,7 +837,7 @@ SolveOutcome KrylovSolver::solvePersistent(const Dcsr<double>& A, const SolverCo
     const int n = A.n;
     if (amg) amg->prepareCg();
     if (cfg.precision == 1 && amg && amg->fp32VCycle()) return solveRefined(A, cfg, amg, b, x);
-    if (amg && amg->hasTree()) m.ensureTree(amg->treePositions());
+    if (amg && amg->hasTree()) m.ensureTree(*amg);
     else m.ensure(n);
     if (amg && amg->wantsTuning()) tuneCorrection(A, *amg);
     if (m.pst.size() < 1) m.pst.resize(1);
@@ -1081,7 +1083,7 @@ void KrylovSolver::solveBatch(Context& ctx, std::vector<BatchSolve>& items) {
         Impl& m = *it.solver->impl_;
         if (&m.ctx != &ctx) fail(kArgument, "batched solves must share one context");
         it.amg->prepareCg();
-        if (it.amg->hasTree()) m.ensureTree(it.amg->treePositions());
+        if (it.amg->hasTree()) m.ensureTree(*it.amg);
         else m.ensure(it.A.n);
         if (it.amg->wantsTuning()) it.solver->tuneCorrection(it.A, *it.amg);
         if (m.pst.size() < 1) m.pst.resize(1);
@@ -1233,10 +1235,12 @@ void KrylovSolver::persistentBicgstab(Context& ctx, std::vector<BicgItem>& items
         Impl& m = *it.solver->impl_;
         const int n = it.A.n;
         m.ensure(C * static_cast<std::size_t>(n));
-        for (DeviceArray<double>* a : {&m.gph, &m.gsh})
-            if (a->size() < kGatherStride<C> * static_cast<std::size_t>(n)) a->resize(kGatherStride<C> * static_cast<std::size_t>(n));
         if (m.bst.size() < 1) m.bst.resize(1);
         sell[k] = m.sellOf(it.A);
+        if (!batched && bicgstabOnChip<C>(ctx, sell[k], static_cast<long long>(m.sell.sval.size())))
+            for (DeviceArray<double>* a : {&m.gph, &m.gsh})
+                if (a->size() < kGatherStride<C> * static_cast<std::size_t>(n))
+                    a->resize(kGatherStride<C> * static_cast<std::size_t>(n));
         if (!it.cfg.warm_start) BSG_CUDA(cudaMemsetAsync(it.x, 0, sizeof(double) * C * n, ctx.stream));
         BicgState& h = t[k].h;
         for (int c = 0; c < C; ++c) {

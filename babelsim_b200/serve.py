@@ -59,15 +59,17 @@ class Result:
 
 
 def device_bytes(n_cells: int, n_faces: int) -> int:
-    """Device-memory estimate of one resident SIMPLE solve: geometry (152 B per face,
-    40 B per cell), fields and workspaces (~60 doubles per cell), two LDU systems on
-    the cell-to-face pattern, the AMG hierarchy with its SELL copies (~1.6x the
-    level-0 matrix), the SELL copy of the momentum matrix (~1.3x its off-diagonal
-    entries, 12 B each), the per-slot records of the diffusion face pass (64 B per
-    face) and Krylov workspaces."""
-    matrix = 8 * n_cells + 12 * 2 * n_faces
-    return int(152 * n_faces + 40 * n_cells + 480 * n_cells + 2 * matrix + 1.6 * (matrix + 8 * 2 * n_faces) +
-               1.3 * 12 * 2 * n_faces + 64 * n_faces + 16 * 8 * n_cells)
+    """Device-memory bound of one resident SIMPLE solve, linear in its mesh so that admission stays so.
+
+    Per face: geometry 152 B, two LDU systems 48, the AMG hierarchy with its SELL copies 64, the SELL copy of
+    the momentum matrix 31, the records of the diffusion face pass 64, column positions of the on-chip
+    CG 8, and what the allocator rounds up.  Per cell: geometry, fields and workspaces 520 B, diagonals 30,
+    Krylov vectors 320 (ten of three components and of one), the on-chip solvers' gathered vectors,
+    positions, maps and level vectors 300, and again the rounding, which is up to half of an array of one to
+    four MB.  4 MB for the coarsest levels.  Held against bound, MB: hex cubes of 13.8k cells 36 / 42, 111k
+    281 / 305, 1M 1900 / 2716 (its finest level has no on-chip copy); Voronoi cubes of 8k cells 35 / 40,
+    64k 274 / 293."""
+    return int(1500 * n_cells + 400 * n_faces + 4e6)
 
 
 def shard(requests: list[Request], world: int, rank: int) -> list[Request]:
