@@ -7,6 +7,7 @@
 // reads a convergence word every `check_interval` iterations; kernels of
 // iterations issued after convergence return immediately.
 #include "amg.h"
+#include "amg_scale.h"
 #include "bicgstab_sell.cuh"
 #include "pcg_sell.cuh"
 #include "pcg_tree.cuh"
@@ -766,8 +767,6 @@ __global__ void kSigns(int n, double* __restrict__ b) {
     b[i] = (h & 1u) ? 1.0 : -1.0;
 }
 constexpr int kTrialIterations = 24;
-// A hierarchy that gains this much in a trial converges fast enough as it is (1e-10 in about 50).
-constexpr double kTrialGood = 3e-5;
 }  // namespace
 
 // The coarse-correction scale of a new hierarchy.  Unsmoothed aggregation under-corrects smooth error;
@@ -785,8 +784,8 @@ void KrylovSolver::tuneCorrection(const Dcsr<double>& A, AmgPreconditioner& amg)
     if (m.pst.size() < 1) m.pst.resize(1);
     kSigns<<<gridFor(A.n, kBlock), kBlock, 0, ctx.stream>>>(A.n, m.t.data());
     ctx.launched();
-    // the residual's reduction; a trial that may stop there ends once it has gained `enough`
-    const auto reduction = [&](double enough) -> double {
+    const double chosen = chooseCorrection(amg.correction(), [&](double scale, double enough) {
+        if (scale != amg.correction()) amg.setCorrection(scale);
         PcgState h{};
         h.max_iterations = kTrialIterations;
         h.target2 = enough > 0.0 ? -1.0 : 0.0;
@@ -799,20 +798,9 @@ void KrylovSolver::tuneCorrection(const Dcsr<double>& A, AmgPreconditioner& amg)
         std::memcpy(&r, ctx.pinned, sizeof(r));
         if (r.status == 3)
             fail(kCuda, "persistent PCG: a barrier wait ran past its bound" + barrierReport(ctx.grid_barrier));
-        return r.status < 2 && r.rr0 > 0.0 && std::isfinite(r.rr) ? std::sqrt(r.rr / r.rr0) : -1.0;
-    };
-    const double start = amg.correction();
-    double chosen = start, best = reduction(kTrialGood);
-    if (best <= kTrialGood) return;  // good, or no measure (breakdown)
-    for (const double gamma : {1.2, 1.5}) {
-        amg.setCorrection(gamma);
-        const double r = reduction(0.0);
-        if (r >= 0.0 && r < best) {
-            best = r;
-            chosen = gamma;
-        }
-    }
-    amg.setCorrection(chosen);
+        return r.status < 2 && r.rr0 > 0.0 && std::isfinite(r.rr) ? std::sqrt(r.rr / r.rr0) : kTrialFailed;
+    });
+    if (chosen != amg.correction()) amg.setCorrection(chosen);
 }
 
 // The tree solver on this solver's workspace (FP64 Krylov vectors and products; an FP32 V-cycle takes
@@ -836,6 +824,8 @@ SolveOutcome KrylovSolver::solvePersistent(const Dcsr<double>& A, const SolverCo
     Context& ctx = m.ctx;
     const int n = A.n;
     if (amg) amg->prepareCg();
+    // (the FP32 inner solves keep the start scale, with which precision 1 has always given its fields: which
+    // iterate a refinement accepts depends on the cycle)
     if (cfg.precision == 1 && amg && amg->fp32VCycle()) return solveRefined(A, cfg, amg, b, x);
     if (amg && amg->hasTree()) m.ensureTree(*amg);
     else m.ensure(n);
