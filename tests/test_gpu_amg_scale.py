@@ -1,0 +1,74 @@
+"""The AMG correction scale on stretched couplings, through the linear-system seam: a stretched box gets another
+scale than the isotropic one's and needs fewer iterations for it, the isotropic one keeps the fixed scale, and a
+system whose matrices change from one kind to the other takes no more iterations than with the fixed scale (its
+aggregates are the first matrix's in either case).
+
+Bounds: the accepted true residual with 1 % for its recomputation; at least a tenth fewer iterations where the
+scale moves; after a change of kind at most 1.1 times those of the fixed scale plus three."""
+import numpy as np
+import pytest
+
+from babelsim_b200 import meshgen
+
+pytestmark = pytest.mark.gpu
+RTOL = 1e-10
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    import babelsim_b200 as bsg
+    c = bsg.Context(0)
+    yield c
+    c.close()
+
+
+def _system(shape, weights, seed):
+    poly = meshgen.hex_box(*shape, flat=True)
+    own, nbr = np.asarray(poly.owner, np.int64), np.asarray(poly.neighbour, np.int64)
+    inner, n = nbr >= 0, poly.n_cells
+    rng = np.random.default_rng(seed)
+    axis = np.where(nbr - own == 1, 0, np.where(nbr - own == shape[0], 1, 2))
+    c = np.where(inner, np.asarray(weights)[axis] * np.exp(0.3 * rng.standard_normal(len(own))), 0.0)
+    d = np.full(n, 1e-3)
+    np.add.at(d, own[inner], c[inner])
+    np.add.at(d, nbr[inner], c[inner])
+    return d, -c, rng.standard_normal(n), inner, own, nbr
+
+
+def _solve(system, matrix, precision):
+    import babelsim_b200 as bsg
+    d, up, b, inner, own, nbr = matrix
+    cfg = bsg.solver_config("cg", "hypre", 1e-30, RTOL, 3000, precision=precision, rebuild_interval=1)
+    x, res = system.solve(cfg, d, up, up, b)
+    y = d * x
+    np.add.at(y, own[inner], up[inner] * x[nbr[inner]])
+    np.add.at(y, nbr[inner], up[inner] * x[own[inner]])
+    assert res[0].status == 0
+    assert np.linalg.norm(b - y) <= 1.01 * RTOL * np.linalg.norm(b)
+    return res[0].iterations
+
+
+@pytest.mark.parametrize("precision", [0, 2])
+@pytest.mark.parametrize("shape,weights", [((48, 48, 48), (1, 1, 100)), ((60, 50, 40), (1, 1000, 30))])
+def test_scale_and_iterations(ctx, monkeypatch, shape, weights, precision):
+    import babelsim_b200 as bsg
+    mesh = bsg.Mesh.from_polyhedral(ctx, meshgen.hex_box(*shape, flat=True))
+    kinds = {"plain": (1, 1, 1), "stretched": weights}
+
+    def sequence(names, fixed=None):
+        if fixed:
+            monkeypatch.setenv("BSG_AMG_GAMMA", fixed)
+        system = bsg.LinearSystem(mesh)
+        counts = [_solve(system, _system(shape, kinds[k], seed), precision) for seed, k in enumerate(names)]
+        system.close()
+        monkeypatch.delenv("BSG_AMG_GAMMA", raising=False)
+        return counts
+    fresh = {k: sequence([k])[0] for k in kinds}
+    assert fresh["stretched"] <= 0.9 * sequence(["stretched"], "1.8")[0]  # the trial moved the scale
+    assert sequence(["plain"], "1.8")[0] == fresh["plain"]                # and left it here
+    for first, then in (("plain", "stretched"), ("stretched", "plain")):
+        names = [first] + 3 * [then]
+        fixed = sequence(names, "1.8")
+        for n, f in zip(sequence(names)[2:], fixed[2:]):
+            assert n <= 1.1 * f + 3
+    mesh.close()
