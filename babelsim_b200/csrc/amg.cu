@@ -917,6 +917,48 @@ double AmgPreconditioner::sellVcycleBytes() const {
     return bytes;
 }
 
+double AmgPreconditioner::treeSolveBytes(const TreePlan::Place& place, int value, int iterations, bool warm,
+                                         bool started) const {
+    const int levels = place.levels, top = place.top;
+    const double s = fp32_ ? 4.0 : 8.0, k = value, N = levels_[0]->n, it = iterations;
+    const double applications = started ? std::max(1.0, it) : 0.0;
+    const auto rows = [&](int l) { return static_cast<double>(levels_[l]->n); };
+    const auto sweep = [&](int l, double v) {  // one pass over a streamed level's matrix and diagonal
+        const Level* f = levels_[l];
+        return (4.0 + v) * static_cast<double>(f->sell_entries) + 4.0 * (f->nslices + 1) + v * f->n;
+    };
+    double once = 0.0, cycle = 0.0;
+    for (int l = top; l < levels - 1; ++l) {  // CSR row, column positions, diagonals and maps, to shared memory
+        const Level* f = levels_[l];
+        once += 12.0 * static_cast<double>(f->nnz) + 16.0 * f->n + 16.0 * f->npos;
+    }
+    if (levels == 1) {  // the dense inverse alone
+        cycle = s * N * N + (k + s) * N;
+    } else {
+        for (int l = 0; l < top; ++l) {  // levels streamed in their own numbering
+            const double n = rows(l), nc = rows(l + 1);
+            if (l > 0) cycle += sweep(l, s) + 3.0 * s * n;               // w (gathered), b read; t written
+            cycle += s * n + (l + 1 < top ? 4.0 * (nc + 1) + 4.0 * n + 3.0 * s * nc   // lists, t, rd read; b, w written
+                                          : 16.0 * plan_.positions[l + 1] + 2.0 * s * nc);
+            cycle += (l + 1 < top ? 4.0 * (nc + 1) + 4.0 * n : 16.0 * plan_.positions[l + 1]) + 2.0 * s * n;  // pushes
+            cycle += l > 0 ? sweep(l, s) + 4.0 * s * n                   // y (gathered), rd, b read
+                           : sweep(0, s) + 3.0 * s * n + 2.0 * k * n;    // and r for r . z, z written
+        }
+        for (int l = std::max(top, 1); l < levels - 1; ++l)              // b, w twice, e(coarse) read; b, w(coarse), e written
+            cycle += 5.0 * s * rows(l) + 3.0 * s * rows(l + 1);
+        const int c = levels - 1;                                        // dense matrix, b read, e written
+        cycle += s * (rows(c) * (c + 1 < static_cast<int>(levels_.size()) ? plan_.positions[c] : rows(c)) + 2.0 * rows(c));
+        if (top == 0) cycle += (2.0 * k + s) * N + s * rows(1);          // w, e(coarse), r read; z written
+    }
+    // per iteration: the product ({z, p} read; p, q and omega/d q written) and the update with the next residual
+    const double iteration = top == 0 && levels > 1
+                                 ? (2.0 + 3.0) * k * N + (4.0 + 2.0 + 3.0) * k * N + s * N + 2.0 * s * rows(1)
+                                 : sweep(0, k) + 4.0 * k * N + (levels > 1 ? sweep(0, s) + 6.0 * k * N + 4.0 * s * N : 6.0 * k * N);
+    const double first = (warm ? (top == 0 && levels > 1 ? 0.0 : sweep(0, k)) + 4.0 * k * N : 3.0 * k * N) +
+                         (started && levels > 1 ? (top == 0 ? k * N : sweep(0, s)) + 2.0 * s * N : 0.0);
+    return once + first + applications * cycle + it * iteration;
+}
+
 AmgView<double> AmgPreconditioner::deviceView() const {
     AmgView<double> v;
     v.levels = static_cast<int>(levels_.size());

@@ -46,6 +46,10 @@ public:
     VCycleView<double> sellView64() const;
     VCycleView<float> sellView32() const;
     double sellVcycleBytes() const;
+    // Algorithmic bytes of one launch of the tree solver at `place`, with Krylov values of `value` bytes: rows kept
+    // on chip are read once per launch, the folded matrix stands for the levels it replaces, every other array
+    // counts in each phase that reads or writes it.  `started`: the launch got past its first residual.
+    double treeSolveBytes(const TreePlan::Place& place, int value, int iterations, bool warm, bool started) const;
     long long krylovEntries() const;  // padded level-0 SELL entries
 
     // What only the persistent CG solvers read, built before their first solve: the tree numbering of the

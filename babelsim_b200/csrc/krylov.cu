@@ -536,6 +536,7 @@ struct KrylovSolver::Impl {
     DeviceArray<float> r32, s32, z32, p32a, p32b, q32, d32, x32;  // FP32 inner solve of the refined path
     DeviceArray<double2> pair[4];  // the tree solver's paired vectors (pcg_tree.cuh)
     DeviceArray<float2> pair32[4];
+    TreePlan::Place tree_place{};  // of the last launch, for its declared bytes
     // FP32 inner BiCGStab of the refined path: matrix copy (SELL values, diagonal) and
     // the C-interleaved right-hand side, correction and Krylov vectors
     DeviceArray<float> bval32, bdiag32, bb32, bx32, br32, br032, bp32, bv32, bph32, bsh32, bt32;
@@ -714,7 +715,7 @@ SolveOutcome KrylovSolver::solveRefined(const Dcsr<double>& A, const SolverConfi
         h.rtol = cfg.rtol;
         BSG_CUDA(cudaMemcpyAsync(m.pst.data(), &h, sizeof(h), cudaMemcpyHostToDevice, ctx.stream));
         if (amg->hasTree()) {
-            launchTreePcg<float, float>(ctx, amg->treePlan(),
+            m.tree_place = launchTreePcg<float, float>(ctx, amg->treePlan(),
                                         {amg->krylovMatrix32(), amg->treeView32(), 0, n, m.r32.data(), m.d32.data(),
                                          m.s32.data(), m.q32.data(), m.x32.data(), m.pair32[0].data(),
                                          m.pair32[1].data(), m.pair32[2].data(), m.pair32[3].data(), m.partial.data(),
@@ -739,8 +740,10 @@ SolveOutcome KrylovSolver::solveRefined(const Dcsr<double>& A, const SolverConfi
         if (ctx.profiling || trace_solves()) {
             const double N = n;
             const double M0 = 8.0 * N + 4.0 * (amg->krylovMatrix32().nslices + 1) + 8.0 * static_cast<double>(amg->krylovEntries());
-            const double bytes = 12.0 * N + (r.iterations > 0 ? r.iterations : 1) * (amg->sellVcycleBytes() + 8.0 * N) +
-                                 r.iterations * (M0 + 40.0 * N);
+            const double bytes =
+                amg->hasTree() ? amg->treeSolveBytes(m.tree_place, 4, r.iterations, false, r.iterations > 0 || r.status != 0)
+                               : 12.0 * N + (r.iterations > 0 ? r.iterations : 1) * (amg->sellVcycleBytes() + 8.0 * N) +
+                                     r.iterations * (M0 + 40.0 * N);
             ctx.profileNote("pcg_amg_persistent", bytes, r.iterations);
             if (trace_solves())
                 std::fprintf(stderr, "bsg refined pcg (fp32 inner): rows %d iterations %d residual %.3e -> %.3e\n", n,
@@ -812,10 +815,10 @@ void KrylovSolver::launchTree(AmgPreconditioner& amg, int n, const double* b, do
     Impl& m = *impl_;
     const auto solve = [&](auto view, int flexible) {
         using TV = std::decay_t<decltype(view.gamma)>;
-        launchTreePcg<double, TV>(m.ctx, amg.treePlan(),
-                                  {amg.krylovMatrix(), view, 0, n, b, x, m.r.data(), m.q.data(), m.ph.data(),
-                                   m.pair[0].data(), m.pair[1].data(), m.pair[2].data(), m.pair[3].data(),
-                                   m.partial.data(), m.pst.data(), PhaseLog{}, flexible});
+        m.tree_place = launchTreePcg<double, TV>(
+            m.ctx, amg.treePlan(),
+            {amg.krylovMatrix(), view, 0, n, b, x, m.r.data(), m.q.data(), m.ph.data(), m.pair[0].data(),
+             m.pair[1].data(), m.pair[2].data(), m.pair[3].data(), m.partial.data(), m.pst.data(), PhaseLog{}, flexible});
     };
     if (amg.fp32VCycle()) solve(amg.treeView32(), 1);
     else solve(amg.treeView64(), 0);
@@ -884,7 +887,9 @@ SolveOutcome KrylovSolver::solvePersistent(const Dcsr<double>& A, const SolverCo
             // with one smoothing step the update of x and r shares its pass with the next level-0
             // residual sweep, which then no longer reads the level-0 right-hand side and iterate
             const bool fused = amg && amg->levels() >= 2 && cfg.amg_smoothing_steps < 2;
-            const double bytes = init + applications * pre + it * (M0 + 80.0 * N) - (fused ? 16.0 * N * it : 0.0);
+            const double bytes = amg && amg->hasTree()
+                                     ? amg->treeSolveBytes(m.tree_place, 8, r.iterations, h.warm != 0, applications > 0.0)
+                                     : init + applications * pre + it * (M0 + 80.0 * N) - (fused ? 16.0 * N * it : 0.0);
             ctx.profileNote("pcg_amg_persistent", bytes, it);
             if (trace_solves())
                 std::fprintf(stderr, "bsg persistent pcg: rows %d iterations %d status %d algorithmic_bytes %.0f\n", n,

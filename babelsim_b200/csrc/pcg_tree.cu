@@ -860,7 +860,7 @@ __global__ void __launch_bounds__(TB, 1) kPcgTreeCluster(const __grid_constant__
     treeBody<TK, TV>(g, a);
 }
 template <class TK, class TV>
-void place(const TreePlan& plan, TreePcgArgs<TK, TV>& a, int ctas) {
+TreePlan::Place place(const TreePlan& plan, TreePcgArgs<TK, TV>& a, int ctas) {
     const TreePlan::Place p = plan.place(ctas);
     a.top = p.top;
     a.smem = p.smem;
@@ -868,6 +868,7 @@ void place(const TreePlan& plan, TreePcgArgs<TK, TV>& a, int ctas) {
         a.T.levels = p.levels;
         a.T.dense_inv = a.T.folded;
     }
+    return p;
 }
 
 }  // namespace
@@ -905,24 +906,25 @@ TreePlan::Place TreePlan::place(int ctas) const {
 }
 
 template <class TK, class TV>
-void launchTreePcg(Context& ctx, const TreePlan& plan, TreePcgArgs<TK, TV> a) {
+TreePlan::Place launchTreePcg(Context& ctx, const TreePlan& plan, TreePcgArgs<TK, TV> a) {
     a.log = PhaseLog{ctx.phase_entries, ctx.phase_capacity, ctx.phase_count};
     if (plan.nnz <= kClusterEntries) {
         allowSharedMemory<kPcgTreeCluster<TK, TV>>(kTreeSmem);
-        place(plan, a, clusterCtas<kPcgTreeCluster<TK, TV>>(TB, kTreeSmem));
+        const TreePlan::Place at = place(plan, a, clusterCtas<kPcgTreeCluster<TK, TV>>(TB, kTreeSmem));
         BSG_PROFILE(ctx, "pcg_amg_persistent");
         launchCluster<kPcgTreeCluster<TK, TV>>(ctx, 1, TB, a.smem, kTreeSmem, a);
-        return;
+        return at;
     }
     allowSharedMemory<kPcgTree<TK, TV>>(kTreeSmem);
     const int grid = ctx.sm_count;
-    place(plan, a, grid);
+    const TreePlan::Place at = place(plan, a, grid);
     SegmentBarrier* bar = ctx.grid_barrier;
     resetBarriers(ctx, bar, 1, grid);
     void* params[] = {&a, &bar};
     BSG_PROFILE(ctx, "pcg_amg_persistent");
     BSG_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(kPcgTree<TK, TV>), grid, TB, params, a.smem, ctx.stream));
     ctx.launched();
+    return at;
 }
 
 template <class TK, class TV>
@@ -956,9 +958,9 @@ void launchTreePcgBatch(Context& ctx, TreeBatch<TK, TV>& batch) {
     batch.bars_used = static_cast<int>(count);
 }
 
-template void launchTreePcg<double, double>(Context&, const TreePlan&, TreePcgArgs<double, double>);
-template void launchTreePcg<double, float>(Context&, const TreePlan&, TreePcgArgs<double, float>);
-template void launchTreePcg<float, float>(Context&, const TreePlan&, TreePcgArgs<float, float>);
+template TreePlan::Place launchTreePcg<double, double>(Context&, const TreePlan&, TreePcgArgs<double, double>);
+template TreePlan::Place launchTreePcg<double, float>(Context&, const TreePlan&, TreePcgArgs<double, float>);
+template TreePlan::Place launchTreePcg<float, float>(Context&, const TreePlan&, TreePcgArgs<float, float>);
 template void launchTreePcgBatch<double, double>(Context&, TreeBatch<double, double>&);
 template void launchTreePcgBatch<double, float>(Context&, TreeBatch<double, float>&);
 

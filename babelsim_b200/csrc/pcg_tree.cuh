@@ -123,9 +123,9 @@ struct TreePlan {
     Place place(int ctas) const;
 };
 
-// One system: on one thread-block cluster when it is small, else on the whole grid.
+// One system: on one thread-block cluster when it is small, else on the whole grid.  Returns its placement.
 template <class TK, class TV>
-void launchTreePcg(Context& ctx, const TreePlan& plan, TreePcgArgs<TK, TV> args);
+TreePlan::Place launchTreePcg(Context& ctx, const TreePlan& plan, TreePcgArgs<TK, TV> args);
 
 // Systems of a batch, side by side on CTA ranges of one cooperative launch (several launches when
 // they outnumber its argument block), each with barriers of its own.

@@ -158,10 +158,10 @@ def algorithmic_bytes(name, N, nnz_off, amg_rows):
 # DRAM bytes (ncu dram__bytes_read.sum + dram__bytes_write.sum) per algorithmic byte,
 # measured by one ncu capture of the kernel: kPcgTree, first pressure solve of the
 # 512000-cell Voronoi cavity of the same generator and settings (30 CG iterations),
-# 13.09 GB of DRAM traffic for 17.10 GB of algorithmic bytes (coarse levels stay in shared
-# memory).  Both grow with cells and CG iterations in proportion, so the ratio scales the
+# 13.09 GB of DRAM traffic for 16.83 GB of algorithmic bytes (L2 holds part of the vectors;
+# levels in shared memory count once per solve).  Both grow with cells and CG iterations in proportion, so the ratio scales the
 # 1M-cell launches.
-DRAM_PER_ALGORITHMIC_BYTE = {"pcg_amg_persistent": 0.765}
+DRAM_PER_ALGORITHMIC_BYTE = {"pcg_amg_persistent": 0.778}
 
 
 def load_peaks():
@@ -747,6 +747,8 @@ def main():
                     "traffic": round(ratio * ab) if ratio else None, "algorithmic_bytes_per_launch": round(ab),
                     "avg_launch_us": round(avg_s * 1e6, 2), "launches_per_step": cnt,
                     "share_of_step": round(tot / sum(v[1] for v in prof.values()), 3)}
+        if ratio:  # `frac` counts algorithmic bytes, part of which L2 serves; this is the memory's own share
+            roofline["traffic_frac"] = round(ratio * achieved / peak, 3)
         if candidates[top][3] > 0:
             roofline["units_per_launch"] = round(candidates[top][3] / cnt, 1)
     # End to end through the C ABI with host buffers: every step copies U, p, phi in from
