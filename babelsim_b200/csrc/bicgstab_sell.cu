@@ -691,7 +691,8 @@ bool bicgstabOnChip(Context& ctx, const SellMat<double>& A, long long entries) {
 
 template <int C, class T>
 void launchBicgstab(Context& ctx, const BicgArgs<C, T>& args) {
-    BSG_PROFILE(ctx, sizeof(T) == 4 ? "bicgstab3_persistent_fp32" : "bicgstab3_persistent");
+    BSG_PROFILE(ctx, C == 3 ? (sizeof(T) == 4 ? "bicgstab3_persistent_fp32" : "bicgstab3_persistent")
+                            : (sizeof(T) == 4 ? "bicgstab1_persistent_fp32" : "bicgstab1_persistent"));
     BicgArgs<C, T> a = args;
     // FP32 systems are the inner solves of a refined one, which accepts the first iterate under its target:
     // what the inner iterations round decides which one that is, to a part of the target.  They keep the
@@ -753,7 +754,6 @@ template void launchBicgstab<3, double>(Context&, const BicgArgs<3, double>&);
 template void launchBicgstab<1, double>(Context&, const BicgArgs<1, double>&);
 template void launchBicgstab<3, float>(Context&, const BicgArgs<3, float>&);
 template void launchBicgstab<1, float>(Context&, const BicgArgs<1, float>&);
-template void launchBicgstabBatch<3>(Context&, BicgBatch<3>&);
-template void launchBicgstabBatch<1>(Context&, BicgBatch<1>&);
+template void launchBicgstabBatch<3>(Context&, BicgBatch<3>&);  // (scalar systems are not batched)
 
 }  // namespace bsg

@@ -93,18 +93,16 @@ private:
     std::size_t n_ = 0;
 };
 
-// One device, one stream, a launch counter, pinned scratch for scalars read
-// back by the host, and optional per-kernel CUDA-event timing.
 // Barrier of one group of CTAs in a persistent solver launch (set by
-// resetBarriers before the launch): the arrival count, whose top bit flips once
-// per phase; the flag a wait that ran past its bound sets, with what that wait
-// saw; and where each CTA of the launch last arrived.
+// resetBarriers before the launch): the count of arrivals, which only grows; the
+// flag a wait that ran past its bound sets, with what that wait saw; and where
+// each CTA of the launch last arrived.
 struct SegmentBarrier {
     unsigned count;
     int abort;
     int who;              // 1 + grid rank of the first CTA whose wait ran out (0: none)
     unsigned where;       // that CTA's barrier number (1 = its first barrier)
-    unsigned seen;        // the count word it last read
+    unsigned seen;        // arrivals at that barrier when it last looked
     int cta0, ncta;       // the group's CTAs (grid ranks)
     int pad;
     unsigned* progress;   // per CTA of the launch (grid rank): number of its latest barrier; may be null
@@ -134,6 +132,8 @@ std::string barrierReport(const SegmentBarrier* dev);
 // The same for the first of `n` barriers of a batched launch whose wait ran out.
 std::string barrierReport(const SegmentBarrier* dev, int n);
 
+// One device, one stream, a launch counter, pinned scratch for scalars read
+// back by the host, and optional per-kernel CUDA-event timing.
 struct Context {
     int device = 0;
     cudaStream_t stream = nullptr;

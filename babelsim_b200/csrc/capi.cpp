@@ -112,7 +112,7 @@ std::string barrierReport(const SegmentBarrier* dev) {
     std::string out = " (group of CTAs " + std::to_string(b.cta0) + ".." + std::to_string(b.cta0 + b.ncta - 1);
     if (b.who > 0)
         out += "; CTA " + std::to_string(b.who - 1) + " gave up at its barrier " + std::to_string(b.where) + " with " +
-               std::to_string(b.seen & 0x7fffffffu) + " arrivals counted";
+               std::to_string(b.seen) + " arrivals counted";
     if (b.progress && b.ncta > 0) {
         std::vector<unsigned> prog(static_cast<std::size_t>(b.ncta));
         if (cudaMemcpy(prog.data(), b.progress + b.cta0, sizeof(unsigned) * prog.size(), cudaMemcpyDeviceToHost) ==

@@ -77,8 +77,6 @@ struct Reducer {
     void ensure(int blocks, int nv);
 };
 
-// Cell arrays between the caller's numbering (host) and the device's (C values per cell):
-// a plain copy, or through the mesh's locality renumbering when it has one.
 // The matrix of a linear-system seam: the caller's arrays of the last update on the device (faces'
 // upper and lower values, cells' diagonal, two buffers in turn).
 struct DeviceEquation;
@@ -91,6 +89,8 @@ struct SeamMatrix {
     bool update(DeviceMesh& m, const double* diagonal, const double* upper, const double* lower, DeviceEquation& eq);
 };
 
+// Cell arrays between the caller's numbering (host) and the device's (C values per cell):
+// a plain copy, or through the mesh's locality renumbering when it has one.
 void uploadCells(DeviceMesh& m, double* device, const double* host, int C);
 void downloadCells(DeviceMesh& m, const double* device, double* host, int C);
 

@@ -1207,9 +1207,9 @@ void KrylovSolver::solveBatch(Context& ctx, std::vector<BatchSolve>& items) {
     }
 }
 
-// Largest system the single-system momentum solve runs on the persistent BiCGStab kernel
-// (110 592-cell Voronoi cube: 8.07 against 8.77 ms per SIMPLE iteration; 1M cells, at 4
-// blocks per SM: 39.24 against 39.93 ms per SIMPLE iteration with the per-phase kernels).
+// Largest system that one solve runs on the persistent BiCGStab kernels.  About 52 iterations on hex boxes, three
+// right-hand sides, ms by launches per phase / persistent: 1M rows 13.8 / 11.0, 2.0M 21.4 / 20.2, 2.7M 27.9 / 28.4,
+// 4.1M 41.1 / 42.7 (one right-hand side: 7.1 / 4.2 to 22.0 / 19.7).
 #ifndef BSG_PERSISTENT_BICGSTAB_ROWS
 #define BSG_PERSISTENT_BICGSTAB_ROWS 2000000
 #endif
@@ -1266,11 +1266,11 @@ void KrylovSolver::persistentBicgstab(Context& ctx, std::vector<BicgItem>& items
                                   m.ph.data(), m.sh.data(), m.t.data(), m.gph.data(), m.gsh.data(), m.partial.data(),
                                   m.bst.data(), static_cast<long long>(m.sell.sval.size())});
         }
-        if (batched) {
-            launchBicgstabBatch<C>(ctx, batch);
-        } else {
-            for (const auto& a : batch.args) launchBicgstab<C, double>(ctx, a);
+        if constexpr (C == 3) {
+            if (batched) launchBicgstabBatch(ctx, batch);
         }
+        if (!batched)
+            for (const auto& a : batch.args) launchBicgstab<C, double>(ctx, a);
         for (int k : active)
             BSG_CUDA(cudaMemcpyAsync(&res[k], items[k].solver->impl_->bst.data(), sizeof(BicgState),
                                      cudaMemcpyDeviceToHost, ctx.stream));
