@@ -599,9 +599,9 @@ __device__ void treeSolve(G& g, const TreePcgArgs<TK, TV>& a) {
         }
         const auto seed = [&](int p, const TreeOwn<TV>& o, TK bi, TK ri) {
             a.r[p] = ri;
-            const TK wi = sweptResidual(o.rd, ri);
-            w0[p] = static_cast<TV>(wi);
-            a.wq0[p].x = wi;
+            const TV wi = o.rd * static_cast<TV>(ri);
+            w0[p] = wi;
+            a.wq0[p].x = static_cast<TK>(wi);
             v[0] += static_cast<double>(ri) * static_cast<double>(ri);
             v[1] += static_cast<double>(bi) * static_cast<double>(bi);
         };
@@ -735,7 +735,7 @@ __device__ void treeSolve(G& g, const TreePcgArgs<TK, TV>& a) {
         const TK ak = static_cast<TK>(alpha);
         const auto wj = [&](int j) {
             const TK2 v2 = wq[j];
-            return sweptUpdate<TV>(v2.x, ak, v2.y);
+            return static_cast<TV>(v2.x - ak * v2.y);
         };
         double nr[2] = {0.0, 0.0};
         if (tree0) {
@@ -752,13 +752,12 @@ __device__ void treeSolve(G& g, const TreePcgArgs<TK, TV>& a) {
                 },
                 [&](int p, int sub, int K, const TreeOwn<TV>& o, const Own& m, TV sum) {
                     const TV rv = static_cast<TV>(m.r);
-                    const TK wk = sweptResidual(o.rd, m.r);
-                    const TV wi = static_cast<TV>(wk);
+                    const TV wi = o.rd * rv;
                     if (sub == 0 && o.rank >= 0) {
                         x[p] = m.x;
                         r[p] = m.r;
                         w0[p] = wi;
-                        wqn[p].x = wk;
+                        wqn[p].x = static_cast<TK>(wi);
                         nr[0] += static_cast<double>(m.r) * static_cast<double>(m.r);
                         nr[1] += static_cast<double>(m.r) * static_cast<double>(m.z);
                     }

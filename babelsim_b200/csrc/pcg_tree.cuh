@@ -56,19 +56,6 @@ struct Pair<float> {
     using type = float2;
 };
 
-// A row's first Jacobi sweep w = omega / diagonal * r as its neighbours hold it between iterations, and what
-// they make of it once r has become r - alpha q (wq: omega / diagonal * q).  Both stay in the Krylov
-// vectors' type until the difference is formed: with an FP32 V-cycle, w rounded before would carry the old
-// residual's rounding into one that may be orders of magnitude smaller.
-template <class TK, class TV>
-__host__ __device__ inline TK sweptResidual(TV rd, TK r) {
-    return static_cast<TK>(rd) * r;
-}
-template <class TV, class TK>
-__host__ __device__ inline TV sweptUpdate(TK w, TK alpha, TK wq) {
-    return static_cast<TV>(w - alpha * wq);
-}
-
 template <class TV>
 struct TreeView {
     int levels = 0;                    // L
