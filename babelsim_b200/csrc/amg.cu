@@ -8,7 +8,6 @@
 #include <algorithm>
 #include <cmath>
 #include <numeric>
-#include <type_traits>
 
 namespace bsg {
 
@@ -44,7 +43,6 @@ struct AmgPreconditioner::Level {
     int *t_row = nullptr, *t_rank = nullptr, *t_pos = nullptr, *t_pcol = nullptr, *at = nullptr;  // at: row -> position
     int4* t_memb = nullptr;
     double *tb = nullptr, *tw = nullptr, *te = nullptr;
-    float *tb32 = nullptr, *tw32 = nullptr, *te32 = nullptr;
     // SELL-32 pattern from the level's CSR: row pointers on the host, both arrays on the device.
     void buildSell(const int* hptr, const int* dptr_, const int* dcol_, cudaStream_t s) {
         const std::vector<int> sptr = sellOffsets(n, hptr);
@@ -262,11 +260,10 @@ __global__ void kFoldColumns(int n, int nc, const int* __restrict__ ptr, const i
 }
 
 // Second pass: the row of rank blockIdx.x, its entries by position.
-template <class T>
 __global__ void kFoldLines(int n, int npos, const int* __restrict__ pos, const int* __restrict__ row,
                            const int* __restrict__ ptr, const int* __restrict__ col, const double* __restrict__ diag,
                            const double* __restrict__ val, const double* __restrict__ rd, const int* __restrict__ agg,
-                           double gamma, const double* __restrict__ Y, const int* __restrict__ at, T* __restrict__ out) {
+                           double gamma, const double* __restrict__ Y, const int* __restrict__ at, double* __restrict__ out) {
     extern __shared__ double line[];
     const int i = row[pos[blockIdx.x]];
     const double wi = rd[i];
@@ -288,7 +285,7 @@ __global__ void kFoldLines(int n, int npos, const int* __restrict__ pos, const i
     }
     __syncthreads();
     for (int p = threadIdx.x; p < npos; p += blockDim.x)
-        out[static_cast<long long>(blockIdx.x) * npos + p] = static_cast<T>(line[p]);
+        out[static_cast<long long>(blockIdx.x) * npos + p] = line[p];
 }
 
 __global__ void kDenseSolve(int n, const double* __restrict__ Minv, const double* __restrict__ b, double* __restrict__ x) {
@@ -535,7 +532,7 @@ void AmgPreconditioner::buildTree() {
     const std::vector<std::vector<int>>&ptr = host_ptr_, &agg = host_agg_;
     const int L = static_cast<int>(levels_.size());
     plan_ = TreePlan{};
-    tree_ = cfg_.amg_smoothing_steps <= 1 && L <= kMaxTreeLevels;
+    tree_ = cfg_.amg_smoothing_steps <= 1 && L <= kMaxTreeLevels && !fp32_;  // (why not in FP32: pcg_tree.cuh)
     if (L < 2 || levels_[0]->n < kTuneRows) tuned_ = true;
     for (int l = 0; tree_ && l + 1 < L; ++l) {
         std::vector<int> size(levels_[l + 1]->n, 0);
@@ -548,8 +545,6 @@ void AmgPreconditioner::buildTree() {
     plan_.rows.assign(L, 0);
     plan_.positions.assign(L, 0);
     plan_.nnz = levels_[0]->nnz;
-    plan_.value_bytes = fp32_ ? 4 : 8;
-    plan_.level0_bytes = cfg_.precision == 1 ? 4 : 8;
     // One host image of every level's maps, one allocation, one upload and one clearing: with an array each
     // (nine per level), a synchronisation per level and the trial to its end, a new 4096-cell system's first
     // solve took 4.5 ms, now 3.9 (16x16x16 cells; 4.9 and 4.0 for a 64x64 cavity's first outer iteration).
@@ -607,7 +602,6 @@ void AmgPreconditioner::buildTree() {
     }
     // level L - 2 and its V-cycle as one dense matrix (foldCoarse), where that level is small
     plan_.folded = L >= 3 && plan_.first <= L - 2 && levels_[L - 2]->n <= kFoldRows;
-    const std::size_t value = fp32_ ? sizeof(float) : sizeof(double);
     std::size_t bytes = sizeof(int) * image.size();
     const auto take = [&](std::size_t b) {
         const std::size_t at = bytes;
@@ -618,16 +612,16 @@ void AmgPreconditioner::buildTree() {
     const std::size_t vectors = bytes;
     std::vector<std::size_t> vec(L);
     for (int l = plan_.first; l < L; ++l) {
-        vec[l] = take(value * levels_[l]->npos);
-        take(value * levels_[l]->npos);
-        take(value * levels_[l]->npos);
+        vec[l] = take(sizeof(double) * levels_[l]->npos);
+        take(sizeof(double) * levels_[l]->npos);
+        take(sizeof(double) * levels_[l]->npos);
     }
     const std::size_t vectors_end = bytes;
     std::size_t fold_y = 0, folded = 0;
     if (plan_.folded) {
         const std::size_t n = levels_[L - 2]->n;
         fold_y = take(sizeof(double) * levels_[L - 1]->n * n);
-        folded = take(value * n * levels_[L - 2]->npos);
+        folded = take(sizeof(double) * n * levels_[L - 2]->npos);
     }
     cudaStream_t s = ctx_.stream;
     tree_store_.resize(bytes);
@@ -652,20 +646,14 @@ void AmgPreconditioner::buildTree() {
                 ctx_.launched();
             }
         }
-        const auto vectorsOf = [&](auto*& b, auto*& w, auto*& e) {
-            using T = std::remove_reference_t<decltype(*b)>;
-            const std::size_t step = (value * lv->npos + 255) / 256 * 256;
-            b = reinterpret_cast<T*>(store + vec[l]);
-            w = reinterpret_cast<T*>(store + vec[l] + step);
-            e = reinterpret_cast<T*>(store + vec[l] + 2 * step);
-        };
-        if (fp32_) vectorsOf(lv->tb32, lv->tw32, lv->te32);
-        else vectorsOf(lv->tb, lv->tw, lv->te);
+        const std::size_t step = (sizeof(double) * lv->npos + 255) / 256 * 256;
+        lv->tb = reinterpret_cast<double*>(store + vec[l]);
+        lv->tw = reinterpret_cast<double*>(store + vec[l] + step);
+        lv->te = reinterpret_cast<double*>(store + vec[l] + 2 * step);
     }
     if (plan_.folded) {
         fold_y_ = reinterpret_cast<double*>(store + fold_y);
-        if (fp32_) folded32_ = reinterpret_cast<float*>(store + folded);
-        else folded_ = reinterpret_cast<double*>(store + folded);
+        folded_ = reinterpret_cast<double*>(store + folded);
     }
     ctx_.sync();  // the host image goes
 }
@@ -682,13 +670,9 @@ void AmgPreconditioner::foldCoarse() {
     const Level *f = levels_[L - 2], *c = levels_[L - 1];
     kFoldColumns<<<f->n, kBlock, 0, ctx_.stream>>>(f->n, c->n, f->dptr, f->dcol, f->ddiag, f->dval, f->rdiag.data(),
                                                    f->agg.data(), c->dense.data(), fold_y_);
-    const auto rows = [&](auto* out) {
-        kFoldLines<<<f->n, kBlock, sizeof(double) * f->npos, ctx_.stream>>>(
-            f->n, f->npos, f->t_pos, f->t_row, f->dptr, f->dcol, f->ddiag, f->dval, f->rdiag.data(),
-            f->agg.data(), gamma_, fold_y_, f->at, out);
-    };
-    if (fp32_) rows(folded32_);
-    else rows(folded_);
+    kFoldLines<<<f->n, kBlock, sizeof(double) * f->npos, ctx_.stream>>>(
+        f->n, f->npos, f->t_pos, f->t_row, f->dptr, f->dcol, f->ddiag, f->dval, f->rdiag.data(), f->agg.data(), gamma_,
+        fold_y_, f->at, folded_);
     BSG_CUDA(cudaGetLastError());
     ctx_.launches += 2;
 }
@@ -702,14 +686,9 @@ int AmgPreconditioner::treePositions() const {
     return plan_.first == 0 ? std::max(levels_.front()->npos, levels_.front()->n) : levels_.front()->n;
 }
 
-TreeView<double> AmgPreconditioner::treeView64() const {
+TreeView AmgPreconditioner::treeView() const {
     return {static_cast<int>(levels_.size()), plan_.first, gamma_, omega_, d_tree_.data(), d_vl64_.data(),
-            d_tvec64_.data(), levels_.back()->dense.data(), folded_};
-}
-
-TreeView<float> AmgPreconditioner::treeView32() const {
-    return {static_cast<int>(levels_.size()), plan_.first, static_cast<float>(gamma_), omega_, d_tree_.data(),
-            d_vl32_.data(), d_tvec32_.data(), dense32_.data(), folded32_};
+            d_tvec_.data(), levels_.back()->dense.data(), folded_};
 }
 
 void AmgPreconditioner::update(const Dcsr<double>& A, bool numeric) {
@@ -843,22 +822,17 @@ void AmgPreconditioner::uploadTree() {
     if (!tree_) return;  // also before prepareCg
     const int L = static_cast<int>(levels_.size());
     std::vector<TreeLevel> t(L);
-    std::vector<double*> v64(3 * L, nullptr);
-    std::vector<float*> v32(3 * L, nullptr);
+    std::vector<double*> vec(3 * L, nullptr);
     for (int l = plan_.first; l < L; ++l) {
         Level* lv = levels_[l];
         t[l] = TreeLevel{lv->n, lv->npos, lv->t_row, lv->t_rank, lv->t_pos, lv->t_memb,
                          lv->dptr, lv->t_pcol, lv->dval, lv->ddiag};
-        v64[3 * l] = lv->tb;
-        v64[3 * l + 1] = lv->tw;
-        v64[3 * l + 2] = lv->te;
-        v32[3 * l] = lv->tb32;
-        v32[3 * l + 1] = lv->tw32;
-        v32[3 * l + 2] = lv->te32;
+        vec[3 * l] = lv->tb;
+        vec[3 * l + 1] = lv->tw;
+        vec[3 * l + 2] = lv->te;
     }
     d_tree_.upload(t, ctx_.stream);
-    if (fp32_) d_tvec32_.upload(v32, ctx_.stream);
-    else d_tvec64_.upload(v64, ctx_.stream);
+    d_tvec_.upload(vec, ctx_.stream);
 }
 
 SellMat<double> AmgPreconditioner::krylovMatrix() const {
@@ -917,15 +891,15 @@ double AmgPreconditioner::sellVcycleBytes() const {
     return bytes;
 }
 
-double AmgPreconditioner::treeSolveBytes(const TreePlan::Place& place, int value, int iterations, bool warm,
-                                         bool started) const {
+double AmgPreconditioner::treeSolveBytes(const TreePlan::Place& place, int iterations, bool warm, bool started) const {
     const int levels = place.levels, top = place.top;
-    const double s = fp32_ ? 4.0 : 8.0, k = value, N = levels_[0]->n, it = iterations;
+    constexpr double s = 8.0, k = 8.0;  // V-cycle and Krylov values
+    const double N = levels_[0]->n, it = iterations;
     const double applications = started ? std::max(1.0, it) : 0.0;
     const auto rows = [&](int l) { return static_cast<double>(levels_[l]->n); };
-    const auto sweep = [&](int l, double v) {  // one pass over a streamed level's matrix and diagonal
+    const auto sweep = [&](int l) {  // one pass over a streamed level's matrix and diagonal
         const Level* f = levels_[l];
-        return (4.0 + v) * static_cast<double>(f->sell_entries) + 4.0 * (f->nslices + 1) + v * f->n;
+        return 12.0 * static_cast<double>(f->sell_entries) + 4.0 * (f->nslices + 1) + 8.0 * f->n;
     };
     double once = 0.0, cycle = 0.0;
     for (int l = top; l < levels - 1; ++l) {  // CSR row, column positions, diagonals and maps, to shared memory
@@ -937,12 +911,12 @@ double AmgPreconditioner::treeSolveBytes(const TreePlan::Place& place, int value
     } else {
         for (int l = 0; l < top; ++l) {  // levels streamed in their own numbering
             const double n = rows(l), nc = rows(l + 1);
-            if (l > 0) cycle += sweep(l, s) + 3.0 * s * n;               // w (gathered), b read; t written
+            if (l > 0) cycle += sweep(l) + 3.0 * s * n;               // w (gathered), b read; t written
             cycle += s * n + (l + 1 < top ? 4.0 * (nc + 1) + 4.0 * n + 3.0 * s * nc   // lists, t, rd read; b, w written
                                           : 16.0 * plan_.positions[l + 1] + 2.0 * s * nc);
             cycle += (l + 1 < top ? 4.0 * (nc + 1) + 4.0 * n : 16.0 * plan_.positions[l + 1]) + 2.0 * s * n;  // pushes
-            cycle += l > 0 ? sweep(l, s) + 4.0 * s * n                   // y (gathered), rd, b read
-                           : sweep(0, s) + 3.0 * s * n + 2.0 * k * n;    // and r for r . z, z written
+            cycle += l > 0 ? sweep(l) + 4.0 * s * n                   // y (gathered), rd, b read
+                           : sweep(0) + 3.0 * s * n + 2.0 * k * n;    // and r for r . z, z written
         }
         for (int l = std::max(top, 1); l < levels - 1; ++l)              // b, w twice, e(coarse) read; b, w(coarse), e written
             cycle += 5.0 * s * rows(l) + 3.0 * s * rows(l + 1);
@@ -953,9 +927,9 @@ double AmgPreconditioner::treeSolveBytes(const TreePlan::Place& place, int value
     // per iteration: the product ({z, p} read; p, q and omega/d q written) and the update with the next residual
     const double iteration = top == 0 && levels > 1
                                  ? (2.0 + 3.0) * k * N + (4.0 + 2.0 + 3.0) * k * N + s * N + 2.0 * s * rows(1)
-                                 : sweep(0, k) + 4.0 * k * N + (levels > 1 ? sweep(0, s) + 6.0 * k * N + 4.0 * s * N : 6.0 * k * N);
-    const double first = (warm ? (top == 0 && levels > 1 ? 0.0 : sweep(0, k)) + 4.0 * k * N : 3.0 * k * N) +
-                         (started && levels > 1 ? (top == 0 ? k * N : sweep(0, s)) + 2.0 * s * N : 0.0);
+                                 : sweep(0) + 4.0 * k * N + (levels > 1 ? sweep(0) + 6.0 * k * N + 4.0 * s * N : 6.0 * k * N);
+    const double first = (warm ? (top == 0 && levels > 1 ? 0.0 : sweep(0)) + 4.0 * k * N : 3.0 * k * N) +
+                         (started && levels > 1 ? (top == 0 ? k * N : sweep(0)) + 2.0 * s * N : 0.0);
     return once + first + applications * cycle + it * iteration;
 }
 

@@ -46,21 +46,19 @@ public:
     VCycleView<double> sellView64() const;
     VCycleView<float> sellView32() const;
     double sellVcycleBytes() const;
-    // Algorithmic bytes of one launch of the tree solver at `place`, with Krylov values of `value` bytes: rows kept
-    // on chip are read once per launch, the folded matrix stands for the levels it replaces, every other array
+    // Algorithmic bytes of one launch of the tree solver at `place`: rows kept on chip are read once per launch, the folded matrix stands for the levels it replaces, every other array
     // counts in each phase that reads or writes it.  `started`: the launch got past its first residual.
-    double treeSolveBytes(const TreePlan::Place& place, int value, int iterations, bool warm, bool started) const;
+    double treeSolveBytes(const TreePlan::Place& place, int iterations, bool warm, bool started) const;
     long long krylovEntries() const;  // padded level-0 SELL entries
 
     // What only the persistent CG solvers read, built before their first solve: the tree numbering of the
-    // coarse levels (pcg_tree.cuh; for one smoothing step and aggregates of at most four rows) and the folded
+    // coarse levels (pcg_tree.cuh; for FP64, one smoothing step and aggregates of at most four rows) and the folded
     // coarse matrix.  GMRES, which applies the V-cycle level by level, never asks for it.
     void prepareCg();
     bool hasTree() const { return tree_; }
     const TreePlan& treePlan() const { return plan_; }
     int treePositions() const;  // entries the Krylov vectors need (rows of level 0, or its positions)
-    TreeView<double> treeView64() const;
-    TreeView<float> treeView32() const;
+    TreeView treeView() const;
 
     // The coarse-correction scale of a hierarchy is chosen once, with its first matrix
     // (KrylovSolver's tuneCorrection); fixed by a tuning override, and on systems so small that
@@ -96,11 +94,9 @@ private:
     TreePlan plan_;
     DeviceArray<char> tree_store_;         // everything buildTree makes
     double *fold_y_ = nullptr, *folded_ = nullptr;  // foldCoarse
-    float* folded32_ = nullptr;
     DeviceArray<double> inv_panel_;        // kDenseInverseBlocked's panel, two halves
     DeviceArray<TreeLevel> d_tree_;
-    DeviceArray<double*> d_tvec64_;
-    DeviceArray<float*> d_tvec32_;
+    DeviceArray<double*> d_tvec_;
     // Damped-Jacobi weight and coarse-correction scale (the start value; see wantsTuning).  Piecewise-constant
     // aggregation under-corrects smooth error; scaling the coarse correction by
     // 1.8 (kept fixed, so the V-cycle stays a symmetric operator for CG) cut the

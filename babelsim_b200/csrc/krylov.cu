@@ -533,9 +533,8 @@ struct KrylovSolver::Impl {
     DeviceArray<BicgState> bst;    // state of the persistent BiCGStab
     DeviceArray<unsigned> ticket;  // arrivals of the current reduction (reduceThenFinish), zero between launches
     DeviceArray<PcgState> pst;
-    DeviceArray<float> r32, s32, z32, p32a, p32b, q32, d32, x32;  // FP32 inner solve of the refined path
+    DeviceArray<float> r32, s32, z32, p32a, p32b, q32, d32;  // FP32 inner solve of the refined path
     DeviceArray<double2> pair[4];  // the tree solver's paired vectors (pcg_tree.cuh)
-    DeviceArray<float2> pair32[4];
     TreePlan::Place tree_place{};  // of the last launch, for its declared bytes
     // FP32 inner BiCGStab of the refined path: matrix copy (SELL values, diagonal) and
     // the C-interleaved right-hand side, correction and Krylov vectors
@@ -680,17 +679,8 @@ SolveOutcome KrylovSolver::solveRefined(const Dcsr<double>& A, const SolverConfi
     Context& ctx = m.ctx;
     const int n = A.n;
     m.ensure(n);
-    const std::size_t entries = amg->hasTree() ? amg->treePositions() : n;
-    for (DeviceArray<float>* a : {&m.r32, &m.s32, &m.q32, &m.d32})
-        if (a->size() < entries) a->resize(entries);
-    if (amg->hasTree()) {
-        if (m.x32.size() < entries) m.x32.resize(entries);
-        for (int k = 0; k < (amg->treePlan().first == 0 ? 4 : 2); ++k)
-            if (m.pair32[k].size() < entries) m.pair32[k].resize(entries);
-    } else {
-        for (DeviceArray<float>* a : {&m.z32, &m.p32a, &m.p32b})
-            if (a->size() < entries) a->resize(entries);
-    }
+    for (DeviceArray<float>* a : {&m.r32, &m.s32, &m.z32, &m.p32a, &m.p32b, &m.q32, &m.d32})
+        if (a->size() < static_cast<std::size_t>(n)) a->resize(n);
     if (m.pst.size() < 1) m.pst.resize(1);
     SolveOutcome out;
     if (!cfg.warm_start) BSG_CUDA(cudaMemsetAsync(x, 0, sizeof(double) * n, ctx.stream));
@@ -714,18 +704,10 @@ SolveOutcome KrylovSolver::solveRefined(const Dcsr<double>& A, const SolverConfi
         h.atol = cfg.atol;
         h.rtol = cfg.rtol;
         BSG_CUDA(cudaMemcpyAsync(m.pst.data(), &h, sizeof(h), cudaMemcpyHostToDevice, ctx.stream));
-        if (amg->hasTree()) {
-            m.tree_place = launchTreePcg<float, float>(ctx, amg->treePlan(),
-                                        {amg->krylovMatrix32(), amg->treeView32(), 0, n, m.r32.data(), m.d32.data(),
-                                         m.s32.data(), m.q32.data(), m.x32.data(), m.pair32[0].data(),
-                                         m.pair32[1].data(), m.pair32[2].data(), m.pair32[3].data(), m.partial.data(),
-                                         m.pst.data(), PhaseLog{}});
-        } else {
-            SellPcgArgs<float, float> args{amg->krylovMatrix32(), amg->sellView32(), m.r32.data(), m.d32.data(),
-                                           m.s32.data(), m.z32.data(), m.p32a.data(), m.p32b.data(), m.q32.data(),
-                                           m.partial.data(), m.pst.data(), PhaseLog{}};
-            launchSellPcg(ctx, args);
-        }
+        SellPcgArgs<float, float> args{amg->krylovMatrix32(), amg->sellView32(), m.r32.data(), m.d32.data(),
+                                       m.s32.data(), m.z32.data(), m.p32a.data(), m.p32b.data(), m.q32.data(),
+                                       m.partial.data(), m.pst.data(), PhaseLog{}};
+        launchSellPcg(ctx, args);
         BSG_CUDA(cudaMemcpyAsync(ctx.pinned, m.pst.data(), sizeof(PcgState), cudaMemcpyDeviceToHost, ctx.stream));
         kAddCorrection<<<g, 256, 0, ctx.stream>>>(n, x, m.d32.data());
         ctx.launched();
@@ -740,10 +722,8 @@ SolveOutcome KrylovSolver::solveRefined(const Dcsr<double>& A, const SolverConfi
         if (ctx.profiling || trace_solves()) {
             const double N = n;
             const double M0 = 8.0 * N + 4.0 * (amg->krylovMatrix32().nslices + 1) + 8.0 * static_cast<double>(amg->krylovEntries());
-            const double bytes =
-                amg->hasTree() ? amg->treeSolveBytes(m.tree_place, 4, r.iterations, false, r.iterations > 0 || r.status != 0)
-                               : 12.0 * N + (r.iterations > 0 ? r.iterations : 1) * (amg->sellVcycleBytes() + 8.0 * N) +
-                                     r.iterations * (M0 + 40.0 * N);
+            const double bytes = 12.0 * N + (r.iterations > 0 ? r.iterations : 1) * (amg->sellVcycleBytes() + 8.0 * N) +
+                                 r.iterations * (M0 + 40.0 * N);
             ctx.profileNote("pcg_amg_persistent", bytes, r.iterations);
             if (trace_solves())
                 std::fprintf(stderr, "bsg refined pcg (fp32 inner): rows %d iterations %d residual %.3e -> %.3e\n", n,
@@ -809,19 +789,13 @@ void KrylovSolver::tuneCorrection(const Dcsr<double>& A, AmgPreconditioner& amg)
     if (chosen != amg.correction()) amg.setCorrection(chosen);
 }
 
-// The tree solver on this solver's workspace (FP64 Krylov vectors and products; an FP32 V-cycle takes
-// the flexible beta).
+// The tree solver on this solver's workspace.
 void KrylovSolver::launchTree(AmgPreconditioner& amg, int n, const double* b, double* x) {
     Impl& m = *impl_;
-    const auto solve = [&](auto view, int flexible) {
-        using TV = std::decay_t<decltype(view.gamma)>;
-        m.tree_place = launchTreePcg<double, TV>(
-            m.ctx, amg.treePlan(),
-            {amg.krylovMatrix(), view, 0, n, b, x, m.r.data(), m.q.data(), m.ph.data(), m.pair[0].data(),
-             m.pair[1].data(), m.pair[2].data(), m.pair[3].data(), m.partial.data(), m.pst.data(), PhaseLog{}, flexible});
-    };
-    if (amg.fp32VCycle()) solve(amg.treeView32(), 1);
-    else solve(amg.treeView64(), 0);
+    m.tree_place = launchTreePcg(m.ctx, amg.treePlan(),
+                                 {amg.krylovMatrix(), amg.treeView(), 0, n, b, x, m.r.data(), m.q.data(), m.ph.data(),
+                                  m.pair[0].data(), m.pair[1].data(), m.pair[2].data(), m.pair[3].data(),
+                                  m.partial.data(), m.pst.data(), PhaseLog{}});
 }
 
 SolveOutcome KrylovSolver::solvePersistent(const Dcsr<double>& A, const SolverConfig& cfg, AmgPreconditioner* amg,
@@ -888,7 +862,7 @@ SolveOutcome KrylovSolver::solvePersistent(const Dcsr<double>& A, const SolverCo
             // residual sweep, which then no longer reads the level-0 right-hand side and iterate
             const bool fused = amg && amg->levels() >= 2 && cfg.amg_smoothing_steps < 2;
             const double bytes = amg && amg->hasTree()
-                                     ? amg->treeSolveBytes(m.tree_place, 8, r.iterations, h.warm != 0, applications > 0.0)
+                                     ? amg->treeSolveBytes(m.tree_place, r.iterations, h.warm != 0, applications > 0.0)
                                      : init + applications * pre + it * (M0 + 80.0 * N) - (fused ? 16.0 * N * it : 0.0);
             ctx.profileNote("pcg_amg_persistent", bytes, it);
             if (trace_solves())
@@ -1096,8 +1070,7 @@ void KrylovSolver::solveBatch(Context& ctx, std::vector<BatchSolve>& items) {
     if (norms.size() < static_cast<std::size_t>(K)) norms.resize(K);
     std::vector<PcgState> states(K);
     std::vector<double> nrm(K);
-    TreeBatch<double, double> tree64;
-    TreeBatch<double, float> tree32;
+    TreeBatch tree;
     BatchLaunch<double, double> batch64;
     BatchLaunch<double, float> batch32;
     for (int attempt = 0; attempt < 3; ++attempt) {
@@ -1110,19 +1083,20 @@ void KrylovSolver::solveBatch(Context& ctx, std::vector<BatchSolve>& items) {
         for (int k : active)
             BSG_CUDA(cudaMemcpyAsync(items[k].solver->impl_->pst.data(), &t[k].h, sizeof(PcgState),
                                      cudaMemcpyHostToDevice, ctx.stream));
-        tree64.args.clear();
-        tree32.args.clear();
+        tree.args.clear();
+        tree.plans.clear();
+        tree.slices.clear();
         batch64.args.clear();
         batch32.args.clear();
         std::vector<long long> slices64, slices32;
-        const auto addTree = [&](auto& batch, auto view, int k, int flexible) {
+        const auto addTree = [&](int k) {
             BatchSolve& it = items[k];
             Impl& m = *it.solver->impl_;
-            batch.args.push_back({it.amg->krylovMatrix(), view, 0, it.A.n, it.b, it.x, m.r.data(), m.q.data(),
-                                  m.ph.data(), m.pair[0].data(), m.pair[1].data(), m.pair[2].data(), m.pair[3].data(),
-                                  m.partial.data(), m.pst.data(), PhaseLog{}, flexible});
-            batch.plans.push_back(&it.amg->treePlan());
-            batch.slices.push_back(it.amg->krylovMatrix().nslices);
+            tree.args.push_back({it.amg->krylovMatrix(), it.amg->treeView(), 0, it.A.n, it.b, it.x, m.r.data(),
+                                 m.q.data(), m.ph.data(), m.pair[0].data(), m.pair[1].data(), m.pair[2].data(),
+                                 m.pair[3].data(), m.partial.data(), m.pst.data(), PhaseLog{}});
+            tree.plans.push_back(&it.amg->treePlan());
+            tree.slices.push_back(it.amg->krylovMatrix().nslices);
         };
         const auto addSell = [&](auto& batch, auto view, int k, int flexible) {
             BatchSolve& it = items[k];
@@ -1131,15 +1105,10 @@ void KrylovSolver::solveBatch(Context& ctx, std::vector<BatchSolve>& items) {
                                   m.v.data(), m.q.data(), m.partial.data(), m.pst.data(), PhaseLog{}, flexible,
                                   m.t.data()});
         };
-        tree64.plans.clear();
-        tree32.plans.clear();
-        tree64.slices.clear();
-        tree32.slices.clear();
         for (int k : active) {
             AmgPreconditioner& amg = *items[k].amg;
             if (amg.hasTree()) {
-                if (amg.fp32VCycle()) addTree(tree32, amg.treeView32(), k, 1);
-                else addTree(tree64, amg.treeView64(), k, 0);
+                addTree(k);
             } else if (amg.fp32VCycle()) {
                 addSell(batch32, amg.sellView32(), k, 1);
                 slices32.push_back(amg.krylovMatrix().nslices);
@@ -1148,8 +1117,7 @@ void KrylovSolver::solveBatch(Context& ctx, std::vector<BatchSolve>& items) {
                 slices64.push_back(amg.krylovMatrix().nslices);
             }
         }
-        if (!tree64.args.empty()) launchTreePcgBatch(ctx, tree64);
-        if (!tree32.args.empty()) launchTreePcgBatch(ctx, tree32);
+        launchTreePcgBatch(ctx, tree);
         launchSellPcgBatch(ctx, batch64, slices64);
         launchSellPcgBatch(ctx, batch32, slices32);
         // solve states and true residuals of every system of this attempt, read back together
@@ -1171,8 +1139,7 @@ void KrylovSolver::solveBatch(Context& ctx, std::vector<BatchSolve>& items) {
             const PcgState& r = states[k];
             if (r.status == 3)
                 fail(kCuda, "batched persistent PCG: a segment barrier wait ran past its bound" +
-                                barrierReport(tree64.d_bars.data(), tree64.bars_used) +
-                                barrierReport(tree32.d_bars.data(), tree32.bars_used) +
+                                barrierReport(tree.d_bars.data(), tree.bars_used) +
                                 barrierReport(batch64.d_bars.data(), static_cast<int>(batch64.d_bars.size())) +
                                 barrierReport(batch32.d_bars.data(), static_cast<int>(batch32.d_bars.size())));
             ++it.out.checks;

@@ -36,10 +36,9 @@ __device__ __forceinline__ void mark(const PhaseLog& log, int id) {
 }
 
 // What a row's update needs besides its matrix entries.
-template <class TV>
 struct alignas(8) TreeOwn {
     double d;     // diagonal
-    TV rd, qrd;   // omega / diagonal of the row, and of the next level's row it belongs to
+    double rd, qrd;   // omega / diagonal of the row, and of the next level's row it belongs to
     int rank;     // -1: a hole
     int qpos;     // position of the next level's row (-1 past the last aggregate)
 };
@@ -56,16 +55,14 @@ struct LevelSlot {
     int u0, nu, k, dir;  // this CTA's units [u0, u0 + nu), 2^k lanes per row, first directory entry
 };
 
-template <class TV>
 struct TreeShared {
     TreeLevel lv[kMaxTreeLevels];
     LevelSlot slot[kMaxTreeLevels];
-    TV* vec[3 * kMaxTreeLevels];
+    double* vec[3 * kMaxTreeLevels];
     int used;
 };
-template <class TV>
-__device__ __forceinline__ TreeShared<TV>& treeShared() {
-    __shared__ TreeShared<TV> s;
+__device__ __forceinline__ TreeShared& treeShared() {
+    __shared__ TreeShared s;
     return s;
 }
 __device__ __forceinline__ char* treeRows() {
@@ -74,32 +71,30 @@ __device__ __forceinline__ char* treeRows() {
 }
 
 // A unit's block: values (T, 32 per step), TreeOwn per row, columns (int, 32 per step).
-template <class T, class TV>
 __device__ __forceinline__ int unitBytes(int steps, int k) {
-    return steps * 32 * static_cast<int>(sizeof(T)) + (32 >> k) * static_cast<int>(sizeof(TreeOwn<TV>)) + steps * 128;
+    return steps * 32 * static_cast<int>(sizeof(double)) + (32 >> k) * static_cast<int>(sizeof(TreeOwn)) + steps * 128;
 }
 
-template <class TV>
-__device__ __forceinline__ TreeOwn<TV> ownOf(const TreeLevel& t, const TreeLevel* next, double omega, int p) {
-    TreeOwn<TV> o;
+__device__ __forceinline__ TreeOwn ownOf(const TreeLevel& t, const TreeLevel* next, double omega, int p) {
+    TreeOwn o;
     const int i = p < t.npos ? t.row[p] : -1;
     o.rank = i >= 0 ? t.rank[p] : -1;
     o.d = i >= 0 ? t.diag[i] : 1.0;
-    o.rd = i >= 0 ? static_cast<TV>(omega / o.d) : TV(0);
+    o.rd = i >= 0 ? omega / o.d : 0.0;
     o.qpos = -1;
-    o.qrd = TV(0);
+    o.qrd = 0.0;
     if (next && (p >> 2) < next->n) {
         o.qpos = next->pos[p >> 2];
-        o.qrd = static_cast<TV>(omega / next->diag[next->row[o.qpos]]);
+        o.qrd = omega / next->diag[next->row[o.qpos]];
     }
     return o;
 }
 
 // Copies this CTA's rows of the tree levels into shared memory, coarsest first, until it is
 // full; the directory (offset, steps per unit; offset -1: not copied) lies at its start.
-template <class TK, class TV, class G>
-__device__ void openTree(const G& g, const TreePcgArgs<TK, TV>& a) {
-    TreeShared<TV>& s = treeShared<TV>();
+template <class G>
+__device__ void openTree(const G& g, const TreePcgArgs& a) {
+    TreeShared& s = treeShared();
     const int L = a.T.levels, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int l = max(a.top, a.T.first) + threadIdx.x; l < L; l += TB) s.lv[l] = a.T.lv[l];
     for (int k = threadIdx.x; k < 3 * L; k += TB) s.vec[k] = a.T.vec[k];
@@ -149,7 +144,7 @@ __device__ void openTree(const G& g, const TreePcgArgs<TK, TV>& a) {
                 int bytes = 0;
                 if (u < t.nu) {
                     const int steps = dir[t.dir + u].y;
-                    bytes = l == 0 ? unitBytes<TK, TV>(steps, t.k) : unitBytes<TV, TV>(steps, t.k);
+                    bytes = unitBytes(steps, t.k);
                 }
                 int sum = bytes;
                 for (int o = 1; o < 32; o <<= 1) {
@@ -170,11 +165,11 @@ __device__ void openTree(const G& g, const TreePcgArgs<TK, TV>& a) {
             const int2 e = dir[t.dir + u];
             if (e.x < 0) continue;
             char* block = treeRows() + e.x;
-            const int vb = e.y * 32 * static_cast<int>(l == 0 ? sizeof(TK) : sizeof(TV));
-            TreeOwn<TV>* own = reinterpret_cast<TreeOwn<TV>*>(block + vb);
+            const int vb = e.y * 32 * static_cast<int>(sizeof(double));
+            TreeOwn* own = reinterpret_cast<TreeOwn*>(block + vb);
             int* col = reinterpret_cast<int*>(own + (32 >> t.k));
             const int rows = 32 >> t.k, p0 = (t.u0 + u) * rows;
-            if (lane < rows) own[lane] = ownOf<TV>(v, next, a.T.omega, p0 + lane);
+            if (lane < rows) own[lane] = ownOf(v, next, a.T.omega, p0 + lane);
             const int p = p0 + (lane >> t.k), q = lane & ((1 << t.k) - 1);
             const int i = p < v.npos ? v.row[p] : -1;
             const int k0 = i >= 0 ? v.ptr[i] : 0, len = i >= 0 ? v.ptr[i + 1] - k0 : 0;
@@ -182,9 +177,7 @@ __device__ void openTree(const G& g, const TreePcgArgs<TK, TV>& a) {
                 const int k = q + (step << t.k);
                 const bool on = k < len;
                 col[32 * step + lane] = on ? v.pcol[k0 + k] : min(p, v.npos - 1);  // padding: its own value, times zero
-                const double x = on ? v.val[k0 + k] : 0.0;
-                if (l == 0) reinterpret_cast<TK*>(block)[32 * step + lane] = static_cast<TK>(x);
-                else reinterpret_cast<TV*>(block)[32 * step + lane] = static_cast<TV>(x);
+                reinterpret_cast<double*>(block)[32 * step + lane] = on ? v.val[k0 + k] : 0.0;
             }
         }
     }
@@ -193,11 +186,10 @@ __device__ void openTree(const G& g, const TreePcgArgs<TK, TV>& a) {
 
 // f(p, q, own, sum) for every unit of tree level l, with sum = sum_k a_pk y(col) (all K lanes of
 // a row hold it); pre(p, own) runs before the gathers and its result is passed on, so the
-// row's own vector entries travel together with them.  TM: the type the entries are stored
-// and multiplied in is TM, results are TR.
-template <class TM, class TR, class TV, class Y, class P, class F>
+// row's own vector entries travel together with them.
+template <class Y, class P, class F>
 __device__ __forceinline__ void sweepTree(int l, bool stored, double omega, Y y, P pre, F f) {
-    const TreeShared<TV>& s = treeShared<TV>();
+    const TreeShared& s = treeShared();
     const LevelSlot t = s.slot[l];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int K = 1 << t.k, rows = 32 >> t.k, sub = lane >> t.k, q = lane & (K - 1);
@@ -207,41 +199,41 @@ __device__ __forceinline__ void sweepTree(int l, bool stored, double omega, Y y,
         const int2 e = stored ? dir[u] : make_int2(-1, 0);
         if (e.x >= 0) {
             const char* block = treeRows() + e.x;
-            const TM* v = reinterpret_cast<const TM*>(block) + lane;
-            const TreeOwn<TV>& o = *(reinterpret_cast<const TreeOwn<TV>*>(block + e.y * 32 * sizeof(TM)) + sub);
-            const int* c = reinterpret_cast<const int*>(reinterpret_cast<const TreeOwn<TV>*>(block + e.y * 32 * sizeof(TM)) + rows) + lane;
+            const double* v = reinterpret_cast<const double*>(block) + lane;
+            const TreeOwn& o = *(reinterpret_cast<const TreeOwn*>(block + e.y * 32 * sizeof(double)) + sub);
+            const int* c = reinterpret_cast<const int*>(reinterpret_cast<const TreeOwn*>(block + e.y * 32 * sizeof(double)) + rows) + lane;
             const auto mine = pre(p, o);
-            TR a0 = TR(0), a1 = TR(0);
+            double a0 = 0.0, a1 = 0.0;
             int k = 0;
             for (; k + 8 <= e.y; k += 8) {
-                TR yy[8];
+                double yy[8];
 #pragma unroll
                 for (int i = 0; i < 8; ++i) yy[i] = y(c[32 * (k + i)]);
 #pragma unroll
                 for (int i = 0; i < 8; i += 2) {
-                    a0 += static_cast<TR>(v[32 * (k + i)]) * yy[i];
-                    a1 += static_cast<TR>(v[32 * (k + i + 1)]) * yy[i + 1];
+                    a0 += v[32 * (k + i)] * yy[i];
+                    a1 += v[32 * (k + i + 1)] * yy[i + 1];
                 }
             }
             for (; k < e.y; k += 4) {  // the last one to seven steps, still gathered four at a time
-                TR yy[4];
+                double yy[4];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) yy[i] = k + i < e.y ? y(c[32 * (k + i)]) : TR(0);
+                for (int i = 0; i < 4; ++i) yy[i] = k + i < e.y ? y(c[32 * (k + i)]) : 0.0;
 #pragma unroll
                 for (int i = 0; i < 4; ++i)
-                    if (k + i < e.y) a0 += static_cast<TR>(v[32 * (k + i)]) * yy[i];
+                    if (k + i < e.y) a0 += v[32 * (k + i)] * yy[i];
             }
-            TR sum = a0 + a1;
+            double sum = a0 + a1;
             for (int o2 = K >> 1; o2 > 0; o2 >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o2);
             f(p, q, K, o, mine, sum);
         } else {  // rows that did not fit
             const TreeLevel& v = s.lv[l];
-            const TreeOwn<TV> o = ownOf<TV>(v, &s.lv[l + 1], omega, p);
+            const TreeOwn o = ownOf(v, &s.lv[l + 1], omega, p);
             const auto mine = pre(p, o);
-            TR sum = TR(0);
+            double sum = 0.0;
             if (o.rank >= 0)
                 for (int i = v.row[p], k = v.ptr[i] + q; k < v.ptr[i + 1]; k += K)
-                    sum += static_cast<TR>(static_cast<TM>(v.val[k])) * y(v.pcol[k]);
+                    sum += v.val[k] * y(v.pcol[k]);
             for (int o2 = K >> 1; o2 > 0; o2 >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o2);
             f(p, q, K, o, mine, sum);
         }
@@ -249,17 +241,16 @@ __device__ __forceinline__ void sweepTree(int l, bool stored, double omega, Y y,
 }
 
 // Sum over the four rows of an aggregate (K lanes each hold their row's value).
-template <class T>
-__device__ __forceinline__ T quadSum(T t, int K) {
+__device__ __forceinline__ double quadSum(double t, int K) {
     t += __shfl_xor_sync(0xffffffffu, t, K);
     t += __shfl_xor_sync(0xffffffffu, t, 2 * K);
     return t;
 }
 
 // f(p, own) for every position of tree level l that holds a row, one lane each.
-template <class TM, class TV, class F>
+template <class F>
 __device__ __forceinline__ void treeRowsOf(int l, bool stored, double omega, F f) {
-    const TreeShared<TV>& s = treeShared<TV>();
+    const TreeShared& s = treeShared();
     const LevelSlot t = s.slot[l];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, rows = 32 >> t.k;
     const int2* dir = reinterpret_cast<const int2*>(treeRows()) + t.dir;
@@ -268,28 +259,27 @@ __device__ __forceinline__ void treeRowsOf(int l, bool stored, double omega, F f
         const int p = (t.u0 + u) * rows + lane;
         const int2 e = stored ? dir[u] : make_int2(-1, 0);
         if (e.x >= 0) {
-            const TreeOwn<TV>& o = reinterpret_cast<const TreeOwn<TV>*>(treeRows() + e.x + e.y * 32 * sizeof(TM))[lane];
+            const TreeOwn& o = reinterpret_cast<const TreeOwn*>(treeRows() + e.x + e.y * 32 * sizeof(double))[lane];
             if (o.rank >= 0) f(p, o);
         } else {
-            const TreeOwn<TV> o = ownOf<TV>(s.lv[l], &s.lv[l + 1], omega, p);
+            const TreeOwn o = ownOf(s.lv[l], &s.lv[l + 1], omega, p);
             if (o.rank >= 0) f(p, o);
         }
     }
 }
 
-template <class T>
-__device__ __forceinline__ T memberSum(const T* t, int4 m) {
-    const T t0 = m.x >= 0 ? t[m.x] : T(0), t1 = m.y >= 0 ? t[m.y] : T(0);
-    const T t2 = m.z >= 0 ? t[m.z] : T(0), t3 = m.w >= 0 ? t[m.w] : T(0);
+__device__ __forceinline__ double memberSum(const double* t, int4 m) {
+    const double t0 = m.x >= 0 ? t[m.x] : 0.0, t1 = m.y >= 0 ? t[m.y] : 0.0;
+    const double t2 = m.z >= 0 ? t[m.z] : 0.0, t3 = m.w >= 0 ? t[m.w] : 0.0;
     return ((t0 + t1) + t2) + t3;
 }
 
 // Coarsest level: e_I = sum_J inv_IJ b_J, I < n, J < cols.  A CTA's rows are split over its warps, so
 // that each lane has a few loads in flight instead of a long chain.  emit(I, value) runs on one
 // thread per row.
-template <class TV, class G, class B, class F>
-__device__ __forceinline__ void denseRows(const G& g, int n, int cols, const TV* __restrict__ inv, B b, F emit) {
-    __shared__ TV part[TB / 32];
+template <class G, class B, class F>
+__device__ __forceinline__ void denseRows(const G& g, int n, int cols, const double* __restrict__ inv, B b, F emit) {
+    __shared__ double part[TB / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int size = g.size(), r0 = static_cast<int>(static_cast<long long>(n) * g.rank() / size);
     const int mine = static_cast<int>(static_cast<long long>(n) * (g.rank() + 1) / size) - r0;
@@ -298,16 +288,16 @@ __device__ __forceinline__ void denseRows(const G& g, int n, int cols, const TV*
     const int per = (TB / 32) >> lw, step = 32 << lw;
     for (int first = 0; first < mine; first += per) {
         const int r = first + (warp >> lw);
-        TV s = TV(0);
+        double s = 0.0;
         if (r < mine) {
-            const TV* row = inv + static_cast<long long>(r0 + r) * cols;
+            const double* row = inv + static_cast<long long>(r0 + r) * cols;
             for (int J = ((warp & ((1 << lw) - 1)) << 5) + lane; J < cols; J += 8 * step) {
-                TV x[8], y[8];
+                double x[8], y[8];
 #pragma unroll
                 for (int k = 0; k < 8; ++k) {
                     const bool on = J + k * step < cols;
-                    x[k] = on ? __ldg(row + J + k * step) : TV(0);
-                    y[k] = on ? b(J + k * step) : TV(0);
+                    x[k] = on ? __ldg(row + J + k * step) : 0.0;
+                    y[k] = on ? b(J + k * step) : 0.0;
                 }
 #pragma unroll
                 for (int k = 0; k < 8; ++k) s += x[k] * y[k];
@@ -318,7 +308,7 @@ __device__ __forceinline__ void denseRows(const G& g, int n, int cols, const TV*
         if (lane == 0) part[warp] = s;
         __syncthreads();
         if (threadIdx.x < per && first + static_cast<int>(threadIdx.x) < mine) {
-            TV v = TV(0);
+            double v = 0.0;
             for (int k = 0; k < (1 << lw); ++k) v += part[(threadIdx.x << lw) + k];
             emit(r0 + first + static_cast<int>(threadIdx.x), v);
         }
@@ -329,44 +319,44 @@ __device__ __forceinline__ void denseRows(const G& g, int n, int cols, const TV*
 // The V-cycle below the finest level: on entry the residual of level 0 has been restricted
 // (top = 0: level 1's b and w are set) or is in nat[0].t (top > 0); on return level 1's result is in
 // its e (top = 0) or has been pushed into nat[0].x.
-template <class TK, class TV, bool TREE0, class G>
-__device__ __forceinline__ void treeCoarse(G& g, const TreePcgArgs<TK, TV>& a, bool stored) {
-    TreeShared<TV>& s = treeShared<TV>();
+template <bool TREE0, class G>
+__device__ __forceinline__ void treeCoarse(G& g, const TreePcgArgs& a, bool stored) {
+    TreeShared& s = treeShared();
     const int L = a.T.levels, top = TREE0 ? 0 : a.top;
     const Lanes c = lanes<TB>(g);
-    const TV gamma = a.T.gamma;
+    const double gamma = a.T.gamma;
     const double omega = a.T.omega;
     // ---- down, levels in their own numbering
     for (int l = 0; l < top; ++l) {
-        const VLevel<TV> f = a.T.nat[l];
+        const VLevel<double> f = a.T.nat[l];
         if (l > 0) {
-            const TV* w = f.w;
+            const double* w = f.w;
             for (int sl = c.gwarp; sl < f.A.nslices; sl += c.nwarps) {
                 const int i = 32 * sl + c.lane;
-                const TV ax = sellRow(f.A, sl, c.lane, [&](int j) { return w[j]; });
+                const double ax = sellRow(f.A, sl, c.lane, [&](int j) { return w[j]; });
                 if (i < f.A.n) f.t[i] = f.b[i] - (f.A.diag[i] * w[i] + ax);
             }
             g.sync();
             mark(a.log, 30 + l);
         }
-        const TV* t = f.t;
+        const double* t = f.t;
         if (l + 1 < top) {
-            const VLevel<TV> cl = a.T.nat[l + 1];
+            const VLevel<double> cl = a.T.nat[l + 1];
             for (int I = c.gthread; I < cl.A.n; I += c.nthreads) {
-                TV x = TV(0);
+                double x = 0.0;
                 for (int m = f.agg_ptr[I]; m < f.agg_ptr[I + 1]; ++m) x += t[f.agg_rows[m]];
                 cl.b[I] = x;
                 cl.w[I] = cl.rd[I] * x;
             }
         } else if (top == L - 1) {
-            TV* b = s.vec[3 * top];
+            double* b = s.vec[3 * top];
             const TreeLevel& v = s.lv[top];
             for (int p = c.gthread; p < v.npos; p += c.nthreads) b[p] = memberSum(t, v.memb[p]);  // zero in holes
         } else {
-            TV *b = s.vec[3 * top], *w = s.vec[3 * top + 1];
+            double *b = s.vec[3 * top], *w = s.vec[3 * top + 1];
             const int4* memb = s.lv[top].memb;
-            treeRowsOf<TV, TV>(top, stored, omega, [&](int p, const TreeOwn<TV>& o) {
-                const TV x = memberSum(t, memb[p]);
+            treeRowsOf(top, stored, omega, [&](int p, const TreeOwn& o) {
+                const double x = memberSum(t, memb[p]);
                 b[p] = x;
                 w[p] = o.rd * x;
             });
@@ -376,16 +366,16 @@ __device__ __forceinline__ void treeCoarse(G& g, const TreePcgArgs<TK, TV>& a, b
     }
     // ---- down, tree levels: residual and restriction in one phase
     for (int l = max(top, 1); l < L - 1; ++l) {
-        const TV *b = s.vec[3 * l], *w = s.vec[3 * l + 1];
-        TV *cb = s.vec[3 * l + 3], *cw = s.vec[3 * l + 4];
+        const double *b = s.vec[3 * l], *w = s.vec[3 * l + 1];
+        double *cb = s.vec[3 * l + 3], *cw = s.vec[3 * l + 4];
         struct Own {
-            TV b, w;
+            double b, w;
         };
-        sweepTree<TV, TV, TV>(
+        sweepTree(
             l, stored, omega, [&](int j) { return w[j]; },
-            [&](int p, const TreeOwn<TV>& o) { return o.rank >= 0 ? Own{b[p], w[p]} : Own{TV(0), TV(0)}; },
-            [&](int p, int q, int K, const TreeOwn<TV>& o, const Own& m, TV sum) {
-                const TV x = quadSum(o.rank >= 0 ? m.b - (static_cast<TV>(o.d) * m.w + sum) : TV(0), K);
+            [&](int p, const TreeOwn& o) { return o.rank >= 0 ? Own{b[p], w[p]} : Own{0.0, 0.0}; },
+            [&](int p, int q, int K, const TreeOwn& o, const Own& m, double sum) {
+                const double x = quadSum(o.rank >= 0 ? m.b - (o.d * m.w + sum) : 0.0, K);
                 if (q == 0 && (p & 3) == 0 && o.qpos >= 0) {
                     cb[o.qpos] = x;
                     cw[o.qpos] = o.qrd * x;
@@ -396,12 +386,12 @@ __device__ __forceinline__ void treeCoarse(G& g, const TreePcgArgs<TK, TV>& a, b
     }
     // ---- coarsest level
     {
-        const TV* b = s.vec[3 * (L - 1)];
-        TV* e = s.vec[3 * (L - 1) + 2];
+        const double* b = s.vec[3 * (L - 1)];
+        double* e = s.vec[3 * (L - 1) + 2];
         const TreeLevel& v = s.lv[L - 1];
         if (top == L - 1) {
-            const VLevel<TV> f = a.T.nat[L - 2];
-            denseRows<TV>(g, v.n, v.npos, a.T.dense_inv, [&](int J) { return b[J]; }, [&](int I, TV x) {
+            const VLevel<double> f = a.T.nat[L - 2];
+            denseRows(g, v.n, v.npos, a.T.dense_inv, [&](int J) { return b[J]; }, [&](int I, double x) {
                 const int4 m = v.memb[v.pos[I]];
                 if (m.x >= 0) f.x[m.x] = f.w[m.x] + gamma * x;
                 if (m.y >= 0) f.x[m.y] = f.w[m.y] + gamma * x;
@@ -409,39 +399,39 @@ __device__ __forceinline__ void treeCoarse(G& g, const TreePcgArgs<TK, TV>& a, b
                 if (m.w >= 0) f.x[m.w] = f.w[m.w] + gamma * x;
             });
         } else {
-            denseRows<TV>(g, v.n, v.npos, a.T.dense_inv, [&](int J) { return b[J]; }, [&](int I, TV x) { e[I] = x; });
+            denseRows(g, v.n, v.npos, a.T.dense_inv, [&](int J) { return b[J]; }, [&](int I, double x) { e[I] = x; });
         }
         g.sync();
         mark(a.log, 50);
     }
     // ---- up, tree levels: the iterate is w + gamma e(coarse) of its rank
     for (int l = L - 2; l >= max(top, 1); --l) {
-        const TV *b = s.vec[3 * l], *w = s.vec[3 * l + 1], *ce = s.vec[3 * l + 5];
-        TV* e = s.vec[3 * l + 2];
+        const double *b = s.vec[3 * l], *w = s.vec[3 * l + 1], *ce = s.vec[3 * l + 5];
+        double* e = s.vec[3 * l + 2];
         const auto y = [&](int j) { return w[j] + gamma * ce[j >> 2]; };
         if (l > top || top == 0) {
             struct Own {
-                TV b, y;
+                double b, y;
             };
-            sweepTree<TV, TV, TV>(
+            sweepTree(
                 l, stored, omega, y,
-                [&](int p, const TreeOwn<TV>& o) { return o.rank >= 0 ? Own{b[p], y(p)} : Own{TV(0), TV(0)}; },
-                [&](int p, int q, int K, const TreeOwn<TV>& o, const Own& m, TV sum) {
-                    if (q == 0 && o.rank >= 0) e[o.rank] = m.y + o.rd * (m.b - (static_cast<TV>(o.d) * m.y + sum));
+                [&](int p, const TreeOwn& o) { return o.rank >= 0 ? Own{b[p], y(p)} : Own{0.0, 0.0}; },
+                [&](int p, int q, int K, const TreeOwn& o, const Own& m, double sum) {
+                    if (q == 0 && o.rank >= 0) e[o.rank] = m.y + o.rd * (m.b - (o.d * m.y + sum));
                 });
         } else {
             // the last tree level pushes into the streamed level above it
-            const VLevel<TV> f = a.T.nat[l - 1];
+            const VLevel<double> f = a.T.nat[l - 1];
             const int4* memb = s.lv[l].memb;
             struct Own {
-                TV b, y, w[4];
+                double b, y, w[4];
                 int4 m;
             };
             const int K0 = 1 << s.slot[l].k, q0 = threadIdx.x & (K0 - 1);  // lane q takes members q, q + K, ...
-            sweepTree<TV, TV, TV>(
+            sweepTree(
                 l, stored, omega, y,
-                [&](int p, const TreeOwn<TV>& o) {
-                    Own m{TV(0), TV(0), {TV(0), TV(0), TV(0), TV(0)}, make_int4(-1, -1, -1, -1)};
+                [&](int p, const TreeOwn& o) {
+                    Own m{0.0, 0.0, {0.0, 0.0, 0.0, 0.0}, make_int4(-1, -1, -1, -1)};
                     if (o.rank >= 0) {
                         m.m = memb[p];
                         m.b = b[p];
@@ -457,8 +447,8 @@ __device__ __forceinline__ void treeCoarse(G& g, const TreePcgArgs<TK, TV>& a, b
                     }
                     return m;
                 },
-                [&](int p, int q, int K, const TreeOwn<TV>& o, const Own& m, TV sum) {
-                    const TV add = gamma * (m.y + o.rd * (m.b - (static_cast<TV>(o.d) * m.y + sum)));
+                [&](int p, int q, int K, const TreeOwn& o, const Own& m, double sum) {
+                    const double add = gamma * (m.y + o.rd * (m.b - (o.d * m.y + sum)));
                     if (m.m.x >= 0) f.x[m.m.x] = m.w[0] + add;
                     if (m.m.y >= 0) f.x[m.m.y] = m.w[1] + add;
                     if (m.m.z >= 0) f.x[m.m.z] = m.w[2] + add;
@@ -470,15 +460,15 @@ __device__ __forceinline__ void treeCoarse(G& g, const TreePcgArgs<TK, TV>& a, b
     }
     // ---- up, streamed levels
     for (int l = top - 1; l >= 1; --l) {
-        const VLevel<TV> f = a.T.nat[l], fin = a.T.nat[l - 1];
+        const VLevel<double> f = a.T.nat[l], fin = a.T.nat[l - 1];
         if (l == L - 1) continue;  // the coarsest level is the dense one
-        const TV* x = f.x;
+        const double* x = f.x;
         for (int sl = c.gwarp; sl < f.A.nslices; sl += c.nwarps) {
             const int i = 32 * sl + c.lane;
-            const TV ax = sellRow(f.A, sl, c.lane, [&](int j) { return x[j]; });
+            const double ax = sellRow(f.A, sl, c.lane, [&](int j) { return x[j]; });
             if (i < f.A.n) {
-                const TV yi = x[i];
-                const TV add = gamma * (yi + f.rd[i] * (f.b[i] - (f.A.diag[i] * yi + ax)));
+                const double yi = x[i];
+                const double add = gamma * (yi + f.rd[i] * (f.b[i] - (f.A.diag[i] * yi + ax)));
                 for (int m = fin.agg_ptr[i]; m < fin.agg_ptr[i + 1]; ++m) {
                     const int ii = fin.agg_rows[m];
                     fin.x[ii] = fin.w[ii] + add;
@@ -491,26 +481,25 @@ __device__ __forceinline__ void treeCoarse(G& g, const TreePcgArgs<TK, TV>& a, b
 }
 
 // The CG iteration; see pcgBody in pcg_sell.cu for the recurrences and the fused update.
-template <class TK, class TV, bool TREE0, class G>
-__device__ void treeSolve(G& g, const TreePcgArgs<TK, TV>& a) {
-    openTree<TK, TV>(g, a);
-    TreeShared<TV>& s = treeShared<TV>();
+template <bool TREE0, class G>
+__device__ void treeSolve(G& g, const TreePcgArgs& a) {
+    openTree(g, a);
+    TreeShared& s = treeShared();
     const bool stored = s.used >= 0;
     const Lanes c = lanes<TB>(g);
     const int L = a.T.levels, n = a.n;
     constexpr bool tree0 = TREE0;           // level 0 in tree numbering too
     const bool flat = !TREE0 && L == 1;     // the preconditioner is the dense inverse
     const double omega = a.T.omega;
-    const TV gamma = a.T.gamma;
-    const SellMat<TK>& A = a.A;
-    VLevel<TV> f0{};
+    const double gamma = a.T.gamma;
+    const SellMat<double>& A = a.A;
+    VLevel<double> f0{};
     if (!tree0 && !flat) f0 = a.T.nat[0];
-    using TK2 = typename Pair<TK>::type;
-    TV* w0 = tree0 ? s.vec[1] : f0.w;  // omega / diagonal * r on level 0
-    TV *b1 = L > 1 ? s.vec[3] : nullptr, *w1 = L > 1 ? s.vec[4] : nullptr;
-    const TV* e1 = L > 1 ? s.vec[5] : nullptr;
+    double* w0 = tree0 ? s.vec[1] : f0.w;  // omega / diagonal * r on level 0
+    double *b1 = L > 1 ? s.vec[3] : nullptr, *w1 = L > 1 ? s.vec[4] : nullptr;
+    const double* e1 = L > 1 ? s.vec[5] : nullptr;
     const int* row0 = tree0 ? s.lv[0].row : nullptr;
-    TK* x = tree0 ? a.xt : a.x;
+    double* x = tree0 ? a.xt : a.x;
     int buf = 0;
     PcgState& st = *a.st;
     const int warm = st.warm;
@@ -519,27 +508,27 @@ __device__ void treeSolve(G& g, const TreePcgArgs<TK, TV>& a) {
     // the residual of the vector w on level 0 and its restriction, after w and r are set everywhere
     const auto firstResidual = [&] {
         if (tree0) {
-            const TK* r = a.r;
+            const double* r = a.r;
             struct Own {
-                TV b, w;
+                double b, w;
             };
-            sweepTree<TK, TV, TV>(
+            sweepTree(
                 0, stored, omega, [&](int j) { return w0[j]; },
-                [&](int p, const TreeOwn<TV>& o) {
-                    return o.rank >= 0 ? Own{static_cast<TV>(r[p]), w0[p]} : Own{TV(0), TV(0)};
+                [&](int p, const TreeOwn& o) {
+                    return o.rank >= 0 ? Own{r[p], w0[p]} : Own{0.0, 0.0};
                 },
-                [&](int p, int q, int K, const TreeOwn<TV>& o, const Own& m, TV sum) {
-                    const TV t = quadSum(o.rank >= 0 ? m.b - (static_cast<TV>(o.d) * m.w + sum) : TV(0), K);
+                [&](int p, int q, int K, const TreeOwn& o, const Own& m, double sum) {
+                    const double t = quadSum(o.rank >= 0 ? m.b - (o.d * m.w + sum) : 0.0, K);
                     if (q == 0 && (p & 3) == 0 && o.qpos >= 0) {
                         b1[o.qpos] = t;
                         w1[o.qpos] = o.qrd * t;
                     }
                 });
         } else {
-            const TV* w = f0.w;
+            const double* w = f0.w;
             for (int sl = c.gwarp; sl < f0.A.nslices; sl += c.nwarps) {
                 const int i = 32 * sl + c.lane;
-                const TV aw = sellRow(f0.A, sl, c.lane, [&](int j) { return w[j]; });
+                const double aw = sellRow(f0.A, sl, c.lane, [&](int j) { return w[j]; });
                 if (i < n) f0.t[i] = f0.b[i] - (f0.A.diag[i] * w[i] + aw);
             }
         }
@@ -547,44 +536,41 @@ __device__ void treeSolve(G& g, const TreePcgArgs<TK, TV>& a) {
         mark(a.log, 30);
     };
     // z = M r; this thread's share of r . z
-    const auto precondition = [&](const TK* r, TK2* zp) -> double {
+    const auto precondition = [&](const double* r, double2* zp) -> double {
         double rz = 0.0;
-        TK* z = reinterpret_cast<TK*>(a.zp0);  // level 0 in its own numbering
+        double* z = reinterpret_cast<double*>(a.zp0);  // level 0 in its own numbering
         if (flat) {
-            denseRows<TV>(g, n, n, a.T.dense_inv, [&](int J) { return static_cast<TV>(r[J]); }, [&](int I, TV v) {
-                const TK zi = static_cast<TK>(v);
-                z[I] = zi;
-                rz += static_cast<double>(r[I]) * static_cast<double>(zi);
+            denseRows(g, n, n, a.T.dense_inv, [&](int J) { return r[J]; }, [&](int I, double v) {
+                z[I] = v;
+                rz += r[I] * v;
             });
             return rz;
         }
-        treeCoarse<TK, TV, TREE0>(g, a, stored);
+        treeCoarse<TREE0>(g, a, stored);
         if (tree0) {
             const auto y = [&](int j) { return w0[j] + gamma * e1[j >> 2]; };
             struct Own {
-                TK r;
-                TV y;
+                double r, y;
             };
-            sweepTree<TK, TV, TV>(
+            sweepTree(
                 0, stored, omega, y,
-                [&](int p, const TreeOwn<TV>& o) { return o.rank >= 0 ? Own{r[p], y(p)} : Own{TK(0), TV(0)}; },
-                [&](int p, int q, int K, const TreeOwn<TV>& o, const Own& m, TV sum) {
+                [&](int p, const TreeOwn& o) { return o.rank >= 0 ? Own{r[p], y(p)} : Own{0.0, 0.0}; },
+                [&](int p, int q, int K, const TreeOwn& o, const Own& m, double sum) {
                     if (q != 0 || o.rank < 0) return;
-                    const TK zi = static_cast<TK>(
-                        m.y + o.rd * (static_cast<TV>(m.r) - (static_cast<TV>(o.d) * m.y + sum)));
+                    const double zi = m.y + o.rd * (m.r - (o.d * m.y + sum));
                     zp[p].x = zi;
-                    rz += static_cast<double>(m.r) * static_cast<double>(zi);
+                    rz += m.r * zi;
                 });
         } else {
-            const TV* y = f0.x;
+            const double* y = f0.x;
             for (int sl = c.gwarp; sl < f0.A.nslices; sl += c.nwarps) {
                 const int i = 32 * sl + c.lane;
-                const TV ay = sellRow(f0.A, sl, c.lane, [&](int j) { return y[j]; });
+                const double ay = sellRow(f0.A, sl, c.lane, [&](int j) { return y[j]; });
                 if (i < n) {
-                    const TV yi = y[i];
-                    const TK zi = static_cast<TK>(yi + f0.rd[i] * (f0.b[i] - (f0.A.diag[i] * yi + ay)));
+                    const double yi = y[i];
+                    const double zi = yi + f0.rd[i] * (f0.b[i] - (f0.A.diag[i] * yi + ay));
                     z[i] = zi;
-                    rz += static_cast<double>(r[i]) * static_cast<double>(zi);
+                    rz += r[i] * zi;
                 }
             }
         }
@@ -594,53 +580,52 @@ __device__ void treeSolve(G& g, const TreePcgArgs<TK, TV>& a) {
     double v[2] = {0.0, 0.0};
     if (tree0) {
         if (warm) {
-            treeRowsOf<TK, TV>(0, stored, omega, [&](int p, const TreeOwn<TV>& o) { x[p] = a.x[row0[p]]; });
+            treeRowsOf(0, stored, omega, [&](int p, const TreeOwn& o) { x[p] = a.x[row0[p]]; });
             g.sync();
         }
-        const auto seed = [&](int p, const TreeOwn<TV>& o, TK bi, TK ri) {
+        const auto seed = [&](int p, const TreeOwn& o, double bi, double ri) {
             a.r[p] = ri;
-            const TV wi = o.rd * static_cast<TV>(ri);
+            const double wi = o.rd * ri;
             w0[p] = wi;
-            a.wq0[p].x = static_cast<TK>(wi);
-            v[0] += static_cast<double>(ri) * static_cast<double>(ri);
-            v[1] += static_cast<double>(bi) * static_cast<double>(bi);
+            a.wq0[p].x = wi;
+            v[0] += ri * ri;
+            v[1] += bi * bi;
         };
         if (warm) {
-            const TK* xx = x;
-            sweepTree<TK, TK, TV>(
+            const double* xx = x;
+            sweepTree(
                 0, stored, omega, [&](int j) { return xx[j]; },
-                [&](int p, const TreeOwn<TV>& o) { return o.rank >= 0 ? a.b[row0[p]] : TK(0); },
-                [&](int p, int q, int K, const TreeOwn<TV>& o, TK bi, TK sum) {
-                    if (q == 0 && o.rank >= 0) seed(p, o, bi, bi - (static_cast<TK>(o.d) * xx[p] + sum));
+                [&](int p, const TreeOwn& o) { return o.rank >= 0 ? a.b[row0[p]] : 0.0; },
+                [&](int p, int q, int K, const TreeOwn& o, double bi, double sum) {
+                    if (q == 0 && o.rank >= 0) seed(p, o, bi, bi - (o.d * xx[p] + sum));
                 });
         } else {
-            treeRowsOf<TK, TV>(0, stored, omega, [&](int p, const TreeOwn<TV>& o) {
-                x[p] = TK(0);
-                const TK bi = a.b[row0[p]];
+            treeRowsOf(0, stored, omega, [&](int p, const TreeOwn& o) {
+                x[p] = 0.0;
+                const double bi = a.b[row0[p]];
                 seed(p, o, bi, bi);
             });
         }
     } else {
         for (int sl = c.gwarp; sl < A.nslices; sl += c.nwarps) {
             const int i = 32 * sl + c.lane;
-            TK ri = TK(0);
+            double ri = 0.0;
             if (warm) {
-                const TK* xx = x;
-                const TK ax = sellRow(A, sl, c.lane, [&](int j) { return xx[j]; });
+                const double* xx = x;
+                const double ax = sellRow(A, sl, c.lane, [&](int j) { return xx[j]; });
                 if (i < n) ri = a.b[i] - (A.diag[i] * xx[i] + ax);
             } else if (i < n) {
                 ri = a.b[i];
-                x[i] = TK(0);
+                x[i] = 0.0;
             }
             if (i < n) {
                 a.r[i] = ri;
                 if (!flat) {
-                    const TV rv = static_cast<TV>(ri);
-                    f0.b[i] = rv;
-                    f0.w[i] = f0.rd[i] * rv;
+                    f0.b[i] = ri;
+                    f0.w[i] = f0.rd[i] * ri;
                 }
-                v[0] += static_cast<double>(ri) * static_cast<double>(ri);
-                v[1] += static_cast<double>(a.b[i]) * static_cast<double>(a.b[i]);
+                v[0] += ri * ri;
+                v[1] += a.b[i] * a.b[i];
             }
         }
     }
@@ -664,7 +649,7 @@ __device__ void treeSolve(G& g, const TreePcgArgs<TK, TV>& a) {
     }
     const auto finish = [&](int status, int it, double rr) {
         if (tree0)
-            treeRowsOf<TK, TV>(0, stored, omega, [&](int p, const TreeOwn<TV>& o) { a.x[row0[p]] = x[p]; });
+            treeRowsOf(0, stored, omega, [&](int p, const TreeOwn& o) { a.x[row0[p]] = x[p]; });
         if (g.rank() == 0 && threadIdx.x == 0) {
             st.rr = rr;
             st.iterations = it;
@@ -676,12 +661,12 @@ __device__ void treeSolve(G& g, const TreePcgArgs<TK, TV>& a) {
         return;
     }
     if (!flat) firstResidual();
-    double rz = 0.0, rz_old_new = 0.0, beta = 0.0;
-    TK2 *zp = a.zp0, *zpn = a.zp1;  // {z, p} of this iteration, and of the next
-    TK2 *wq = a.wq0, *wqn = a.wq1;  // {w, omega / diagonal * q}
-    TK *r = a.r, *q = a.q;
+    double rz = 0.0, beta = 0.0;
+    double2 *zp = a.zp0, *zpn = a.zp1;  // {z, p} of this iteration, and of the next
+    double2 *wq = a.wq0, *wqn = a.wq1;  // {w, omega / diagonal * q}
+    double *r = a.r, *q = a.q;
     // level 0 in its own numbering keeps each vector apart (see TreePcgArgs)
-    TK *zs = reinterpret_cast<TK*>(a.zp0), *pold = zs + n, *pnew = reinterpret_cast<TK*>(a.zp1), *rn = pnew + n;
+    double *zs = reinterpret_cast<double*>(a.zp0), *pold = zs + n, *pnew = reinterpret_cast<double*>(a.zp1), *rn = pnew + n;
     int it = 0;
     int status = 1;
     double rr = v[0];
@@ -690,41 +675,40 @@ __device__ void treeSolve(G& g, const TreePcgArgs<TK, TV>& a) {
         gridSum<1, TB>(g, zr, a.partial, buf);
         mark(a.log, 4);
         if (g.aborted()) { status = 3; break; }
-        if (it > 0) beta = a.flexible ? (zr[0] - rz_old_new) / rz : zr[0] / rz;
+        if (it > 0) beta = zr[0] / rz;
         rz = zr[0];
         if (!isfinite(rz) || rz == 0.0) { status = 2; break; }
         // p_new = z + beta p_old and q = A p_new in one sweep (neighbours' p_new formed on the fly)
-        const TK bk = static_cast<TK>(beta);
         const bool first = beta == 0.0;
         const auto pj = [&](int j) {
-            const TK2 v2 = zp[j];
-            return first ? v2.x : v2.x + bk * v2.y;
+            const double2 v2 = zp[j];
+            return first ? v2.x : v2.x + beta * v2.y;
         };
         double pq[1] = {0.0};
         if (tree0) {
-            sweepTree<TK, TK, TV>(
-                0, stored, omega, pj, [&](int p, const TreeOwn<TV>& o) { return o.rank >= 0 ? pj(p) : TK(0); },
-                [&](int p, int sub, int K, const TreeOwn<TV>& o, TK pi, TK sum) {
+            sweepTree(
+                0, stored, omega, pj, [&](int p, const TreeOwn& o) { return o.rank >= 0 ? pj(p) : 0.0; },
+                [&](int p, int sub, int K, const TreeOwn& o, double pi, double sum) {
                     if (sub != 0 || o.rank < 0) return;
-                    const TK qi = static_cast<TK>(o.d) * pi + sum;
+                    const double qi = o.d * pi + sum;
                     zpn[p].y = pi;
                     q[p] = qi;
-                    wq[p].y = static_cast<TK>(o.rd) * qi;
-                    pq[0] += static_cast<double>(pi) * static_cast<double>(qi);
+                    wq[p].y = o.rd * qi;
+                    pq[0] += pi * qi;
                 });
         } else {
-            const TK* zz = zs;
-            const TK* po = pold;
+            const double* zz = zs;
+            const double* po = pold;
             for (int sl = c.gwarp; sl < A.nslices; sl += c.nwarps) {
                 const int i = 32 * sl + c.lane;
-                const TK ap = first ? sellRow(A, sl, c.lane, [&](int j) { return zz[j]; })
-                                    : sellRow(A, sl, c.lane, [&](int j) { return zz[j] + bk * po[j]; });
+                const double ap = first ? sellRow(A, sl, c.lane, [&](int j) { return zz[j]; })
+                                    : sellRow(A, sl, c.lane, [&](int j) { return zz[j] + beta * po[j]; });
                 if (i < n) {
-                    const TK pi = first ? zz[i] : zz[i] + bk * po[i];
-                    const TK qi = A.diag[i] * pi + ap;
+                    const double pi = first ? zz[i] : zz[i] + beta * po[i];
+                    const double qi = A.diag[i] * pi + ap;
                     pnew[i] = pi;
                     q[i] = qi;
-                    pq[0] += static_cast<double>(pi) * static_cast<double>(qi);
+                    pq[0] += pi * qi;
                 }
             }
         }
@@ -732,86 +716,77 @@ __device__ void treeSolve(G& g, const TreePcgArgs<TK, TV>& a) {
         mark(a.log, 2);
         if (!(fabs(pq[0]) > 0.0) || !isfinite(pq[0])) { status = 2; break; }
         const double alpha = rz / pq[0];
-        const TK ak = static_cast<TK>(alpha);
         const auto wj = [&](int j) {
-            const TK2 v2 = wq[j];
-            return static_cast<TV>(v2.x - ak * v2.y);
+            const double2 v2 = wq[j];
+            return v2.x - alpha * v2.y;
         };
-        double nr[2] = {0.0, 0.0};
+        double nr[1] = {0.0};
         if (tree0) {
             // x += alpha p, r_new = r - alpha q, w = rd r_new, and the residual of w (neighbours' w
             // formed from their pairs) restricted to level 1, all in this phase
             struct Own {
-                TK r, x, z;
+                double r, x;
             };
-            sweepTree<TK, TV, TV>(
+            sweepTree(
                 0, stored, omega, wj,
-                [&](int p, const TreeOwn<TV>& o) {
-                    return o.rank >= 0 ? Own{r[p] - ak * q[p], x[p] + ak * zpn[p].y, a.flexible ? zp[p].x : TK(0)}
-                                       : Own{TK(0), TK(0), TK(0)};
+                [&](int p, const TreeOwn& o) {
+                    return o.rank >= 0 ? Own{r[p] - alpha * q[p], x[p] + alpha * zpn[p].y} : Own{0.0, 0.0};
                 },
-                [&](int p, int sub, int K, const TreeOwn<TV>& o, const Own& m, TV sum) {
-                    const TV rv = static_cast<TV>(m.r);
-                    const TV wi = o.rd * rv;
+                [&](int p, int sub, int K, const TreeOwn& o, const Own& m, double sum) {
+                    const double wi = o.rd * m.r;
                     if (sub == 0 && o.rank >= 0) {
                         x[p] = m.x;
                         r[p] = m.r;
                         w0[p] = wi;
-                        wqn[p].x = static_cast<TK>(wi);
-                        nr[0] += static_cast<double>(m.r) * static_cast<double>(m.r);
-                        nr[1] += static_cast<double>(m.r) * static_cast<double>(m.z);
+                        wqn[p].x = wi;
+                        nr[0] += m.r * m.r;
                     }
-                    const TV t = quadSum(o.rank >= 0 ? rv - (static_cast<TV>(o.d) * wi + sum) : TV(0), K);
+                    const double t = quadSum(o.rank >= 0 ? m.r - (o.d * wi + sum) : 0.0, K);
                     if (sub == 0 && (p & 3) == 0 && o.qpos >= 0) {
                         b1[o.qpos] = t;
                         w1[o.qpos] = o.qrd * t;
                     }
                 });
         } else if (!flat) {
-            const TV* rd = f0.rd;
-            const TK *rc = r, *qq = q;
+            const double* rd = f0.rd;
+            const double *rc = r, *qq = q;
             for (int sl = c.gwarp; sl < f0.A.nslices; sl += c.nwarps) {
                 const int i = 32 * sl + c.lane;
-                const TV aw = sellRow(f0.A, sl, c.lane,
-                                      [&](int j) { return rd[j] * static_cast<TV>(rc[j] - ak * qq[j]); });
+                const double aw = sellRow(f0.A, sl, c.lane, [&](int j) { return rd[j] * (rc[j] - alpha * qq[j]); });
                 if (i < n) {
-                    x[i] += ak * pnew[i];
-                    const TK ri = rc[i] - ak * qq[i];
+                    x[i] += alpha * pnew[i];
+                    const double ri = rc[i] - alpha * qq[i];
                     rn[i] = ri;
-                    const TV rv = static_cast<TV>(ri);
-                    const TV wi = rd[i] * rv;
-                    f0.b[i] = rv;
+                    const double wi = rd[i] * ri;
+                    f0.b[i] = ri;
                     f0.w[i] = wi;
-                    f0.t[i] = rv - (f0.A.diag[i] * wi + aw);
-                    nr[0] += static_cast<double>(ri) * static_cast<double>(ri);
-                    if (a.flexible) nr[1] += static_cast<double>(ri) * static_cast<double>(zs[i]);
+                    f0.t[i] = ri - (f0.A.diag[i] * wi + aw);
+                    nr[0] += ri * ri;
                 }
             }
         } else {
             for (int i = c.gthread; i < n; i += c.nthreads) {
-                x[i] += ak * pnew[i];
-                const TK ri = r[i] - ak * q[i];
+                x[i] += alpha * pnew[i];
+                const double ri = r[i] - alpha * q[i];
                 rn[i] = ri;
-                nr[0] += static_cast<double>(ri) * static_cast<double>(ri);
-                if (a.flexible) nr[1] += static_cast<double>(ri) * static_cast<double>(zs[i]);
+                nr[0] += ri * ri;
             }
         }
-        gridSum<2, TB>(g, nr, a.partial, buf);
+        gridSum<1, TB>(g, nr, a.partial, buf);
         mark(a.log, 3);
         rr = nr[0];
-        rz_old_new = nr[1];
         ++it;
         if (!isfinite(rr)) { status = 2; break; }
         if (rr <= target2) { status = 0; break; }
         if (!tree0) {
-            TK* t1 = r;
+            double* t1 = r;
             r = rn;
             rn = t1;
         }
-        TK* t1 = pold;
+        double* t1 = pold;
         pold = pnew;
         pnew = t1;
-        TK2* tmp = zp;
+        double2* tmp = zp;
         zp = zpn;
         zpn = tmp;
         tmp = wq;
@@ -821,45 +796,40 @@ __device__ void treeSolve(G& g, const TreePcgArgs<TK, TV>& a) {
     finish(g.failed() ? 3 : status, it, rr);
 }
 
-template <class TK, class TV, class G>
-__device__ __forceinline__ void treeBody(G& g, const TreePcgArgs<TK, TV>& a) {
-    if (a.top == 0 && a.T.levels > 1) treeSolve<TK, TV, true>(g, a);
-    else treeSolve<TK, TV, false>(g, a);
+template <class G>
+__device__ __forceinline__ void treeBody(G& g, const TreePcgArgs& a) {
+    if (a.top == 0 && a.T.levels > 1) treeSolve<true>(g, a);
+    else treeSolve<false>(g, a);
 }
 
-template <class TK, class TV>
-__global__ void __launch_bounds__(TB, 1) kPcgTree(const __grid_constant__ TreePcgArgs<TK, TV> a, SegmentBarrier* bar) {
+__global__ void __launch_bounds__(TB, 1) kPcgTree(const __grid_constant__ TreePcgArgs a, SegmentBarrier* bar) {
     GridGroup g{bar};
-    treeBody<TK, TV>(g, a);
+    treeBody(g, a);
 }
 
 // The systems of a batched launch as one kernel argument.
-template <class TK, class TV>
 struct TreeArgsBlock {
-    TreePcgArgs<TK, TV> a[kBatchArgs];
+    TreePcgArgs a[kBatchArgs];
     int begin[kBatchArgs + 1];  // CTA ranges
     int count;
 };
-static_assert(sizeof(TreeArgsBlock<double, double>) + sizeof(void*) <= kKernelArgumentBytes, "one kernel argument");
+static_assert(sizeof(TreeArgsBlock) + sizeof(void*) <= kKernelArgumentBytes, "one kernel argument");
 
 // A batch: CTAs [begin[s], begin[s+1]) solve system s.
-template <class TK, class TV>
 __global__ void __launch_bounds__(TB, 1)
-    kPcgTreeBatch(const __grid_constant__ TreeArgsBlock<TK, TV> batch, SegmentBarrier* bars) {
+    kPcgTreeBatch(const __grid_constant__ TreeArgsBlock batch, SegmentBarrier* bars) {
     const int s = systemOfBlock(batch.begin, batch.count);
     SegmentGroup g{batch.begin[s], batch.begin[s + 1] - batch.begin[s], bars + s};
-    treeBody<TK, TV>(g, batch.a[s]);
+    treeBody(g, batch.a[s]);
 }
 
 // A small system on one cluster.
-template <class TK, class TV>
-__global__ void __launch_bounds__(TB, 1) kPcgTreeCluster(const __grid_constant__ TreePcgArgs<TK, TV> a) {
+__global__ void __launch_bounds__(TB, 1) kPcgTreeCluster(const __grid_constant__ TreePcgArgs a) {
     ClusterGroup g;
     g.sync();  // every CTA's shared memory is live
-    treeBody<TK, TV>(g, a);
+    treeBody(g, a);
 }
-template <class TK, class TV>
-TreePlan::Place place(const TreePlan& plan, TreePcgArgs<TK, TV>& a, int ctas) {
+TreePlan::Place place(const TreePlan& plan, TreePcgArgs& a, int ctas) {
     const TreePlan::Place p = plan.place(ctas);
     a.top = p.top;
     a.smem = p.smem;
@@ -873,13 +843,13 @@ TreePlan::Place place(const TreePlan& plan, TreePcgArgs<TK, TV>& a, int ctas) {
 }  // namespace
 
 double TreePlan::bytes(int from, int levels, int ctas) const {
-    const double own = value_bytes == 8 ? sizeof(TreeOwn<double>) : sizeof(TreeOwn<float>);
+    const double own = sizeof(TreeOwn);
     double total = 64.0;
     for (int l = from; l < levels - 1; ++l) {
         const int K = 1 << treeLanes(static_cast<int>(slices[l]), ctas * (TB / 32));
         const double wide = slices[l] > 0 ? entries[l] / (32.0 * slices[l]) : 0.0;
         const double steps = K == 1 ? wide : wide / K + 0.5 * (K - 1) / K;
-        const double entry = (l == 0 ? level0_bytes : value_bytes) + 4.0;
+        constexpr double entry = sizeof(double) + sizeof(int);
         // a few per cent for uneven slices, and the unit a CTA may have more than its share
         total += 1.04 * slices[l] * (K * (steps * 32.0 * entry + kDirBytes) + 32.0 * own) / ctas + steps * 32.0 * entry +
                  32.0 / K * own;
@@ -894,7 +864,7 @@ bool TreePlan::fits(int from, int ctas) const {
 TreePlan::Place TreePlan::place(int ctas) const {
     const int L = static_cast<int>(slices.size());
     Place p{L - 1, L, 0};
-    if (folded && static_cast<double>(rows[L - 2]) * positions[L - 2] * value_bytes <= kFoldedBytes * static_cast<double>(ctas))
+    if (folded && static_cast<double>(rows[L - 2]) * positions[L - 2] * sizeof(double) <= kFoldedBytes * static_cast<double>(ctas))
         p.levels = L - 1;
     p.top = p.levels - 1;
     if (first == 0 && p.levels > 1 && bytes(0, p.levels, ctas) <= kTreeSmem) p.top = 0;
@@ -904,39 +874,37 @@ TreePlan::Place TreePlan::place(int ctas) const {
     return p;
 }
 
-template <class TK, class TV>
-TreePlan::Place launchTreePcg(Context& ctx, const TreePlan& plan, TreePcgArgs<TK, TV> a) {
+TreePlan::Place launchTreePcg(Context& ctx, const TreePlan& plan, TreePcgArgs a) {
     a.log = PhaseLog{ctx.phase_entries, ctx.phase_capacity, ctx.phase_count};
     if (plan.nnz <= kClusterEntries) {
-        allowSharedMemory<kPcgTreeCluster<TK, TV>>(kTreeSmem);
-        const TreePlan::Place at = place(plan, a, clusterCtas<kPcgTreeCluster<TK, TV>>(TB, kTreeSmem));
+        allowSharedMemory<kPcgTreeCluster>(kTreeSmem);
+        const TreePlan::Place at = place(plan, a, clusterCtas<kPcgTreeCluster>(TB, kTreeSmem));
         BSG_PROFILE(ctx, "pcg_amg_persistent");
-        launchCluster<kPcgTreeCluster<TK, TV>>(ctx, 1, TB, a.smem, kTreeSmem, a);
+        launchCluster<kPcgTreeCluster>(ctx, 1, TB, a.smem, kTreeSmem, a);
         return at;
     }
-    allowSharedMemory<kPcgTree<TK, TV>>(kTreeSmem);
+    allowSharedMemory<kPcgTree>(kTreeSmem);
     const int grid = ctx.sm_count;
     const TreePlan::Place at = place(plan, a, grid);
     SegmentBarrier* bar = ctx.grid_barrier;
     resetBarriers(ctx, bar, 1, grid);
     void* params[] = {&a, &bar};
     BSG_PROFILE(ctx, "pcg_amg_persistent");
-    BSG_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(kPcgTree<TK, TV>), grid, TB, params, a.smem, ctx.stream));
+    BSG_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(kPcgTree), grid, TB, params, a.smem, ctx.stream));
     ctx.launched();
     return at;
 }
 
-template <class TK, class TV>
-void launchTreePcgBatch(Context& ctx, TreeBatch<TK, TV>& batch) {
+void launchTreePcgBatch(Context& ctx, TreeBatch& batch) {
     const std::size_t count = batch.args.size();
     if (count == 0) return;
-    allowSharedMemory<kPcgTreeBatch<TK, TV>>(kTreeSmem);
+    allowSharedMemory<kPcgTreeBatch>(kTreeSmem);
     batch.d_bars.resize(std::max(batch.d_bars.size(), count));
     const std::vector<long long> slices(batch.slices.begin(), batch.slices.end());
     const std::vector<std::size_t> launches = batchLaunches(slices, TB / 32, ctx.sm_count);
     for (std::size_t l = 0; l + 1 < launches.size(); ++l) {
         const std::size_t k0 = launches[l], k1 = launches[l + 1];
-        TreeArgsBlock<TK, TV> block{};
+        TreeArgsBlock block{};
         const int m = block.count = static_cast<int>(k1 - k0);
         const std::vector<int> begin = allotCtas({slices.begin() + k0, slices.begin() + k1}, TB / 32, ctx.sm_count);
         std::copy(begin.begin(), begin.end(), block.begin);
@@ -950,17 +918,11 @@ void launchTreePcgBatch(Context& ctx, TreeBatch<TK, TV>& batch) {
         resetBarriers(ctx, bars, m, begin.back(), block.begin);
         void* params[] = {&block, &bars};
         BSG_PROFILE(ctx, "pcg_amg_persistent_batch");
-        BSG_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(kPcgTreeBatch<TK, TV>), begin.back(), TB, params,
+        BSG_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(kPcgTreeBatch), begin.back(), TB, params,
                                              smem, ctx.stream));
         ctx.launched();
     }
     batch.bars_used = static_cast<int>(count);
 }
-
-template TreePlan::Place launchTreePcg<double, double>(Context&, const TreePlan&, TreePcgArgs<double, double>);
-template TreePlan::Place launchTreePcg<double, float>(Context&, const TreePlan&, TreePcgArgs<double, float>);
-template TreePlan::Place launchTreePcg<float, float>(Context&, const TreePlan&, TreePcgArgs<float, float>);
-template void launchTreePcgBatch<double, double>(Context&, TreeBatch<double, double>&);
-template void launchTreePcgBatch<double, float>(Context&, TreeBatch<double, float>&);
 
 }  // namespace bsg

@@ -17,6 +17,12 @@
 //
 // Phases per CG iteration with L levels and top = 0: 2 L; with top > 0 one or two more per
 // streamed level.
+//
+// FP64 only.  An FP32 V-cycle (precision 1 and 2) stays on the streaming kernel: there rounding decides after
+// which iteration a solve is accepted, and rows split over lanes, other sums and folded levels round otherwise
+// (CG counts of mixed 110k-cell outer iterations moved by one or two in 7 of 16, p by up to 1.5e-9 relative; in FP64,
+// 7e-13).  Mixed outer iterations, on chip / streamed: 8k cells 2.8 / 4.6 ms, 33k 4.0 / 6.3, 110k 6.9 / 9.5, 373k
+// 17.8 / 21.4.
 #pragma once
 
 #include "group.cuh"
@@ -45,50 +51,36 @@ struct TreeLevel {
     const double* diag = nullptr;
 };
 
-template <class T>
-struct Pair;
-template <>
-struct Pair<double> {
-    using type = double2;
-};
-template <>
-struct Pair<float> {
-    using type = float2;
-};
-
-template <class TV>
 struct TreeView {
     int levels = 0;                    // L
     int first = 0;                     // the finest level that has a tree numbering
-    TV gamma = TV(1);
+    double gamma = 1.0;
     double omega = 1.0;
     const TreeLevel* lv = nullptr;     // device array of L (entries below `first` unused)
-    const VLevel<TV>* nat = nullptr;   // device array of L: the levels in their own numbering
-    TV* const* vec = nullptr;          // device array of 3 L: b, w, e of every tree level
-    const TV* dense_inv = nullptr;     // coarsest inverse, n x n row-major (by row)
-    const TV* folded = nullptr;        // level L - 2: its whole V-cycle as a matrix, rank x position
+    const VLevel<double>* nat = nullptr;   // device array of L: the levels in their own numbering
+    double* const* vec = nullptr;          // device array of 3 L: b, w, e of every tree level
+    const double* dense_inv = nullptr;     // coarsest inverse, n x n row-major (by row)
+    const double* folded = nullptr;        // level L - 2: its whole V-cycle as a matrix, rank x position
 };
 
-template <class TK, class TV>
 struct TreePcgArgs {
-    SellMat<TK> A;    // level 0 in its own numbering (top > 0)
-    TreeView<TV> T;
+    SellMat<double> A;    // level 0 in its own numbering (top > 0)
+    TreeView T;
     int top = 0;      // finest level in tree numbering in this launch
     int n = 0;        // rows of level 0
-    const TK* b;
-    TK* x;
+    const double* b;
+    double* x;
     // At least max(n, positions of level 0) entries each.  With level 0 in tree numbering what
     // neighbours gather together lies together: {z, p} of an iteration, and {w, omega / diagonal
     // * q}, each in two buffers that alternate, so a sweep gathers one 16-byte pair per entry
     // instead of two or three values, which counts where every gather goes to L2.  A streamed
     // level 0 keeps its vectors apart (in the same memory): there the pairs' half-written sectors
     // cost more (1M cells: 70 against 58 us per product).
-    TK *r, *q, *xt;
-    typename Pair<TK>::type *zp0, *zp1, *wq0, *wq1;
+    double *r, *q, *xt;
+    double2 *zp0, *zp1, *wq0, *wq1;
     double* partial;
     PcgState* st;
     PhaseLog log;
-    int flexible = 0;  // Polak-Ribiere beta (see SellPcgArgs)
     int smem = 0;      // bytes of dynamic shared memory for matrix rows
 };
 
@@ -99,7 +91,6 @@ struct TreePlan {
     std::vector<int> rows, positions;
     int first = 0;                   // finest level with a tree numbering
     long long nnz = 0;               // off-diagonal entries of level 0
-    int value_bytes = 8, level0_bytes = 8;
     bool folded = false;             // the V-cycle from level L - 2 down exists as one dense matrix
     // Bytes of shared memory per CTA for the rows of levels [from, levels - 1).
     double bytes(int from, int levels, int ctas) const;
@@ -111,20 +102,17 @@ struct TreePlan {
 };
 
 // One system: on one thread-block cluster when it is small, else on the whole grid.  Returns its placement.
-template <class TK, class TV>
-TreePlan::Place launchTreePcg(Context& ctx, const TreePlan& plan, TreePcgArgs<TK, TV> args);
+TreePlan::Place launchTreePcg(Context& ctx, const TreePlan& plan, TreePcgArgs args);
 
 // Systems of a batch, side by side on CTA ranges of one cooperative launch (several launches when
 // they outnumber its argument block), each with barriers of its own.
-template <class TK, class TV>
 struct TreeBatch {
-    std::vector<TreePcgArgs<TK, TV>> args;
+    std::vector<TreePcgArgs> args;
     std::vector<const TreePlan*> plans;
     std::vector<int> slices;         // level-0 slices, for the CTA shares
     DeviceArray<SegmentBarrier> d_bars;
     int bars_used = 0;               // barriers of the last launch, for its error report
 };
-template <class TK, class TV>
-void launchTreePcgBatch(Context& ctx, TreeBatch<TK, TV>& batch);
+void launchTreePcgBatch(Context& ctx, TreeBatch& batch);
 
 }  // namespace bsg

@@ -64,8 +64,12 @@ def test_scale_and_iterations(ctx, monkeypatch, shape, weights, precision):
         monkeypatch.delenv("BSG_AMG_GAMMA", raising=False)
         return counts
     fresh = {k: sequence([k])[0] for k in kinds}
-    assert fresh["stretched"] <= 0.9 * sequence(["stretched"], "1.8")[0]  # the trial moved the scale
-    assert sequence(["plain"], "1.8")[0] == fresh["plain"]                # and left it here
+    moved = sequence(["stretched"], "1.8")[0]
+    if precision == 0:
+        assert fresh["stretched"] <= 0.9 * moved    # the trial moved the scale
+    else:
+        assert fresh["stretched"] == moved          # FP32 V-cycles keep the fixed one
+    assert sequence(["plain"], "1.8")[0] == fresh["plain"]  # and left it here
     for first, then in (("plain", "stretched"), ("stretched", "plain")):
         names = [first] + 3 * [then]
         fixed = sequence(names, "1.8")

@@ -19,9 +19,8 @@ def ctx():
     c.close()
 
 
-@pytest.mark.parametrize("precision", [0, 1, 2])
 @pytest.mark.parametrize("shape", [(24, 24, 24), (48, 48, 48), (80, 80, 80)], ids=lambda s: "x".join(map(str, s)))
-def test_bytes_per_iteration(ctx, shape, precision):
+def test_bytes_per_iteration(ctx, shape):
     import babelsim_b200 as bsg
     poly = meshgen.hex_box(*shape, flat=True)
     own, nbr = np.asarray(poly.owner, np.int64), np.asarray(poly.neighbour, np.int64)
@@ -35,9 +34,9 @@ def test_bytes_per_iteration(ctx, shape, precision):
     mesh = bsg.Mesh.from_polyhedral(ctx, poly)
     system = bsg.LinearSystem(mesh)
     seen = []
-    for rtol in (1e-3, 1e-3, 1e-5):  # (precision 1: one pass of its inner solver)
+    for rtol in (1e-3, 1e-3, 1e-5):
         ctx.profile(True)
-        _, res = system.solve(bsg.solver_config("cg", "hypre", 1e-30, rtol, 500, precision=precision), d, -c, -c, b)
+        _, res = system.solve(bsg.solver_config("cg", "hypre", 1e-30, rtol, 500), d, -c, -c, b)
         _, _, declared, iterations = ctx.profile_report()["pcg_amg_persistent"]
         ctx.profile(False)
         assert res[0].status == 0
@@ -45,10 +44,9 @@ def test_bytes_per_iteration(ctx, shape, precision):
     (b0, i0), (b1, i1) = seen[1:]
     assert i1 > i0
     per = (b1 - b0) / (i1 - i0)
-    k, s = (4 if precision == 1 else 8), (4 if precision else 8)
     if n < 200000:
-        assert 0.9 * 17 * k * n <= per <= (17 * k + 3 * s + 4 * s) * n + s * 500 * 500
+        assert 0.9 * 17 * 8 * n <= per <= 24 * 8 * n + 8 * 500 * 500
     else:
-        assert per >= 2 * (4 + s) * 6 * n * 0.95 + (4 + k) * 6 * n * 0.95
+        assert per >= 3 * 12 * 6 * n * 0.95
     system.close()
     mesh.close()
