@@ -804,8 +804,6 @@ SolveOutcome KrylovSolver::solvePersistent(const Dcsr<double>& A, const SolverCo
     Context& ctx = m.ctx;
     const int n = A.n;
     if (amg) amg->prepareCg();
-    // (the FP32 inner solves keep the start scale, with which precision 1 has always given its fields: which
-    // iterate a refinement accepts depends on the cycle)
     if (cfg.precision == 1 && amg && amg->fp32VCycle()) return solveRefined(A, cfg, amg, b, x);
     if (amg && amg->hasTree()) m.ensureTree(*amg);
     else m.ensure(n);
