@@ -273,9 +273,10 @@ __device__ void bicgBody(G& g, const BicgArgs<C, T>& a) {
 // A small or middling solve is latency: five barriers per iteration, each followed by loads whose
 // addresses depend on one another (slice offset -> column -> vector).  Here each CTA owns a range of
 // slices and copies its matrix rows into shared memory once; neighbours only ever gather ph and sh, so
-// the other vectors, which nobody else reads, live in shared memory too.  The direction and the solution update share a phase: rho' = r0 . r is taken as r0 . s - omega r0 . t,
-// whose products ride with those of the two phases before, so beta is known when x, r and p are
-// formed and four barriers remain.  ||r|| itself is summed as before.
+// the other vectors, which nobody else reads, live in shared memory too.  The direction and the solution
+// update share a phase: rho' = r0 . r is taken as r0 . s - omega r0 . t, whose products ride with those of
+// the two phases before, so beta is known when x, r and p are formed and four barriers remain.  ||r|| itself
+// is summed as before.  FP64 systems only (see launchBicgstab).
 
 struct ChipSlot {
     int s0, nsl, k, nu;  // slices [s0, s0 + nsl), 2^k lanes per row, nsl << k units

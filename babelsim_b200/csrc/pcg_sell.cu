@@ -8,8 +8,8 @@
 namespace bsg {
 namespace {
 
-// This kernel serves the hierarchies pcg_tree.cu does not take (two smoothing steps, aggregates
-// of more than four rows).  One system: one CTA of 1024 threads per SM, since the grid barrier costs
+// This kernel serves the hierarchies pcg_tree.cu does not take (FP32 V-cycles, two smoothing steps,
+// aggregates of more than four rows).  One system: one CTA of 1024 threads per SM, since the grid barrier costs
 // by its arrivals (592 CTAs of 256 threads 2.1 us, 148 of 1024 1.3; two smoothing steps, 33k-cell
 // Voronoi cube: 7.30 against 6.77 ms per three solves).  A batch: CTAs of 256 threads, three per
 // SM, because its systems share the SMs in fine steps (eight cavities, 9.5 against 10.5 ms).
